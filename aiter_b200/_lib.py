@@ -8,7 +8,9 @@ There is no fallback: if the library is missing or does not load, importing an o
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
+import struct
 
 import torch
 
@@ -33,7 +35,7 @@ class aiter_tensor_t(ctypes.Structure):
 
 assert ctypes.sizeof(aiter_tensor_t) == 160
 
-_T = ctypes.POINTER(aiter_tensor_t)
+_T = ctypes.c_void_p   # const aiter_tensor_t*: a byref() of the structure, or the packed bytes of one (see _pack)
 _SIGNATURES = {
     "aiter_ctypes_abi_version": (ctypes.c_int, []),
     "aiter_get_last_error": (ctypes.c_char_p, []),
@@ -59,6 +61,8 @@ _SIGNATURES = {
     "b200_ep_ipc_open": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int, ctypes.POINTER(ctypes.c_int64)]),
     "b200_ep_ipc_close": (ctypes.c_int, [ctypes.c_int64, ctypes.c_int]),
     "b200_moe_debug_config": (ctypes.c_int, [ctypes.c_int64, ctypes.c_int]),
+    "b200_fused_moe_workspace_size": (ctypes.c_int64, [ctypes.c_int64] * 5 + [ctypes.c_int] * 2),
+    "b200_fused_moe": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p]),
 }
 
 _lib = None
@@ -121,33 +125,63 @@ def call_plain(name: str, *args):
         raise RuntimeError(f"{name} failed: {msg.decode() if msg else 'unknown error'}")
 
 
+# The whole POD in one go: filling the 20 fields of a ctypes.Structure one by one costs ~8 us per tensor, packing them
+# ~1 us, and an entry point takes up to 11 tensors.
+_POD = struct.Struct("@PNi8q8qii")
+assert _POD.size == 160
+
+
+def _pack(t: torch.Tensor) -> bytes:
+    """The aiter_tensor_t of ``t`` as bytes (the struct only borrows the storage)."""
+    code = AITER_DTYPE.get(t.dtype)
+    if code is None:
+        raise TypeError(f"unsupported dtype for the C-ABI: {t.dtype}")
+    shape, strides = t.shape, t.stride()
+    n = len(shape)
+    if n > 8:
+        raise ValueError("tensors of more than 8 dimensions are not supported")
+    pad = _ZEROS[n:]
+    return _POD.pack(t.data_ptr(), t.numel(), n, *shape, *pad, *strides, *pad, code, t.get_device() if t.is_cuda else -1)
+
+
+_ZEROS = (0,) * 8
+
+
+@functools.lru_cache(maxsize=None)
+def _fn(name: str):
+    return getattr(lib(), name)
+
+
+def raise_last_error(name: str):
+    msg = lib().aiter_get_last_error()
+    raise RuntimeError(f"{name} failed: {msg.decode() if msg else 'unknown error'}")
+
+
+def current_stream(device_index: int) -> int:
+    """Raw handle of torch's current stream on that device (what ``torch.cuda.current_stream().cuda_stream`` holds,
+    without building the two Python objects)."""
+    return torch._C._cuda_getCurrentRawStream(device_index)
+
+
 def call(name: str, *args, device: torch.device | None = None):
     """Calls an int-status entry point; tensors are marshalled, the stream of ``device`` (or of
     the first CUDA tensor) is appended."""
-    handle = lib()
-    fn = getattr(handle, name)
-    keep = []
     cargs = []
+    index = device.index if device is not None else None
     for a in args:
         if isinstance(a, torch.Tensor):
             if device is None and a.is_cuda:
-                device = a.device
-            s = to_aiter(a)
-            keep.append(s)
-            cargs.append(ctypes.byref(s))
-        elif a is None:
-            cargs.append(None)
+                device, index = a.device, a.get_device()
+            cargs.append(_pack(a))
         else:
             cargs.append(a)
     if device is None:
         raise RuntimeError(f"{name}: no CUDA tensor among the arguments")
-    stream = torch.cuda.current_stream(device).cuda_stream
+    stream = current_stream(torch.cuda.current_device() if index is None else index)
     global launch_count
     if name == "b200_moe_sorting_fwd":
         launch_count += 3 if args[0].numel() > 16384 else 1
     else:
         launch_count += _KERNELS_PER_CALL.get(name, 1)
-    status = fn(*cargs, ctypes.c_void_p(stream))
-    if status != 0:
-        msg = handle.aiter_get_last_error()
-        raise RuntimeError(f"{name} failed: {msg.decode() if msg else 'unknown error'}")
+    if _fn(name)(*cargs, stream) != 0:
+        raise_last_error(name)

@@ -32,6 +32,10 @@ void launch_moe_stage2(const aiter_tensor_t*, const aiter_tensor_t*, const aiter
                        const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*,
                        aiter_tensor_t*, aiter_tensor_t*, int, int, int, int, int, cudaStream_t);
 
+int64_t fused_moe_workspace_bytes(int64_t, int64_t, int64_t, int64_t, int64_t, int, int);
+void launch_fused_moe(const b200_fused_moe_args&, cudaStream_t);
+void launch_finalize(aiter_tensor_t*, const aiter_tensor_t*, cudaStream_t);
+
 void set_gemm_debug(long long, int);
 
 void launch_biased_grouped_topk(const aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*, aiter_tensor_t*, int, int,
@@ -71,6 +75,8 @@ __global__ void __launch_bounds__(256) finalize_kernel(const float4* __restrict_
     }
 }
 
+}  // namespace
+
 void launch_finalize(aiter_tensor_t* out, const aiter_tensor_t* acc, cudaStream_t stream) {
     check_tensor(acc, "acc", AITER_DTYPE_fp32, -1);
     check_tensor(out, "out", -1, -1);
@@ -91,7 +97,6 @@ void launch_finalize(aiter_tensor_t* out, const aiter_tensor_t* acc, cudaStream_
     B200_CUDA(cudaGetLastError());
 }
 
-}  // namespace
 }  // namespace b200
 
 using namespace b200;
@@ -232,6 +237,19 @@ B200_EXPORT int b200_moe_finalize(aiter_tensor_t* out, const aiter_tensor_t* acc
         B200_CHECK(acc != nullptr, "acc must not be NULL");
         DeviceGuard g(acc->device_id);
         launch_finalize(out, acc, (cudaStream_t)stream);
+    });
+}
+
+B200_EXPORT int64_t b200_fused_moe_workspace_size(int64_t M, int64_t H, int64_t I, int64_t global_E, int64_t topk,
+                                                  int quant_type, int hidden_dtype) {
+    return fused_moe_workspace_bytes(M, H, I, global_E, topk, quant_type, hidden_dtype);
+}
+
+B200_EXPORT int b200_fused_moe(const b200_fused_moe_args* args, void* stream) {
+    return safe_call([&] {
+        B200_CHECK(args != nullptr, "args must not be NULL");
+        DeviceGuard g((int)args->device);
+        launch_fused_moe(*args, (cudaStream_t)stream);
     });
 }
 

@@ -1,0 +1,136 @@
+// The layer as one host call (b200_fused_moe): the kernels of the separate entry points, enqueued back to back.
+//
+// What it is for: from Python every entry point costs 10-25 us of host time (argument marshalling, allocator, stream
+// lookup), and a decode layer's kernels are over in 50 us: at M=1 the eager layer took 177 us of which the GPU worked 56.
+
+#include "common.cuh"
+
+namespace b200 {
+
+int64_t sorting_workspace_bytes(int tokens, int num_experts, int topk);
+void launch_moe_sorting(const aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*, aiter_tensor_t*,
+                        aiter_tensor_t*, aiter_tensor_t*, aiter_tensor_t*, int, int, const aiter_tensor_t*,
+                        const aiter_tensor_t*, aiter_tensor_t*, aiter_tensor_t*, cudaStream_t);
+void launch_quant_1x128(aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*, const aiter_tensor_t*, int, int, cudaStream_t);
+void launch_quant_per_token(aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*, const aiter_tensor_t*, int, cudaStream_t);
+void launch_quant_per_tensor(aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*, aiter_tensor_t*, aiter_tensor_t*,
+                             const aiter_tensor_t*, cudaStream_t);
+void launch_moe_stage1(const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*,
+                       const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*,
+                       aiter_tensor_t*, aiter_tensor_t*, int, const aiter_tensor_t*, int, cudaStream_t);
+void launch_moe_stage2(const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*,
+                       const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*,
+                       aiter_tensor_t*, aiter_tensor_t*, int, int, int, int, int, cudaStream_t);
+void launch_finalize(aiter_tensor_t*, const aiter_tensor_t*, cudaStream_t);
+
+namespace {
+
+constexpr int kQuantPerTensor = 1, kQuantPerToken = 2;   // QuantType of the reference (csrc/include/aiter_enum.h:16-26)
+constexpr int64_t kUnit = 128;                           // sort unit == row tile of the GEMM kernels
+
+// Workspace map: every buffer starts on a 256-byte boundary. Offsets depend on sizes only.
+struct Layout {
+    int64_t P, sorted_ids, sorted_w, sorted_eids, num_valid, sort_ws, acc, a1, a1_scale, a2, a2_scale, a2_half, words, total;
+    Layout(int64_t M, int64_t H, int64_t I, int64_t E, int64_t topk, int qt, bool fp8_in) {
+        const bool rowwise = qt == kQuantPerToken || qt == kQuantPerTensor;
+        P = M * topk + E * kUnit - topk;
+        int64_t at = 0;
+        auto take = [&](int64_t bytes) {
+            const int64_t o = at;
+            at += (bytes + 255) / 256 * 256;
+            return o;
+        };
+        sorted_ids = take(P * 4);
+        sorted_w = take(P * 4);
+        sorted_eids = take((P + kUnit - 1) / kUnit * 4);
+        num_valid = take(8);
+        words = take(256);                       // per_Tensor: scale and maximum words
+        sort_ws = take(sorting_workspace_bytes((int)M, (int)E, (int)topk));
+        a1_scale = take(M * (rowwise ? 1 : H / 128) * 4);
+        a2_scale = take(P * (rowwise ? 1 : I / 128) * 4);
+        acc = take(M * H * 4);
+        a1 = take(fp8_in ? 0 : M * H);
+        a2 = take(P * I);
+        a2_half = take(rowwise ? P * I * 2 : 0);  // stage-1 activation before the row requantisation
+        total = at;
+    }
+};
+
+aiter_tensor_t tensor(const void* ptr, int dtype, int dev, int64_t d0, int64_t d1 = -1, int64_t d2 = -1) {
+    aiter_tensor_t t{};
+    t.ptr = const_cast<void*>(ptr);
+    t.dtype_ = dtype;
+    t.device_id = dev;
+    const int64_t d[3] = {d0, d1, d2};
+    t.ndim = d2 >= 0 ? 3 : d1 >= 0 ? 2 : 1;
+    int64_t n = 1;
+    for (int i = t.ndim - 1; i >= 0; --i) {
+        t.shape[i] = d[i];
+        t.strides[i] = n;
+        n *= d[i];
+    }
+    t.numel_ = (size_t)n;
+    return t;
+}
+
+}  // namespace
+
+int64_t fused_moe_workspace_bytes(int64_t M, int64_t H, int64_t I, int64_t E, int64_t topk, int qt, int hidden_dtype) {
+    return Layout(M, H, I, E, topk, qt, hidden_dtype == AITER_DTYPE_fp8).total;
+}
+
+void launch_fused_moe(const b200_fused_moe_args& a, cudaStream_t stream) {
+    const int dev = (int)a.device, qt = (int)a.quant_type;
+    const int64_t M = a.M, H = a.H, I = a.I, E = a.E;
+    const bool fp8_in = a.hidden_dtype == AITER_DTYPE_fp8;
+    const bool per_tensor = qt == kQuantPerTensor, rowwise = per_tensor || qt == kQuantPerToken;
+    B200_CHECK(M >= 1 && H >= 1 && I >= 1 && E >= 1 && a.topk >= 1, "sizes must be positive");
+    B200_CHECK(a.workspace != nullptr && ((uintptr_t)a.workspace & 255) == 0, "workspace must be 256-byte aligned");
+    const Layout at(M, H, I, a.global_E, a.topk, qt, fp8_in);
+    B200_CHECK(a.workspace_bytes >= at.total, "workspace needs ", at.total, " bytes, has ", a.workspace_bytes);
+    char* ws = (char*)a.workspace;
+    const int F32 = AITER_DTYPE_fp32, I32 = AITER_DTYPE_i32, FP8 = AITER_DTYPE_fp8;
+
+    aiter_tensor_t ids = tensor(a.topk_ids, I32, dev, M, a.topk), wts = tensor(a.topk_weight, F32, dev, M, a.topk);
+    aiter_tensor_t s_ids = tensor(ws + at.sorted_ids, I32, dev, at.P), s_w = tensor(ws + at.sorted_w, F32, dev, at.P);
+    aiter_tensor_t s_e = tensor(ws + at.sorted_eids, I32, dev, (at.P + kUnit - 1) / kUnit), nv = tensor(ws + at.num_valid, I32, dev, 2);
+    aiter_tensor_t acc = tensor(ws + at.acc, F32, dev, M, H), status = tensor(a.status, I32, dev, 1);
+    aiter_tensor_t mask = tensor(a.expert_mask, I32, dev, a.global_E), live = tensor(a.num_local_tokens, I32, dev, 1);
+    const int64_t sort_bytes = sorting_workspace_bytes((int)M, (int)a.global_E, (int)a.topk);
+    aiter_tensor_t sort_ws = tensor(ws + at.sort_ws, AITER_DTYPE_u8, dev, sort_bytes);
+    launch_moe_sorting(&ids, &wts, &s_ids, &s_w, &s_e, &nv, &acc, (int)a.global_E, (int)kUnit, a.expert_mask ? &mask : nullptr,
+                       a.num_local_tokens ? &live : nullptr, sort_bytes ? &sort_ws : nullptr, nullptr, stream);
+
+    aiter_tensor_t hidden = tensor(a.hidden, (int)a.hidden_dtype, dev, M, H);
+    aiter_tensor_t a1 = hidden, a1_s = rowwise ? tensor(ws + at.a1_scale, F32, dev, M) : tensor(ws + at.a1_scale, F32, dev, M, H / 128);
+    aiter_tensor_t one = tensor(ws + at.words, F32, dev, 1), amax = tensor(ws + at.words + 128, F32, dev, 1);
+    if (fp8_in) {
+        B200_CHECK(a.a1_scale != nullptr, "fp8 hidden states need a1_scale");
+        a1_s = tensor(a.a1_scale, F32, dev, a.a1_scale_numel);
+    } else {
+        a1 = tensor(ws + at.a1, FP8, dev, M, H);
+        if (per_tensor) launch_quant_per_tensor(&a1, &hidden, &one, &amax, nullptr, nullptr, stream), a1_s = one;
+        else if (rowwise) launch_quant_per_token(&a1, &hidden, &a1_s, nullptr, 1, stream);
+        else launch_quant_1x128(&a1, &hidden, &a1_s, nullptr, 1, 0, stream);
+    }
+
+    aiter_tensor_t w1 = tensor(a.w1, FP8, dev, E, 2 * I, H), w1_s = tensor(a.w1_scale, F32, dev, a.w1_scale_numel);
+    aiter_tensor_t w2 = tensor(a.w2, FP8, dev, E, H, I), w2_s = tensor(a.w2_scale, F32, dev, a.w2_scale_numel);
+    aiter_tensor_t a2 = tensor(ws + at.a2, FP8, dev, at.P, I);
+    aiter_tensor_t a2_s = rowwise ? tensor(ws + at.a2_scale, F32, dev, at.P) : tensor(ws + at.a2_scale, F32, dev, at.P, I / 128);
+    const int gemm_qt = rowwise ? kQuantPerToken : qt;   // one scale per tensor runs through the row-scale kernels
+    const aiter_tensor_t* w_stage1 = a.doweight_stage1 ? &s_w : nullptr;
+    if (rowwise) {
+        aiter_tensor_t half = tensor(ws + at.a2_half, AITER_DTYPE_bf16, dev, at.P, I);
+        launch_moe_stage1(&a1, &a1_s, &w1, &w1_s, &s_ids, &s_e, &nv, &half, nullptr, &status, gemm_qt, w_stage1, (int)a.activation, stream);
+        if (per_tensor) launch_quant_per_tensor(&a2, &half, &one, &amax, nullptr, &nv, stream), a2_s = one;
+        else launch_quant_per_token(&a2, &half, &a2_s, &nv, 1, stream);
+    } else {
+        launch_moe_stage1(&a1, &a1_s, &w1, &w1_s, &s_ids, &s_e, &nv, &a2, &a2_s, &status, gemm_qt, w_stage1, (int)a.activation, stream);
+    }
+    launch_moe_stage2(&a2, &a2_s, &w2, &w2_s, &s_ids, &s_w, &s_e, &nv, &acc, &status, 0, 0, 0, gemm_qt, a.doweight_stage1 ? 0 : 1, stream);
+    aiter_tensor_t out = tensor(a.out, (int)a.out_dtype, dev, M, H);
+    launch_finalize(&out, &acc, stream);
+}
+
+}  // namespace b200

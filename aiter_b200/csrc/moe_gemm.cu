@@ -80,8 +80,10 @@ constexpr int kSmemBytes = kSmemUsed + 1024;                // slack for the 102
 
 struct GemmParams {
     const uint8_t* a;        // stage 1: a1 [M,K] by token; stage 2: a2 [P,K] by sorted row
-    const float* a_scale;    // [rows, K/128]
-    const float* w_scale;    // [E, n_rows/128, K/128]
+    const float* a_scale;    // [rows, K/128]; PT: [rows], or [1] (a_scale_ld 0)
+    const float* w_scale;    // [E, n_rows/128, K/128]; PT: [E, n_rows], or [E] (w_scale_by_expert)
+    int a_scale_ld;          // scales per activation row: K/128; PT: 1, or 0 = one scale for all rows
+    int w_scale_by_expert;   // PT: one weight scale per expert instead of one per output channel
     const int* sorted_ids;
     const float* sorted_w;
     const int* sorted_eids;
@@ -375,7 +377,7 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const GemmParams p) 
             // shared memory issued after the UMMA's completion sits ~150 clocks (shared memory is saturated by
             // operand reads and fills) on the path to the first FMA.
             // (32-bit element offsets from the parameter pointers: two registers fewer than pointers)
-            const uint32_t a_so = (uint32_t)(valid ? (STAGE == 1 ? tok : prow) : 0) * (uint32_t)(PT ? 1 : p.KB);
+            const uint32_t a_so = (uint32_t)(valid ? (STAGE == 1 ? tok : prow) : 0) * (uint32_t)p.a_scale_ld;
             uint32_t w_so = 0, w_so1 = 0;
             if (!PT) {
                 const int nb0 = (STAGE == 1) ? nt : nt * 2;
@@ -384,6 +386,7 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const GemmParams p) 
                 w_so1 = w_so + (uint32_t)((nb1 - nb0) * p.KB);
             }
             float pf_a = __ldg(p.a_scale + a_so), pf_w0 = PT ? 1.f : __ldg(p.w_scale + w_so), pf_w1 = PT ? 1.f : __ldg(p.w_scale + w_so1);
+            if (PT && p.w_scale_by_expert) pf_a *= __ldg(p.w_scale + eid);   // per_Tensor: the expert's scale rides on the row scale
 
             // PT: one pass over the finished accumulators per tile (it counts tiles), else one per K block
             for (int kb = PT ? p.KB - 1 : 0; kb < p.KB; ++kb, ++it) {
@@ -424,7 +427,7 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const GemmParams p) 
             }
             if (!ok) break;
 
-            if (PT) {
+            if (PT && !p.w_scale_by_expert) {
                 // weight scales per output channel: column j of the first group is weight row
                 // e*n_rows + c0 + j, of the second group c1 + j (all lanes read the same addresses)
                 const int e = p.sorted_eids[blk];
@@ -682,8 +685,9 @@ void launch_moe_stage1(const aiter_tensor_t* a1, const aiter_tensor_t* a1_scale,
     B200_CHECK(H % 128 == 0, "model_dim must be a multiple of 128, got ", H);
     const int64_t I = N2 / 2;
     if (pt) {
-        B200_CHECK((int64_t)a1_scale->numel_ == M, "a1_scale must have one element per token for per_Token");
-        B200_CHECK((int64_t)w1_scale->numel_ == E * N2, "w1_scale must have E*2*inter_dim elements for per_Token");
+        B200_CHECK((int64_t)a1_scale->numel_ == M || a1_scale->numel_ == 1, "a1_scale must have one element per token for per_Token");
+        B200_CHECK((int64_t)w1_scale->numel_ == E * N2 || (int64_t)w1_scale->numel_ == E,
+                   "w1_scale must have E*2*inter_dim elements for per_Token (or one per expert)");
     } else {
         B200_CHECK((int64_t)a1_scale->numel_ == M * (H / 128), "a1_scale must have M*model_dim/128 elements");
         B200_CHECK((int64_t)w1_scale->numel_ == E * (N2 / 128) * (H / 128),
@@ -699,13 +703,15 @@ void launch_moe_stage1(const aiter_tensor_t* a1, const aiter_tensor_t* a1_scale,
                "sorted_expert_ids must hold one entry per 128 sorted rows (was the sort run with unit_size 128?)");
     B200_CHECK(E * N2 < ((int64_t)1 << 31) && M < (1 << 24), "problem too large");
     B200_CHECK(((uintptr_t)a1->ptr & 15) == 0 && ((uintptr_t)w1->ptr & 15) == 0 && ((uintptr_t)a2->ptr & 15) == 0 &&
-                   ((uintptr_t)w1_scale->ptr & 15) == 0,
+                   (((uintptr_t)w1_scale->ptr & 15) == 0 || (int64_t)w1_scale->numel_ == E),   // read one by one if per expert
                "a1, w1, w1_scale and a2 must be 16-byte aligned");
 
     GemmParams p{};
     p.a = (const uint8_t*)a1->ptr;
     p.a_scale = (const float*)a1_scale->ptr;
     p.w_scale = (const float*)w1_scale->ptr;
+    p.a_scale_ld = pt ? ((int64_t)a1_scale->numel_ == M ? 1 : 0) : (int)(H / 128);
+    p.w_scale_by_expert = pt && (int64_t)w1_scale->numel_ != E * N2;
     p.sorted_ids = (const int*)sorted_ids->ptr;
     p.sorted_eids = (const int*)sorted_eids->ptr;
     p.num_valid = (const int*)num_valid->ptr;
@@ -762,9 +768,10 @@ void launch_moe_stage2(const aiter_tensor_t* a2, const aiter_tensor_t* a2_scale,
     B200_CHECK(sm_margin >= 0, "sm_margin must not be negative");
     B200_CHECK(I % 128 == 0 && H % 128 == 0, "inter_dim and model_dim must be multiples of 128");
     if (pt) {
-        B200_CHECK((int64_t)a2_scale->numel_ >= P, "a2_scale must have one element per sorted row for per_Token");
-        B200_CHECK((int64_t)w2_scale->numel_ == E * H, "w2_scale must have E*model_dim elements for per_Token");
-        B200_CHECK(((uintptr_t)w2_scale->ptr & 15) == 0, "w2_scale must be 16-byte aligned");
+        B200_CHECK((int64_t)a2_scale->numel_ >= P || a2_scale->numel_ == 1, "a2_scale must have one element per sorted row for per_Token");
+        B200_CHECK((int64_t)w2_scale->numel_ == E * H || (int64_t)w2_scale->numel_ == E,
+                   "w2_scale must have E*model_dim elements for per_Token (or one per expert)");
+        B200_CHECK(((uintptr_t)w2_scale->ptr & 15) == 0 || (int64_t)w2_scale->numel_ == E, "w2_scale must be 16-byte aligned");
     } else {
         B200_CHECK((int64_t)a2_scale->numel_ >= P * (I / 128), "a2_scale must have P*inter_dim/128 elements");
         B200_CHECK((int64_t)w2_scale->numel_ == E * (H / 128) * (I / 128),
@@ -783,6 +790,8 @@ void launch_moe_stage2(const aiter_tensor_t* a2, const aiter_tensor_t* a2_scale,
     p.a = (const uint8_t*)a2->ptr;
     p.a_scale = (const float*)a2_scale->ptr;
     p.w_scale = (const float*)w2_scale->ptr;
+    p.a_scale_ld = pt ? ((int64_t)a2_scale->numel_ >= P ? 1 : 0) : (int)(I / 128);
+    p.w_scale_by_expert = pt && (int64_t)w2_scale->numel_ != E * H;
     p.sorted_ids = (const int*)sorted_ids->ptr;
     p.sorted_w = (const float*)sorted_w->ptr;
     p.sorted_eids = (const int*)sorted_eids->ptr;

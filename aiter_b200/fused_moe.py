@@ -10,7 +10,9 @@ tuned-config dispatch and no fallback: options outside the FP8 1x128 / 128x128 p
 
 from __future__ import annotations
 
+import functools
 import os
+import struct
 
 import torch
 
@@ -198,7 +200,6 @@ def get_hip_quant(qType):
     """aiter/ops/quant.py:367-387, restricted to the FP8 paths built here. Like the reference's table, the
     per_1x128 entry is ``per_group_quant_hip`` with group_size bound to 128, so callers can pass ``transpose_scale``,
     ``num_rows`` and ``num_rows_factor`` (aiter/fused_moe.py:1138-1147)."""
-    import functools
     qType = quant_remap.get(QuantType(qType), QuantType(qType))
     if qType == QuantType.per_Token:
         return per_token_quant_hip
@@ -319,7 +320,7 @@ def fused_moe_stages(hidden_states, w1, w2, topk_weight, topk_ids, expert_mask, 
     dw2 = 0 if doweight_stage1 else 1
     qt = int(QuantType.per_Token if per_token else QuantType.per_1x128)
     if hidden_states.dtype == dtypes.fp8:
-        a1, a1_s = hidden_states.contiguous(), a1_scale.contiguous().view(M, -1)
+        a1, a1_s = hidden_states.contiguous(), a1_scale.contiguous()
     elif per_tensor:
         a1, _scale, a1_s = _per_tensor_quant(hidden_states, want_row_scales=True)
     elif per_token:
@@ -393,6 +394,72 @@ def fused_moe_stages(hidden_states, w1, w2, topk_weight, topk_ids, expert_mask, 
     return out
 
 
+# b200_fused_moe_args of include/aiter_b200.h: 13 pointers, then the 16 integers
+_LAYER_ARGS = struct.Struct("@13P16q")
+
+
+@functools.lru_cache(maxsize=1024)
+def _layer_workspace_bytes(M, H, I, E, topk, qt, hidden_code):
+    return int(_lib.lib().b200_fused_moe_workspace_size(M, H, I, E, topk, qt, hidden_code))
+
+
+def _ptr(t):
+    return 0 if t is None else t.data_ptr()
+
+
+def _layer(hidden_states, w1, w2, topk_weight, topk_ids, expert_mask, w1_scale, w2_scale, a1_scale, num_local_tokens, dtype,
+           quant_type, activation, doweight_stage1):
+    """The layer through the one-call entry point: one workspace, one FFI crossing. Arguments as ``fused_moe`` checked
+    them; the tensors' sizes are checked natively. Same kernels and results as ``fused_moe_stages``, which remains for
+    callers that need the stages apart (event marks, column ranges, fp32 sums, intermediates)."""
+    device = hidden_states.device
+    index = hidden_states.get_device()
+    M, topk = topk_ids.shape
+    E, H, I = w2.shape
+    # the shapes of the optional and 2-D inputs; what is read by element count is checked on the other side
+    if topk_weight.shape != topk_ids.shape:
+        raise RuntimeError("topk_weights must have the [tokens, topk] shape of topk_ids")
+    for name, t, code in (("local_expert_mask", expert_mask, dtypes.i32), ("num_local_tokens", num_local_tokens, dtypes.i32),
+                          ("w1_scale", w1_scale, dtypes.fp32), ("w2_scale", w2_scale, dtypes.fp32), ("a1_scale", a1_scale, dtypes.fp32)):
+        if t is not None and (t.dtype != code or not t.is_cuda or t.numel() < 1):
+            raise RuntimeError(f"{name} must be a non-empty {code} CUDA tensor")
+    if not (w1.is_cuda and w2.is_cuda and topk_weight.is_cuda and topk_ids.is_cuda):
+        raise RuntimeError("fused_moe: tensors must live on a CUDA device (there is no CPU path)")
+    if w1.shape != (E, 2 * I, H):
+        raise RuntimeError(f"w1 must be [{E}, {2 * I}, {H}], got {tuple(w1.shape)}")
+    # contiguous() of a contiguous tensor is the tensor itself
+    hidden_states, topk_weight, topk_ids = hidden_states.contiguous(), topk_weight.contiguous(), topk_ids.contiguous()
+    w1, w2, w1_scale, w2_scale = w1.contiguous(), w2.contiguous(), w1_scale.contiguous(), w2_scale.contiguous()
+    if hidden_states.dtype != dtypes.fp8:
+        a1_scale = None
+    elif a1_scale is not None:
+        a1_scale = a1_scale.contiguous()
+    if expert_mask is not None:
+        expert_mask = expert_mask.contiguous()
+    global_E = E if expert_mask is None else expert_mask.numel()
+    code = dtypes.AITER_DTYPE[hidden_states.dtype]
+    nbytes = _layer_workspace_bytes(M, H, I, global_E, topk, int(quant_type), code)
+    workspace = torch.empty(nbytes, dtype=dtypes.u8, device=device)
+    out = torch.empty((M, H), dtype=dtype, device=device)
+    args = _LAYER_ARGS.pack(
+        hidden_states.data_ptr(), _ptr(a1_scale), w1.data_ptr(), w2.data_ptr(), w1_scale.data_ptr(), w2_scale.data_ptr(),
+        topk_weight.data_ptr(), topk_ids.data_ptr(), _ptr(expert_mask), _ptr(num_local_tokens), out.data_ptr(),
+        workspace.data_ptr(), _status(device).data_ptr(),
+        M, H, I, E, global_E, topk, 0 if a1_scale is None else a1_scale.numel(), w1_scale.numel(), w2_scale.numel(), nbytes,
+        code, dtypes.AITER_DTYPE[dtype], int(quant_type), int(activation), int(doweight_stage1), index)
+    if _lib._fn("b200_fused_moe")(args, _lib.current_stream(index)) != 0:
+        _lib.raise_last_error("b200_fused_moe")
+    _lib.launch_count += _layer_launches(M * topk, quant_type, code)
+    return out
+
+
+def _layer_launches(routes, quant_type, hidden_code):
+    """Kernels behind one layer call (for ``_lib.launch_count``): sort, quantiser, two GEMMs, requantiser, final rounding."""
+    quant = _lib._KERNELS_PER_CALL["b200_moe_quant_per_tensor"] if quant_type == QuantType.per_Tensor else 1
+    a1 = 0 if hidden_code == dtypes.AITER_DTYPE[dtypes.fp8] else quant
+    return (3 if routes > 16384 else 1) + a1 + (0 if quant_type == QuantType.per_1x128 else quant) + 3
+
+
 def fused_moe(
     hidden_states,
     w1,  # [expert(local_expert:EP), inter_dim*2, dim] N,K
@@ -452,11 +519,13 @@ def fused_moe(
             "QuantType.per_1x128 / per_128x128 (FP8 block scale), QuantType.per_Token and QuantType.per_Tensor (FP8)")
     if ActivationType(activation) not in (ActivationType.Silu, ActivationType.Gelu):
         raise NotImplementedError(f"fused_moe: activation={ActivationType(activation)!r} is not supported (Silu, Gelu)")
-    _check_unsupported(
-        a2_scale=(a2_scale, None),
-        hidden_pad=(hidden_pad, 0), intermediate_pad=(intermediate_pad, 0), bias1=(bias1, None),
-        bias2=(bias2, None), splitk=(splitk or 0, 0), swiglu_limit=(swiglu_limit, None),
-        beta=(beta, None), linear_beta=(linear_beta, None), stage2_scatter=(stage2_scatter, None))
+    if not (a2_scale is None and bias1 is None and bias2 is None and swiglu_limit is None and beta is None and linear_beta is None
+            and stage2_scatter is None and not hidden_pad and not intermediate_pad and not splitk):
+        _check_unsupported(
+            a2_scale=(a2_scale, None),
+            hidden_pad=(hidden_pad, 0), intermediate_pad=(intermediate_pad, 0), bias1=(bias1, None),
+            bias2=(bias2, None), splitk=(splitk or 0, 0), swiglu_limit=(swiglu_limit, None),
+            beta=(beta, None), linear_beta=(linear_beta, None), stage2_scatter=(stage2_scatter, None))
     if gate_mode not in (None, "separated"):
         raise NotImplementedError(f"fused_moe: gate_mode={gate_mode!r} is not supported (separated only)")
     if not hidden_states.is_cuda:
@@ -490,21 +559,23 @@ def fused_moe(
         raise ValueError("fused_moe: topk_weight must be float32")
     if topk_ids.dtype != dtypes.i32:
         raise ValueError("fused_moe: topk_ids must be int32")
-    if quant_type == QuantType.per_Tensor:
+    if quant_type == QuantType.per_Tensor:   # one scale per expert / per tensor, in fp32
+        w1_scale, w2_scale = w1_scale.to(dtypes.fp32).reshape(E, 1), w2_scale.to(dtypes.fp32).reshape(E, 1)
         if hidden_states.dtype == dtypes.fp8:
-            a1_scale = a1_scale.to(dtypes.fp32).reshape(-1)[:1].expand(M).contiguous()
-        # one scale per expert -> one per output channel, the layout the per_Token kernels read
-        w1_scale = w1_scale.to(dtypes.fp32).reshape(E, 1).expand(E, 2 * inter_dim)
-        w2_scale = w2_scale.to(dtypes.fp32).reshape(E, 1).expand(E, model_dim)
+            a1_scale = a1_scale.to(dtypes.fp32).reshape(-1)[:1]
     shared = (shared_w1, shared_w2, shared_w1_scale, shared_w2_scale)
     if any(t is not None for t in shared) or shared_expert_id != -1:
         _fold_shared_expert(w1, w2, w1_scale, w2_scale, shared, shared_expert_id, quant_type, expert_mask)
     if M == 0:   # nothing to compute: the reference allocates the same empty result (aiter/fused_moe.py:579-619)
         return torch.empty((0, model_dim), dtype=dtype, device=hidden_states.device)
-    out = fused_moe_stages(hidden_states, w1.contiguous(), w2.contiguous(), topk_weight, topk_ids,
-                           expert_mask, w1_scale.contiguous(), w2_scale.contiguous(), a1_scale,
-                           num_local_tokens, dtype, quant_type=quant_type, activation=activation,
-                           doweight_stage1=bool(doweight_stage1))
+    if kernel_bench_events is None:
+        out = _layer(hidden_states, w1, w2, topk_weight, topk_ids, expert_mask, w1_scale, w2_scale, a1_scale, num_local_tokens,
+                     dtype, quant_type, activation, bool(doweight_stage1))
+    else:   # event marks between the kernels
+        out = fused_moe_stages(hidden_states, w1.contiguous(), w2.contiguous(), topk_weight, topk_ids,
+                               expert_mask, w1_scale.contiguous(), w2_scale.contiguous(), a1_scale,
+                               num_local_tokens, dtype, quant_type=quant_type, activation=activation,
+                               doweight_stage1=bool(doweight_stage1))
     if _CHECK_STATUS_EVERY_CALL:
         check_device_status(hidden_states.device)
     return out

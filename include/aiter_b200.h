@@ -133,6 +133,33 @@ int b200_moe_quant_per_tensor(aiter_tensor_t* out, const aiter_tensor_t* input, 
                               aiter_tensor_t* amax, aiter_tensor_t* row_scales, const aiter_tensor_t* row_limit,
                               void* stream);
 
+/* The whole layer of aiter.fused_moe in one call: sort -> activation quantisation -> stage 1 -> (row requantisation)
+ * -> stage 2 -> final rounding, enqueued on one stream from one host call. Same kernels and results as the separate
+ * entry points below; a caller pays one FFI crossing and one workspace instead of six calls and a dozen buffers.
+ * All pointers are device pointers on `device` (16-byte aligned), all tensors contiguous; optional ones are NULL. */
+typedef struct b200_fused_moe_args {
+    const void* hidden;            /* [M,H] bf16 | fp16 | fp8 (hidden_dtype) */
+    const void* a1_scale;          /* fp32, with fp8 hidden: [M,H/128], [M] (per_Token) or [1] (per_Tensor) */
+    const void* w1;                /* [E,2I,H] fp8 */
+    const void* w2;                /* [E,H,I] fp8 */
+    const void* w1_scale;          /* fp32, w1_scale_numel elements */
+    const void* w2_scale;          /* fp32, w2_scale_numel elements */
+    const void* topk_weight;       /* [M,topk] fp32 */
+    const void* topk_ids;          /* [M,topk] i32 */
+    const void* expert_mask;       /* optional [global_E] i32 */
+    const void* num_local_tokens;  /* optional [1] i32 */
+    void* out;                     /* [M,H] bf16 | fp16 (out_dtype) */
+    void* workspace;               /* b200_fused_moe_workspace_size bytes, 256-byte aligned */
+    void* status;                  /* [1] i32 */
+    int64_t M, H, I, E, global_E, topk;
+    int64_t a1_scale_numel, w1_scale_numel, w2_scale_numel, workspace_bytes;
+    int64_t hidden_dtype, out_dtype, quant_type, activation, doweight_stage1, device;
+} b200_fused_moe_args;
+
+int64_t b200_fused_moe_workspace_size(int64_t M, int64_t H, int64_t I, int64_t global_E, int64_t topk, int quant_type,
+                                      int hidden_dtype);
+int b200_fused_moe(const b200_fused_moe_args* args, void* stream);
+
 /* Stage 1: grouped gate/up GEMM over the sorted blocks + SiLU(gate)*up + bf16 rounding +
  * 1x128 FP8 requantisation.  Replaces ck_moe_stage1 followed by the a2 quant
  * (csrc/ck_gemm_moe_2stages_codegen/gemm_moe_ck2stages.cu:68-137, aiter/fused_moe.py:3220-3336).
