@@ -8,8 +8,12 @@
 //   topk_softmax         fp32 softmax, top-k, optional renormalisation (aiter/fused_moe.py:4058-4129,
 //                        csrc/kernels/topk_softmax_kernels.cu:769).
 //
-// Expert e sits in lane e % 32, register e / 32.  Selections are repeated warp arg-max reductions
-// (value, then lower index on ties), so the result does not depend on scheduling.
+// What bounds them: the latency of one token's chain of warp-wide reductions (a token's scores are 1-2 KB, a batch of
+// 8192 fits the warps of one wave). So every reduction is one redux.sync on order-preserving integer keys instead of
+// five (value, index) shuffle rounds, and the grouped router keeps a lane's experts contiguous, so that a routing group
+// is a run of lanes and all groups are reduced at once. DeepSeek-V3 routing (E=256, 8 groups, top 8): 31 -> 4.6 us at 64
+// tokens, 95 -> 17 us at 8192; the first version tested e / group_size against each group in turn.
+// Selections break ties by the lower index, so the result does not depend on scheduling.
 
 #include <cuda_bf16.h>
 #include <math_constants.h>
@@ -21,7 +25,7 @@
 namespace b200 {
 namespace {
 
-constexpr int kWarpsPerBlock = 8;
+constexpr int kWarpsPerBlock = 4;
 #define kNegInf (-CUDART_INF_F)
 
 template <typename T>
@@ -33,54 +37,80 @@ __device__ __forceinline__ float load_f<__nv_bfloat16>(const __nv_bfloat16* p, i
     return __bfloat162float(p[i]);
 }
 
-// warp arg-max over (value, index): larger value wins, lower index on ties. All lanes get the result.
-__device__ __forceinline__ void warp_argmax(float& v, int& idx) {
+// VPL consecutive entries from index i on, those at or past n as 0. One 16-byte (fp32) or 8-byte (bf16) load per four
+// entries where the rows keep that alignment (n a multiple of 4).
+template <int VPL, typename T>
+__device__ __forceinline__ void load_run(const T* row, int i, int n, bool aligned, float (&v)[VPL]) {
+    if (VPL >= 4 && aligned) {
 #pragma unroll
-    for (int d = 16; d >= 1; d >>= 1) {
-        const float ov = __shfl_xor_sync(0xffffffffu, v, d);
-        const int oi = __shfl_xor_sync(0xffffffffu, idx, d);
-        if (ov > v || (ov == v && oi < idx)) {
-            v = ov;
-            idx = oi;
+        for (int j = 0; j < VPL; j += 4) {
+            float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (i + j < n) {
+                if constexpr (std::is_same<T, float>::value) {
+                    f = __ldg(reinterpret_cast<const float4*>(row + i + j));
+                } else {
+                    const uint2 raw = __ldg(reinterpret_cast<const uint2*>(row + i + j));
+                    const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
+                    const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+                    f = make_float4(lo.x, lo.y, hi.x, hi.y);
+                }
+            }
+            v[j] = f.x;
+            if (j + 1 < VPL) v[j + 1] = f.y;
+            if (j + 2 < VPL) v[j + 2] = f.z;
+            if (j + 3 < VPL) v[j + 3] = f.w;
         }
+    } else {
+#pragma unroll
+        for (int j = 0; j < VPL; ++j) v[j] = (i + j < n) ? load_f<T>(row, i + j) : 0.f;
     }
 }
 
-// Picks the k best of val[] (expert e = j*32 + lane) one at a time; lane i < k keeps pick i in (my_id, my_w),
-// where the weight is taken from wsrc[] of the winning expert. Returns the sum of the k weights.
-template <int VPL>
-__device__ __forceinline__ float select_topk(float (&val)[VPL], const float (&wsrc)[VPL], int k, int lane,
+// Unsigned key with the order of the floats (-0 and +0 equal). NaN gets the lowest key: it is never preferred.
+__device__ __forceinline__ uint32_t order_key(float v) {
+    const uint32_t u = __float_as_uint(v + 0.f);
+    return v != v ? 0u : ((u & 0x80000000u) ? ~u : (u | 0x80000000u));
+}
+
+// Picks the k largest of key[] (value, then lower index) one at a time; entry j of a lane is expert index(j), ascending in
+// j; key 0 = not there or already taken. Lane i < k keeps pick i in (my_id, my_w), with the weight wsrc[] of the winning
+// expert. Returns the sum of the k weights, added in the order of the picks.
+template <int VPL, typename Index>
+__device__ __forceinline__ float select_topk(uint32_t (&key)[VPL], const float (&wsrc)[VPL], int k, int lane, Index index,
                                              int& my_id, float& my_w) {
     float wsum = 0.f;
     for (int i = 0; i < k; ++i) {
-        float best = kNegInf;
-        int bidx = 0x7fffffff;
+        uint32_t best = key[0];
 #pragma unroll
-        for (int j = 0; j < VPL; ++j) {
-            const int e = j * 32 + lane;
-            if (val[j] > best || (val[j] == best && e < bidx)) {
-                best = val[j];
-                bidx = e;
-            }
-        }
-        warp_argmax(best, bidx);
-        // the owner of the winner publishes its weight and retires the entry
+        for (int j = 1; j < VPL; ++j) best = max(best, key[j]);
+        best = __reduce_max_sync(0xffffffffu, best);
+        int mine = 0x7fffffff;
         float w = 0.f;
 #pragma unroll
-        for (int j = 0; j < VPL; ++j) {
-            if (j * 32 + lane == bidx) {
+        for (int j = VPL - 1; j >= 0; --j)
+            if (key[j] == best) {
+                mine = index(j);
                 w = wsrc[j];
-                val[j] = kNegInf;
             }
-        }
-        w = __shfl_sync(0xffffffffu, w, bidx & 31);
+        const int win = __reduce_min_sync(0xffffffffu, mine);
+        const unsigned owner = __ballot_sync(0xffffffffu, mine == win);
+        w = __shfl_sync(0xffffffffu, w, __ffs(owner) - 1);
+#pragma unroll
+        for (int j = 0; j < VPL; ++j)
+            if (index(j) == win) key[j] = 0u;   // retired
         wsum += w;
         if (lane == i) {
-            my_id = bidx;
+            my_id = win;
             my_w = w;
         }
     }
     return wsum;
+}
+
+// Two largest of a run of values and of a second such pair
+__device__ __forceinline__ void merge_top2(float& b1, float& b2, float o1, float o2) {
+    b2 = fmaxf(fminf(b1, o1), fmaxf(b2, o2));
+    b1 = fmaxf(b1, o1);
 }
 
 template <typename TG, typename TB, int VPL>
@@ -91,64 +121,64 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) biased_grouped_topk_kerne
     const int token = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
     if (token >= tokens) return;
     const int gsize = E / n_group;
+    const int e0 = lane * VPL;      // this lane's experts: e0 .. e0 + VPL - 1
     float score[VPL], choice[VPL];
+    load_run<VPL>(gating + (int64_t)token * E, e0, E, E % 4 == 0 && ((uintptr_t)gating & 15) == 0, score);
+    load_run<VPL>(bias, e0, E, E % 4 == 0 && ((uintptr_t)bias & 15) == 0, choice);
 #pragma unroll
     for (int j = 0; j < VPL; ++j) {
-        const int e = j * 32 + lane;
-        if (e < E) {
-            const float x = load_f<TG>(gating, (int64_t)token * E + e);
-            score[j] = __fdiv_rn(1.0f, 1.0f + expf(-x));
-            choice[j] = score[j] + load_f<TB>(bias, e);
-        } else {
-            score[j] = 0.f;
-            choice[j] = kNegInf;
-        }
+        const bool there = e0 + j < E;
+        score[j] = there ? __fdiv_rn(1.0f, 1.0f + expf(-score[j])) : 0.f;
+        choice[j] = there ? score[j] + choice[j] : kNegInf;
     }
-    // group score = sum of the two largest biased scores of the group
-    unsigned keep = 0;   // bit g: group g is kept (n_group <= 32)
-    float gscore_mine = kNegInf;   // lane g holds the score of group g
-    for (int g = 0; g < n_group; ++g) {
-        float b1 = kNegInf;
-        int i1 = 0x7fffffff;
+    // group score = sum of the two largest biased scores of the group; kept = the group is among the topk_group best
+    uint32_t kept = 0;   // bit j: the group of expert e0 + j is kept
+    const int span = gsize / VPL;   // lanes per group
+    if (gsize % VPL == 0 && (span & (span - 1)) == 0) {
+        // a group is a power-of-two run of lanes: all groups at once in log2(span) butterfly rounds
+        float b1 = choice[0], b2 = kNegInf;
 #pragma unroll
-        for (int j = 0; j < VPL; ++j) {
-            const int e = j * 32 + lane;
-            if (e < E && e / gsize == g && (choice[j] > b1 || (choice[j] == b1 && e < i1))) {
-                b1 = choice[j];
-                i1 = e;
-            }
-        }
-        warp_argmax(b1, i1);
-        float b2 = kNegInf;
-        int i2 = 0x7fffffff;
-#pragma unroll
-        for (int j = 0; j < VPL; ++j) {
-            const int e = j * 32 + lane;
-            if (e < E && e / gsize == g && e != i1 && (choice[j] > b2 || (choice[j] == b2 && e < i2))) {
-                b2 = choice[j];
-                i2 = e;
-            }
-        }
-        warp_argmax(b2, i2);
+        for (int j = 1; j < VPL; ++j) merge_top2(b1, b2, choice[j], kNegInf);
+        for (int d = 1; d < span; d <<= 1)
+            merge_top2(b1, b2, __shfl_xor_sync(0xffffffffu, b1, d), __shfl_xor_sync(0xffffffffu, b2, d));
         const float gs = (gsize >= 2) ? b1 + b2 : b1;
-        if (lane == g) gscore_mine = gs;
-    }
-    for (int i = 0; i < topk_group; ++i) {
-        float v = (lane < n_group && !((keep >> lane) & 1u)) ? gscore_mine : kNegInf;
-        int idx = lane;
-        warp_argmax(v, idx);
-        keep |= 1u << idx;
+        const int mine = lane / span;
+        int better = 0;
+        for (int g = 0; g < n_group; ++g) {
+            const float o = __shfl_sync(0xffffffffu, gs, g * span);
+            better += (o > gs || (o == gs && g < mine)) ? 1 : 0;
+        }
+        kept = better < topk_group ? 0xffffffffu : 0u;
+    } else {
+        // any other group size: one group at a time
+        float gs_mine = kNegInf;   // lane g holds the score of group g (n_group <= 32)
+        for (int g = 0; g < n_group; ++g) {
+            float b1 = kNegInf, b2 = kNegInf;
+#pragma unroll
+            for (int j = 0; j < VPL; ++j)
+                if (e0 + j >= g * gsize && e0 + j < (g + 1) * gsize) merge_top2(b1, b2, choice[j], kNegInf);
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1)
+                merge_top2(b1, b2, __shfl_xor_sync(0xffffffffu, b1, d), __shfl_xor_sync(0xffffffffu, b2, d));
+            if (lane == g) gs_mine = (gsize >= 2) ? b1 + b2 : b1;
+        }
+        int better = 0;
+        for (int g = 0; g < n_group; ++g) {
+            const float o = __shfl_sync(0xffffffffu, gs_mine, g);
+            better += (o > gs_mine || (o == gs_mine && g < lane)) ? 1 : 0;
+        }
+        const unsigned groups = __ballot_sync(0xffffffffu, lane < n_group && better < topk_group);
+#pragma unroll
+        for (int j = 0; j < VPL; ++j)
+            if (e0 + j < E) kept |= ((groups >> ((e0 + j) / gsize)) & 1u) << j;
     }
     // experts of dropped groups compete with the value 0.0, as masked_fill(~mask, 0.0) does
-    float cand[VPL];
+    uint32_t key[VPL];
 #pragma unroll
-    for (int j = 0; j < VPL; ++j) {
-        const int e = j * 32 + lane;
-        cand[j] = (e < E) ? (((keep >> (e / gsize)) & 1u) ? choice[j] : 0.0f) : kNegInf;
-    }
+    for (int j = 0; j < VPL; ++j) key[j] = (e0 + j < E) ? order_key(((kept >> j) & 1u) ? choice[j] : 0.0f) : 0u;
     int my_id = 0;
     float my_w = 0.f;
-    const float wsum = select_topk<VPL>(cand, score, topk, lane, my_id, my_w);
+    const float wsum = select_topk<VPL>(key, score, topk, lane, [&](int j) { return e0 + j; }, my_id, my_w);
     if (lane < topk) {
         float w = renorm ? __fdiv_rn(my_w, wsum) : my_w;
         out_w[(int64_t)token * topk + lane] = w * scale;
@@ -163,7 +193,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) topk_softmax_kernel(
     const int lane = threadIdx.x & 31;
     const int token = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
     if (token >= tokens) return;
-    float x[VPL], prob[VPL];
+    float x[VPL], prob[VPL];   // entry j of a lane is expert j * 32 + lane
     float mx = kNegInf;
 #pragma unroll
     for (int j = 0; j < VPL; ++j) {
@@ -181,14 +211,15 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) topk_softmax_kernel(
     }
 #pragma unroll
     for (int d = 16; d >= 1; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+    uint32_t key[VPL];
 #pragma unroll
     for (int j = 0; j < VPL; ++j) {
         prob[j] = __fdiv_rn(prob[j], sum);
-        x[j] = (j * 32 + lane < E) ? prob[j] : kNegInf;   // selection keys
+        key[j] = (j * 32 + lane < E) ? order_key(prob[j]) : 0u;
     }
     int my_id = 0;
     float my_w = 0.f;
-    const float wsum = select_topk<VPL>(x, prob, topk, lane, my_id, my_w);
+    const float wsum = select_topk<VPL>(key, prob, topk, lane, [&](int j) { return j * 32 + lane; }, my_id, my_w);
     if (lane < topk) {
         out_w[(int64_t)token * topk + lane] = renorm ? __fdiv_rn(my_w, wsum) : my_w;
         out_id[(int64_t)token * topk + lane] = my_id;
