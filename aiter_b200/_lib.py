@@ -67,7 +67,7 @@ _SIGNATURES = {
 
 _lib = None
 
-# Kernel launches behind one call of an entry point (the sort takes three kernels above 16384 routes, one below;
+# Kernel launches behind one call of an entry point (the sort takes two kernels above 16384 routes, one below;
 # the per-tensor quantiser two). ``launch_count`` adds them up for callers that report how many kernels they ran.
 _KERNELS_PER_CALL = {"b200_moe_quant_per_tensor": 2}
 launch_count = 0
@@ -180,7 +180,7 @@ def call(name: str, *args, device: torch.device | None = None):
     stream = current_stream(torch.cuda.current_device() if index is None else index)
     global launch_count
     if name == "b200_moe_sorting_fwd":
-        launch_count += 3 if args[0].numel() > 16384 else 1
+        launch_count += 2 if args[0].numel() > 16384 else 1
     else:
         launch_count += _KERNELS_PER_CALL.get(name, 1)
     if _fn(name)(*cargs, stream) != 0:

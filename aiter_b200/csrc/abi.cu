@@ -21,10 +21,10 @@ void launch_moe_sorting(const aiter_tensor_t*, const aiter_tensor_t*, aiter_tens
 void launch_moe_sorting_noalloc(const aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*, aiter_tensor_t*,
                                 aiter_tensor_t*, aiter_tensor_t*, aiter_tensor_t*, int, int, const aiter_tensor_t*,
                                 const aiter_tensor_t*, aiter_tensor_t*, cudaStream_t);
-void launch_quant_1x128(aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*, const aiter_tensor_t*, int, int, cudaStream_t);
-void launch_quant_per_token(aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*, const aiter_tensor_t*, int, cudaStream_t);
+void launch_quant_1x128(aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*, const aiter_tensor_t*, int, int, bool, cudaStream_t);
+void launch_quant_per_token(aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*, const aiter_tensor_t*, int, bool, cudaStream_t);
 void launch_quant_per_tensor(aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*, aiter_tensor_t*, aiter_tensor_t*,
-                             const aiter_tensor_t*, cudaStream_t);
+                             const aiter_tensor_t*, bool, cudaStream_t);
 void launch_moe_stage1(const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*,
                        const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*,
                        aiter_tensor_t*, aiter_tensor_t*, int, const aiter_tensor_t*, int, cudaStream_t);
@@ -57,10 +57,11 @@ namespace {
 
 // out = RNE(acc): 8 fp32 in, 8 half-precision values out per thread.
 template <typename T2>
-__global__ void __launch_bounds__(256) finalize_kernel(const float4* __restrict__ acc, uint4* __restrict__ out,
-                                                       int64_t n8) {
+__global__ void __launch_bounds__(256) finalize_kernel(const float4* acc, uint4* out, int64_t n8) {
+    pdl_wait();
+    pdl_trigger();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += (int64_t)gridDim.x * blockDim.x) {
-        const float4 a = __ldcs(acc + 2 * i), b = __ldcs(acc + 2 * i + 1);
+        const float4 a = acc[2 * i], b = acc[2 * i + 1];
         uint4 o;
         if constexpr (sizeof(T2) == sizeof(__nv_bfloat162) && std::is_same<T2, __nv_bfloat162>::value) {
             __nv_bfloat162 p0 = __floats2bfloat162_rn(a.x, a.y), p1 = __floats2bfloat162_rn(a.z, a.w);
@@ -91,10 +92,9 @@ void launch_finalize(aiter_tensor_t* out, const aiter_tensor_t* acc, cudaStream_
     const int64_t cap = (int64_t)sm_count(acc->device_id) * 8;
     if (blocks > cap) blocks = cap;
     if (out->dtype_ == AITER_DTYPE_bf16)
-        finalize_kernel<__nv_bfloat162><<<(unsigned)blocks, 256, 0, stream>>>((const float4*)acc->ptr, (uint4*)out->ptr, n8);
+        launch_pdl(finalize_kernel<__nv_bfloat162>, (unsigned)blocks, 256, 0, stream, (const float4*)acc->ptr, (uint4*)out->ptr, n8);
     else
-        finalize_kernel<__half2><<<(unsigned)blocks, 256, 0, stream>>>((const float4*)acc->ptr, (uint4*)out->ptr, n8);
-    B200_CUDA(cudaGetLastError());
+        launch_pdl(finalize_kernel<__half2>, (unsigned)blocks, 256, 0, stream, (const float4*)acc->ptr, (uint4*)out->ptr, n8);
 }
 
 }  // namespace b200
@@ -163,7 +163,7 @@ B200_EXPORT int b200_moe_quant_1x128(aiter_tensor_t* out, const aiter_tensor_t* 
     return safe_call([&] {
         B200_CHECK(input != nullptr, "input must not be NULL");
         DeviceGuard g(input->device_id);
-        launch_quant_1x128(out, input, scales, num_rows, num_rows_factor, transpose_scale, (cudaStream_t)stream);
+        launch_quant_1x128(out, input, scales, num_rows, num_rows_factor, transpose_scale, true, (cudaStream_t)stream);
     });
 }
 
@@ -172,7 +172,7 @@ B200_EXPORT int b200_moe_quant_per_token(aiter_tensor_t* out, const aiter_tensor
     return safe_call([&] {
         B200_CHECK(input != nullptr, "input must not be NULL");
         DeviceGuard g(input->device_id);
-        launch_quant_per_token(out, input, scales, num_rows, num_rows_factor, (cudaStream_t)stream);
+        launch_quant_per_token(out, input, scales, num_rows, num_rows_factor, true, (cudaStream_t)stream);
     });
 }
 
@@ -259,7 +259,7 @@ B200_EXPORT int b200_moe_quant_per_tensor(aiter_tensor_t* out, const aiter_tenso
     return safe_call([&] {
         B200_CHECK(input != nullptr, "input must not be NULL");
         DeviceGuard g(input->device_id);
-        launch_quant_per_tensor(out, input, scale, amax, row_scales, row_limit, (cudaStream_t)stream);
+        launch_quant_per_tensor(out, input, scale, amax, row_scales, row_limit, false, (cudaStream_t)stream);
     });
 }
 

@@ -7,6 +7,7 @@
 #include <sstream>
 #include <stdexcept>
 #include <string>
+#include <utility>
 
 #include "../../include/aiter_b200.h"
 
@@ -72,6 +73,36 @@ inline void check_tensor(const aiter_tensor_t* t, const char* name, int dtype, i
     B200_CHECK(is_contiguous(t), name, " must be contiguous");
     B200_CHECK(t->numel_ == 0 || t->ptr != nullptr, name, ": NULL data pointer");
 }
+
+// Programmatic dependent launch: the grid may be placed while its predecessor on the stream still runs; the kernel calls
+// pdl_wait() before it touches anything an earlier kernel wrote or reads. Convention of this library: a kernel triggers
+// its successor (pdl_trigger) only after its own pdl_wait() in at least one CTA, so when a kernel starts, everything up to
+// the predecessor of its predecessor is complete; and every kernel calls pdl_wait() somewhere, so a grid's completion
+// implies the completion of all before it. Saves the 1-2 us between two dependent short kernels and hides their start-up.
+template <typename... Params, typename... Args>
+inline void launch_kernel(bool overlap, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                          Args&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = overlap ? 1 : 0;
+    B200_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...));
+}
+template <typename... Params, typename... Args>
+inline void launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+    launch_kernel(true, kernel, grid, block, smem, stream, std::forward<Args>(args)...);
+}
+
+#ifdef __CUDACC__
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+#endif
 
 struct DeviceGuard {
     int prev = -1;

@@ -11,10 +11,10 @@ int64_t sorting_workspace_bytes(int tokens, int num_experts, int topk);
 void launch_moe_sorting(const aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*, aiter_tensor_t*,
                         aiter_tensor_t*, aiter_tensor_t*, aiter_tensor_t*, int, int, const aiter_tensor_t*,
                         const aiter_tensor_t*, aiter_tensor_t*, aiter_tensor_t*, cudaStream_t);
-void launch_quant_1x128(aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*, const aiter_tensor_t*, int, int, cudaStream_t);
-void launch_quant_per_token(aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*, const aiter_tensor_t*, int, cudaStream_t);
+void launch_quant_1x128(aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*, const aiter_tensor_t*, int, int, bool, cudaStream_t);
+void launch_quant_per_token(aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*, const aiter_tensor_t*, int, bool, cudaStream_t);
 void launch_quant_per_tensor(aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*, aiter_tensor_t*, aiter_tensor_t*,
-                             const aiter_tensor_t*, cudaStream_t);
+                             const aiter_tensor_t*, bool, cudaStream_t);
 void launch_moe_stage1(const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*,
                        const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*,
                        aiter_tensor_t*, aiter_tensor_t*, int, const aiter_tensor_t*, int, cudaStream_t);
@@ -44,10 +44,10 @@ struct Layout {
         sorted_w = take(P * 4);
         sorted_eids = take((P + kUnit - 1) / kUnit * 4);
         num_valid = take(8);
-        words = take(256);                       // per_Tensor: scale and maximum words
         sort_ws = take(sorting_workspace_bytes((int)M, (int)E, (int)topk));
         a1_scale = take(M * (rowwise ? 1 : H / 128) * 4);
         a2_scale = take(P * (rowwise ? 1 : I / 128) * 4);
+        words = take(256);                       // per_Tensor: a maximum and a scale word per quantisation
         acc = take(M * H * 4);
         a1 = take(fp8_in ? 0 : M * H);
         a2 = take(P * I);
@@ -94,24 +94,27 @@ void launch_fused_moe(const b200_fused_moe_args& a, cudaStream_t stream) {
     aiter_tensor_t ids = tensor(a.topk_ids, I32, dev, M, a.topk), wts = tensor(a.topk_weight, F32, dev, M, a.topk);
     aiter_tensor_t s_ids = tensor(ws + at.sorted_ids, I32, dev, at.P), s_w = tensor(ws + at.sorted_w, F32, dev, at.P);
     aiter_tensor_t s_e = tensor(ws + at.sorted_eids, I32, dev, (at.P + kUnit - 1) / kUnit), nv = tensor(ws + at.num_valid, I32, dev, 2);
-    aiter_tensor_t acc = tensor(ws + at.acc, F32, dev, M, H), status = tensor(a.status, I32, dev, 1);
+    aiter_tensor_t acc = tensor(ws + at.acc, F32, dev, M, H),
+                   cleared = tensor(ws + at.words, F32, dev, 64 + M * H), status = tensor(a.status, I32, dev, 1);
     aiter_tensor_t mask = tensor(a.expert_mask, I32, dev, a.global_E), live = tensor(a.num_local_tokens, I32, dev, 1);
     const int64_t sort_bytes = sorting_workspace_bytes((int)M, (int)a.global_E, (int)a.topk);
     aiter_tensor_t sort_ws = tensor(ws + at.sort_ws, AITER_DTYPE_u8, dev, sort_bytes);
-    launch_moe_sorting(&ids, &wts, &s_ids, &s_w, &s_e, &nv, &acc, (int)a.global_E, (int)kUnit, a.expert_mask ? &mask : nullptr,
+    launch_moe_sorting(&ids, &wts, &s_ids, &s_w, &s_e, &nv, &cleared, (int)a.global_E, (int)kUnit, a.expert_mask ? &mask : nullptr,
                        a.num_local_tokens ? &live : nullptr, sort_bytes ? &sort_ws : nullptr, nullptr, stream);
 
     aiter_tensor_t hidden = tensor(a.hidden, (int)a.hidden_dtype, dev, M, H);
     aiter_tensor_t a1 = hidden, a1_s = rowwise ? tensor(ws + at.a1_scale, F32, dev, M) : tensor(ws + at.a1_scale, F32, dev, M, H / 128);
-    aiter_tensor_t one = tensor(ws + at.words, F32, dev, 1), amax = tensor(ws + at.words + 128, F32, dev, 1);
+    // the sort clears the accumulator and the words in front of it; the quantiser runs beside the sort
+    aiter_tensor_t one = tensor(ws + at.words, F32, dev, 1), amax = tensor(ws + at.words + 64, F32, dev, 1);
+    aiter_tensor_t one2 = tensor(ws + at.words + 128, F32, dev, 1), amax2 = tensor(ws + at.words + 192, F32, dev, 1);
     if (fp8_in) {
         B200_CHECK(a.a1_scale != nullptr, "fp8 hidden states need a1_scale");
         a1_s = tensor(a.a1_scale, F32, dev, a.a1_scale_numel);
     } else {
         a1 = tensor(ws + at.a1, FP8, dev, M, H);
-        if (per_tensor) launch_quant_per_tensor(&a1, &hidden, &one, &amax, nullptr, nullptr, stream), a1_s = one;
-        else if (rowwise) launch_quant_per_token(&a1, &hidden, &a1_s, nullptr, 1, stream);
-        else launch_quant_1x128(&a1, &hidden, &a1_s, nullptr, 1, 0, stream);
+        if (per_tensor) launch_quant_per_tensor(&a1, &hidden, &one, &amax, nullptr, nullptr, true, stream), a1_s = one;
+        else if (rowwise) launch_quant_per_token(&a1, &hidden, &a1_s, nullptr, 1, false, stream);
+        else launch_quant_1x128(&a1, &hidden, &a1_s, nullptr, 1, 0, false, stream);
     }
 
     aiter_tensor_t w1 = tensor(a.w1, FP8, dev, E, 2 * I, H), w1_s = tensor(a.w1_scale, F32, dev, a.w1_scale_numel);
@@ -123,8 +126,8 @@ void launch_fused_moe(const b200_fused_moe_args& a, cudaStream_t stream) {
     if (rowwise) {
         aiter_tensor_t half = tensor(ws + at.a2_half, AITER_DTYPE_bf16, dev, at.P, I);
         launch_moe_stage1(&a1, &a1_s, &w1, &w1_s, &s_ids, &s_e, &nv, &half, nullptr, &status, gemm_qt, w_stage1, (int)a.activation, stream);
-        if (per_tensor) launch_quant_per_tensor(&a2, &half, &one, &amax, nullptr, &nv, stream), a2_s = one;
-        else launch_quant_per_token(&a2, &half, &a2_s, &nv, 1, stream);
+        if (per_tensor) launch_quant_per_tensor(&a2, &half, &one2, &amax2, nullptr, &nv, true, stream), a2_s = one2;
+        else launch_quant_per_token(&a2, &half, &a2_s, &nv, 1, true, stream);
     } else {
         launch_moe_stage1(&a1, &a1_s, &w1, &w1_s, &s_ids, &s_e, &nv, &a2, &a2_s, &status, gemm_qt, w_stage1, (int)a.activation, stream);
     }

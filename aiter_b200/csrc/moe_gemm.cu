@@ -31,6 +31,7 @@
 #include <cuda_bf16.h>
 
 #include "common.cuh"
+#include "quant_device.cuh"
 #include "sm100_ptx.cuh"
 
 namespace b200 {
@@ -143,14 +144,6 @@ __device__ __forceinline__ void act_mul_n(const float (&g)[N], const float (&u)[
     }
 }
 
-// Correctly rounded a / b given rb = RN(1/b): two FMA residual corrections (the first makes the
-// quotient faithful, the second then rounds it correctly), valid while nothing over- or underflows.
-__device__ __forceinline__ float div_rn_by(float a, float b, float rb) {
-    float q = a * rb;
-    q = fmaf(fmaf(-q, b, a), rb, q);
-    return fmaf(fmaf(-q, b, a), rb, q);
-}
-
 // acc[0..7] += v[0..15] * s with packed fp32x2 FMAs (one instruction per column pair)
 __device__ __forceinline__ void fold16(float2* acc, const uint32_t* v, float2 s) {
 #pragma unroll
@@ -204,6 +197,8 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const GemmParams p) 
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_wait();      // everything above overlaps the kernels before this one
+    pdl_trigger();
 
     const int num_valid = p.num_valid[0];
     const int tokens = min(p.num_valid[1], p.M);
@@ -643,8 +638,10 @@ void launch_gemm(const CUtensorMap& tmap, const GemmParams& p, int64_t max_tiles
     GemmParams q = p;
     q.wait_limit = g_wait_limit;
     q.stall_producer = g_stall_producer;
-    moe_gemm_kernel<STAGE, PT, ACT><<<(unsigned)grid, kThreads, kSmemBytes, stream>>>(tmap, q);
-    B200_CUDA(cudaGetLastError());
+    // Overlapping the launch with the kernel before it pays while the layer is short. With tens of tiles per SM the few
+    // microseconds are nothing, and at the power limit the early CTAs cost more than they give (1-2 % at 65 K routes).
+    const bool overlap = max_tiles <= 64 * grid;
+    launch_kernel(overlap, moe_gemm_kernel<STAGE, PT, ACT>, (unsigned)grid, kThreads, kSmemBytes, stream, tmap, q);
 }
 
 }  // namespace

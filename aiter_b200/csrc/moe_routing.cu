@@ -31,7 +31,7 @@ constexpr int kWarpsPerBlock = 4;
 template <typename T>
 __device__ __forceinline__ float load_f(const T* p, int64_t i);
 template <>
-__device__ __forceinline__ float load_f<float>(const float* p, int64_t i) { return __ldg(p + i); }
+__device__ __forceinline__ float load_f<float>(const float* p, int64_t i) { return p[i]; }
 template <>
 __device__ __forceinline__ float load_f<__nv_bfloat16>(const __nv_bfloat16* p, int64_t i) {
     return __bfloat162float(p[i]);
@@ -47,9 +47,9 @@ __device__ __forceinline__ void load_run(const T* row, int i, int n, bool aligne
             float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
             if (i + j < n) {
                 if constexpr (std::is_same<T, float>::value) {
-                    f = __ldg(reinterpret_cast<const float4*>(row + i + j));
+                    f = *reinterpret_cast<const float4*>(row + i + j);
                 } else {
-                    const uint2 raw = __ldg(reinterpret_cast<const uint2*>(row + i + j));
+                    const uint2 raw = *reinterpret_cast<const uint2*>(row + i + j);
                     const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
                     const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
                     f = make_float4(lo.x, lo.y, hi.x, hi.y);
@@ -115,10 +115,12 @@ __device__ __forceinline__ void merge_top2(float& b1, float& b2, float o1, float
 
 template <typename TG, typename TB, int VPL>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32) biased_grouped_topk_kernel(
-    const TG* __restrict__ gating, const TB* __restrict__ bias, float* __restrict__ out_w, int* __restrict__ out_id,
+    const TG* gating, const TB* bias, float* out_w, int* out_id,
     int tokens, int E, int topk, int n_group, int topk_group, int renorm, float scale) {
     const int lane = threadIdx.x & 31;
     const int token = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+    pdl_wait();
+    pdl_trigger();
     if (token >= tokens) return;
     const int gsize = E / n_group;
     const int e0 = lane * VPL;      // this lane's experts: e0 .. e0 + VPL - 1
@@ -188,10 +190,12 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) biased_grouped_topk_kerne
 
 template <typename TG, int VPL>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32) topk_softmax_kernel(
-    const TG* __restrict__ gating, float* __restrict__ out_w, int* __restrict__ out_id, int* __restrict__ src_row,
+    const TG* gating, float* out_w, int* out_id, int* src_row,
     int tokens, int E, int topk, int renorm) {
     const int lane = threadIdx.x & 31;
     const int token = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+    pdl_wait();
+    pdl_trigger();
     if (token >= tokens) return;
     float x[VPL], prob[VPL];   // entry j of a lane is expert j * 32 + lane
     float mx = kNegInf;
@@ -273,8 +277,7 @@ void launch_biased_grouped_topk(const aiter_tensor_t* gating, const aiter_tensor
         auto go = [&](auto* g, auto* b) {
             using TG = std::remove_cv_t<std::remove_pointer_t<decltype(g)>>;
             using TB = std::remove_cv_t<std::remove_pointer_t<decltype(b)>>;
-            biased_grouped_topk_kernel<TG, TB, V><<<grid, kWarpsPerBlock * 32, 0, stream>>>(
-                g, b, (float*)w->ptr, (int*)ids->ptr, (int)tokens, (int)E, (int)topk, n_group, topk_group, renorm, scale);
+            launch_pdl(biased_grouped_topk_kernel<TG, TB, V>, grid, kWarpsPerBlock * 32, 0, stream, g, b, (float*)w->ptr, (int*)ids->ptr, (int)tokens, (int)E, (int)topk, n_group, topk_group, renorm, scale);
         };
         const bool gf = gating->dtype_ == AITER_DTYPE_fp32, bf = bias->dtype_ == AITER_DTYPE_fp32;
         if (gf && bf) go((const float*)gating->ptr, (const float*)bias->ptr);
@@ -282,7 +285,6 @@ void launch_biased_grouped_topk(const aiter_tensor_t* gating, const aiter_tensor
         else if (bf) go((const __nv_bfloat16*)gating->ptr, (const float*)bias->ptr);
         else go((const __nv_bfloat16*)gating->ptr, (const __nv_bfloat16*)bias->ptr);
     });
-    B200_CUDA(cudaGetLastError());
 }
 
 void launch_topk_softmax(aiter_tensor_t* w, aiter_tensor_t* ids, aiter_tensor_t* src_row, const aiter_tensor_t* gating,
@@ -298,15 +300,12 @@ void launch_topk_softmax(aiter_tensor_t* w, aiter_tensor_t* ids, aiter_tensor_t*
     dispatch_vpl((int)E, [&](auto vpl) {
         constexpr int V = decltype(vpl)::value;
         if (gating->dtype_ == AITER_DTYPE_fp32)
-            topk_softmax_kernel<float, V><<<grid, kWarpsPerBlock * 32, 0, stream>>>(
-                (const float*)gating->ptr, (float*)w->ptr, (int*)ids->ptr, src_row ? (int*)src_row->ptr : nullptr,
+            launch_pdl(topk_softmax_kernel<float, V>, grid, kWarpsPerBlock * 32, 0, stream, (const float*)gating->ptr, (float*)w->ptr, (int*)ids->ptr, src_row ? (int*)src_row->ptr : nullptr,
                 (int)tokens, (int)E, (int)topk, renorm);
         else
-            topk_softmax_kernel<__nv_bfloat16, V><<<grid, kWarpsPerBlock * 32, 0, stream>>>(
-                (const __nv_bfloat16*)gating->ptr, (float*)w->ptr, (int*)ids->ptr, src_row ? (int*)src_row->ptr : nullptr,
+            launch_pdl(topk_softmax_kernel<__nv_bfloat16, V>, grid, kWarpsPerBlock * 32, 0, stream, (const __nv_bfloat16*)gating->ptr, (float*)w->ptr, (int*)ids->ptr, src_row ? (int*)src_row->ptr : nullptr,
                 (int)tokens, (int)E, (int)topk, renorm);
     });
-    B200_CUDA(cudaGetLastError());
 }
 
 }  // namespace b200

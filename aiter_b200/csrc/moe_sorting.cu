@@ -3,19 +3,25 @@
 // (csrc/include/moe_sorting_opus.h:280-359) with the padding values of its torch oracle
 // (op_tests/test_moe_sorting.py:45-99).
 //
-// Route r = token*topk + slot.  Within an expert routes keep ascending r, which is the order
-// torch.where() yields in the oracle.  Each warp owns a contiguous run of routes, so the
-// position of a route is
-//     base[expert] + (routes of that expert in earlier CTAs) + (in earlier warps of this CTA)
-//                  + (in earlier 32-route steps of this warp) + (in lower lanes of this step)
-// where the last term comes from __match_any_sync + popc.  No atomics on the output side:
-// the result is deterministic.
+// Route r = token*topk + slot.  Within an expert routes keep ascending r, which is the order torch.where() yields in the
+// oracle.  The position of a route is
+//     base[expert] + (routes of that expert in earlier chunks) + (in earlier 32-route runs of its chunk)
+//                  + (in lower lanes of its run)
+// where the last term comes from __match_any_sync + popc and the third from one byte per (expert, run) that the run's
+// leader lane writes: no atomics on the output side, the result is deterministic.
 //
-// Two launch shapes:
-//   single CTA   routes <= kSingleMaxRoutes: count, scan, fill and scatter in one kernel;
-//   multi CTA    count per 4096-route chunk -> scan (1 CTA) -> scatter per chunk, with the
-//                per-chunk counts and expert bases in a caller-provided workspace.
-// Extra CTAs zero-fill moe_buf when the caller passes one (in the single kernel, or beside the scan).
+// Launch shapes (a chunk is 4096 routes, one CTA of 1024 threads):
+//   routes <= kSingleMaxRoutes  one kernel; every CTA counts the other chunks' routes itself (a few shared-memory atomics
+//                               per thread), which is cheaper than a grid-wide dependency;
+//   more                        count per chunk -> scatter, whose CTAs each add up the per-chunk counts, with the counts in
+//                               a caller-provided workspace. (A scan kernel in between, one CTA for all experts, was 9 us
+//                               at 24 K routes and 50 us with the fill of a 235 MB moe_buf beside it.)
+// What bounds it: latency, a handful of dependent phases of one CTA. Padding entries and block ids are written by warps,
+// an expert each: a thread per expert wrote up to 127 pads one after the other, 12-27 us of decode layers.
+// Measured (DeepSeek-V3 routing, unit 128): 64 tokens 26 -> 5 us, 3001 tokens (unit 32) 20 -> 11 us.
+// Extra CTAs zero-fill moe_buf when the caller passes one.
+
+#include <algorithm>
 
 #include "common.cuh"
 
@@ -24,8 +30,8 @@ namespace {
 
 constexpr int kThreads = 1024;
 constexpr int kWarps = kThreads / 32;
-constexpr int kChunk = 4096;            // routes per CTA on the multi-CTA path
-constexpr int kSingleMaxRoutes = 16384; // above this the multi-CTA path is used
+constexpr int kChunk = 4096;            // routes per sorting CTA
+constexpr int kSingleMaxRoutes = 16384; // above this the two-kernel path is used
 constexpr int kMaxExperts = 1024;
 
 struct SortArgs {
@@ -38,15 +44,15 @@ struct SortArgs {
     int* sorted_eids;
     int* num_valid;
     int* local_topk_ids;   // [M*topk] or null
-    int* ws_cnt;           // [nchunks*E]   (multi-CTA only)
-    int* ws_base;          // [E]           (multi-CTA only)
+    int* ws_cnt;           // [nchunks*E]   (two-kernel path only)
     uint4* zero_buf;       // moe_buf or null
     size_t zero_vec16;     // number of 16-byte words to clear
     unsigned char* zero_tail;
     int zero_tail_bytes;
     int M, topk, E, unit;
     int max_padded, max_blocks;
-    int nchunks;           // CTAs that sort (1 on the single-CTA path)
+    int nchunks;           // CTAs that sort
+    int runs;              // 32-route runs per chunk: 32 times the rounds of kThreads routes a CTA makes
 };
 
 __device__ __forceinline__ int eff_tokens(const SortArgs& a) {
@@ -59,33 +65,27 @@ __device__ __forceinline__ int eff_tokens(const SortArgs& a) {
     return t;
 }
 
-// Exclusive scan of one int per thread over the whole CTA (kThreads threads).
-__device__ __forceinline__ int block_scan_excl(int v, int* warp_tot, int& total) {
+// Exclusive scans of two ints per thread over the whole CTA (kThreads threads).
+__device__ __forceinline__ void block_scan2_excl(int& u, int& v, int2* warp_tot, int& total_v) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int incl = v;
+    int iu = u, iv = v;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
-        int n = __shfl_up_sync(0xffffffffu, incl, d);
-        if (lane >= d) incl += n;
-    }
-    if (lane == 31) warp_tot[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-        int t = warp_tot[lane];
-        int ti = t;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            int n = __shfl_up_sync(0xffffffffu, ti, d);
-            if (lane >= d) ti += n;
+        const int nu = __shfl_up_sync(0xffffffffu, iu, d), nv = __shfl_up_sync(0xffffffffu, iv, d);
+        if (lane >= d) {
+            iu += nu;
+            iv += nv;
         }
-        warp_tot[lane] = ti - t;  // exclusive prefix of warp totals
-        if (lane == 31) warp_tot[32] = ti;
     }
+    if (lane == 31) warp_tot[warp] = make_int2(iu, iv);
     __syncthreads();
-    total = warp_tot[32];
-    int r = warp_tot[warp] + incl - v;
-    __syncthreads();
-    return r;
+    // every warp adds up the totals before it (no second round trip through shared memory)
+    const int2 t = warp_tot[lane];
+    const bool before = lane < warp;
+    const int bu = __reduce_add_sync(0xffffffffu, before ? t.x : 0), bv = __reduce_add_sync(0xffffffffu, before ? t.y : 0);
+    total_v = __reduce_add_sync(0xffffffffu, t.y);
+    u = bu + iu - u;
+    v = bv + iv - v;
 }
 
 __device__ __forceinline__ void zero_fill(const SortArgs& a, int part, int nparts) {
@@ -96,201 +96,186 @@ __device__ __forceinline__ void zero_fill(const SortArgs& a, int part, int npart
     if (part == 0 && (int)threadIdx.x < a.zero_tail_bytes) a.zero_tail[threadIdx.x] = 0;
 }
 
-// local_id[e] = cumsum(mask)-1 for kept experts, -1 for dropped ones.
-__device__ __forceinline__ void build_local_ids(const SortArgs& a, int* local_id, int* warp_tot) {
-    const int e = threadIdx.x;
-    int keep = (e < a.E) ? (a.mask ? (a.mask[e] != 0) : 1) : 0;
-    int total;
-    int excl = block_scan_excl(keep, warp_tot, total);
-    if (e < a.E) local_id[e] = keep ? excl : -1;
-    __syncthreads();
-}
+__device__ __forceinline__ int byte_sum(uint32_t w, int acc) { return __dp4a(w, 0x01010101u, (unsigned)acc); }
 
-// Per-warp histogram of routes [r0, r1): hist[w*E + e].  Warp w owns
-// [r0 + w*seg, r0 + (w+1)*seg) with seg a multiple of 32.
-__device__ __forceinline__ int warp_segment(int r0, int r1) {
-    int n = r1 - r0;
-    int seg = (n + kWarps - 1) / kWarps;
-    return (seg + 31) & ~31;
-}
-
-__device__ __forceinline__ void count_routes(const SortArgs& a, int* hist, int r0, int r1) {
-    for (int i = threadIdx.x; i < kWarps * a.E; i += kThreads) hist[i] = 0;
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int seg = warp_segment(r0, r1);
-    const int s0 = r0 + warp * seg;
-    const int s1 = min(s0 + seg, r1);
-    for (int i = s0 + lane; i < s1; i += 32) {
-        int e = a.ids[i];
-        if (e >= 0 && e < a.E) atomicAdd(&hist[warp * a.E + e], 1);
+// Sum of the first n bytes of a 16-byte aligned row (n up to its length).
+__device__ __forceinline__ int prefix_bytes(const unsigned char* row, int n) {
+    const uint4* p = reinterpret_cast<const uint4*>(row);
+    int s = 0;
+    for (; n >= 16; n -= 16, ++p) {
+        const uint4 x = *p;
+        s = byte_sum(x.w, byte_sum(x.z, byte_sum(x.y, byte_sum(x.x, s))));
     }
-    __syncthreads();
-}
-
-// hist[w][e] -> exclusive prefix over w; returns the CTA total for expert e = threadIdx.x.
-__device__ __forceinline__ int prefix_over_warps(const SortArgs& a, int* hist) {
-    int run = 0;
-    const int e = threadIdx.x;
-    if (e < a.E) {
-#pragma unroll 4
-        for (int w = 0; w < kWarps; ++w) {
-            int c = hist[w * a.E + e];
-            hist[w * a.E + e] = run;
-            run += c;
+    if (n > 0) {
+        const uint4 x = *p;
+        const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int nb = n - 4 * k;
+            if (nb > 0) s = byte_sum(nb >= 4 ? w[k] : w[k] & ((1u << (8 * nb)) - 1u), s);
         }
     }
-    return run;
+    return s;
 }
 
-__device__ __forceinline__ void scatter_routes(const SortArgs& a, int* hist, const int* gbase,
-                                               const int* local_id, int r0, int r1) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int seg = warp_segment(r0, r1);
-    const int s0 = r0 + warp * seg;
-    const int s1 = min(s0 + seg, r1);
-    const unsigned lt = (1u << lane) - 1u;
-    for (int it = s0; it < s1; it += 32) {
-        const int i = it + lane;
-        const bool in = i < s1;
-        int e = in ? a.ids[i] : -1;
-        int lid = (in && e >= 0 && e < a.E) ? local_id[e] : -1;
-        const bool live = in && e >= 0 && e < a.E;
-        // lanes with the same expert form a group; others get a private key
-        unsigned grp = __match_any_sync(0xffffffffu, live ? e : (a.E + lane));
-        int rank = __popc(grp & lt);
-        int off = live ? hist[warp * a.E + e] : 0;
-        __syncwarp();
-        if (live && rank == 0) hist[warp * a.E + e] = off + __popc(grp);
-        __syncwarp();
-        if (in && a.local_topk_ids) a.local_topk_ids[i] = lid;
-        if (lid >= 0) {
-            int pos = gbase[e] + off + rank;
-            int token = i / a.topk;
-            int slot = i - token * a.topk;
-            a.sorted_ids[pos] = (slot << 24) | token;
-            a.sorted_w[pos] = a.weights[i];
-        }
-    }
-}
+extern __shared__ __align__(16) unsigned char smem_b[];
+// smem of the sorting CTAs: run_cnt[E][row_bytes] | before[E] | after[E] | start[E] | base[E] | warp_tot[32]
+__host__ __device__ inline int row_bytes(int runs) { return runs + 16; }   // + 16: rows start in different banks
 
-// Given cnt (routes of expert e) writes: base[e] (smem), expert ids of its blocks, its pad
-// entries, the tail past the padded total, num_valid.
-__device__ __forceinline__ void layout_experts(const SortArgs& a, int cnt, const int* local_id,
-                                               int* base, int* warp_tot, int tokens) {
-    const int e = threadIdx.x;
-    int lid = (e < a.E) ? local_id[e] : -1;
-    int padded = (lid >= 0 && cnt > 0) ? ((cnt + a.unit - 1) / a.unit) * a.unit : 0;
-    int total;
-    int b = block_scan_excl(padded, warp_tot, total);
-    if (e < a.E) base[e] = b;
-    const int pad_id = (a.topk << 24) | a.M;
-    if (padded > 0) {
-        for (int k = 0; k < padded / a.unit; ++k) a.sorted_eids[b / a.unit + k] = lid;
-        for (int p = b + cnt; p < b + padded; ++p) {
-            a.sorted_ids[p] = pad_id;
-            a.sorted_w[p] = 0.f;
+// FROM_WS: the routes of the other chunks come from the counts in the workspace; else they are counted here.
+template <bool FROM_WS>
+__global__ void __launch_bounds__(kThreads, 1) sort_kernel(SortArgs a) {
+    if ((int)blockIdx.x >= a.nchunks) {
+        // the fill beside the two-kernel sort starts at once: the kernel before it is the count, which does not touch moe_buf
+        if (!FROM_WS) pdl_wait();
+        pdl_trigger();
+        zero_fill(a, blockIdx.x - a.nchunks, gridDim.x - a.nchunks);
+        if (FROM_WS) pdl_wait();
+        return;
+    }
+    const int rb = row_bytes(a.runs), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    unsigned char* run_cnt = smem_b;
+    int* before = reinterpret_cast<int*>(smem_b + (size_t)a.E * rb);   // routes of e in earlier chunks
+    int* after = before + a.E;                                         // ... in later chunks
+    int* start = after + a.E;    // position of this chunk's first route of e, -1: expert dropped
+    int* base = start + a.E;     // first position of e
+    int2* warp_tot = reinterpret_cast<int2*>(base + a.E);
+    for (int i = tid; i < a.E * rb / 16; i += kThreads) reinterpret_cast<uint4*>(run_cnt)[i] = make_uint4(0, 0, 0, 0);
+    for (int i = tid; i < a.E; i += kThreads) before[i] = after[i] = 0;
+    pdl_wait();
+    pdl_trigger();
+    const int tokens = eff_tokens(a);
+    const int routes = tokens * a.topk;
+    const int c = blockIdx.x, r0 = min(c * kChunk, routes), r1 = min(r0 + kChunk, routes);
+    // this chunk's ids and weights, kept in registers
+    const int rounds = a.runs / kWarps;
+    int e[kChunk / kThreads], rank[kChunk / kThreads];
+    float w[kChunk / kThreads];
+#pragma unroll
+    for (int q = 0; q < kChunk / kThreads; ++q) {
+        const int i = r0 + q * kThreads + tid;
+        const bool in = q < rounds && i < r1;
+        e[q] = in ? a.ids[i] : -1;
+        w[q] = in ? a.weights[i] : 0.f;
+        if (e[q] >= a.E) e[q] = -1;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kChunk / kThreads; ++q) {
+        if (q >= rounds) break;
+        const bool live = e[q] >= 0;
+        const unsigned grp = __match_any_sync(0xffffffffu, live ? e[q] : a.E + lane);   // lanes without a route: a key each
+        rank[q] = __popc(grp & ((1u << lane) - 1u));
+        if (live && rank[q] == 0) run_cnt[e[q] * rb + q * kWarps + warp] = (unsigned char)__popc(grp);
+    }
+    if (FROM_WS) {
+        // thread (part, expert): parts of the chunks in parallel, eight loads in flight each
+        const int parts = kThreads / a.E;   // E <= kThreads
+        const int ex = tid % a.E, part = tid / a.E;
+        if (part < parts) {
+            int b = 0, f = 0;
+            for (int k0 = part; k0 < a.nchunks; k0 += 8 * parts) {
+                int v[8];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    const int ch = k0 + k * parts;
+                    v[k] = ch < a.nchunks ? __ldcg(a.ws_cnt + (size_t)ch * a.E + ex) : 0;
+                }
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    const int ch = k0 + k * parts;
+                    b += ch < c ? v[k] : 0;
+                    f += ch > c ? v[k] : 0;
+                }
+            }
+            if (b) atomicAdd(before + ex, b);
+            if (f) atomicAdd(after + ex, f);
         }
+    } else {
+        for (int i = tid; i < routes; i += kThreads)
+            if (i < r0 || i >= r1) {
+                const int x = a.ids[i];
+                if (x >= 0 && x < a.E) atomicAdd((i < r0 ? before : after) + x, 1);
+            }
     }
-    for (int k = total / a.unit + threadIdx.x; k < a.max_blocks; k += kThreads) a.sorted_eids[k] = -1;
-    for (int p = total + threadIdx.x; p < a.max_padded; p += kThreads) {
-        a.sorted_ids[p] = pad_id;
-        a.sorted_w[p] = 0.f;
+    __syncthreads();
+    // layout: thread e owns expert e
+    int cnt = 0, lid = 0, at = 0, total;
+    bool keep = false;
+    if (tid < a.E) {
+        keep = a.mask ? a.mask[tid] != 0 : true;
+        cnt = before[tid] + after[tid] + prefix_bytes(run_cnt + tid * rb, a.runs);
     }
-    if (threadIdx.x == 0) {
+    const int padded = keep ? (cnt + a.unit - 1) / a.unit * a.unit : 0;
+    lid = keep ? 1 : 0;
+    at = padded;
+    block_scan2_excl(lid, at, warp_tot, total);   // local expert id, first position
+    if (tid < a.E) {
+        start[tid] = keep ? at + before[tid] : -1;
+        base[tid] = keep ? at : -1;
+        after[tid] = cnt;       // from here on: routes of e in all chunks
+        before[tid] = lid;      // ... and the local id
+    }
+    if (c == 0 && tid == 0) {
         a.num_valid[0] = total;
         a.num_valid[1] = tokens;
     }
     __syncthreads();
-}
-
-__device__ __forceinline__ void clear_unsorted_local_ids(const SortArgs& a, int routes, int part,
-                                                         int nparts) {
-    if (!a.local_topk_ids) return;
-    for (int i = routes + part * kThreads + threadIdx.x; i < a.M * a.topk; i += nparts * kThreads)
-        a.local_topk_ids[i] = -1;
-}
-
-extern __shared__ int smem_i[];
-// smem: hist[kWarps*E] | local_id[E] | base[E] | warp_tot[40]
-
-__global__ void __launch_bounds__(kThreads, 1) sort_single_kernel(SortArgs a) {
-    if ((int)blockIdx.x >= a.nchunks) {
-        zero_fill(a, blockIdx.x - a.nchunks, gridDim.x - a.nchunks);
-        return;
-    }
-    int* hist = smem_i;
-    int* local_id = hist + kWarps * a.E;
-    int* base = local_id + a.E;
-    int* warp_tot = base + a.E;
-    const int tokens = eff_tokens(a);
-    const int routes = tokens * a.topk;
-    build_local_ids(a, local_id, warp_tot);
-    count_routes(a, hist, 0, routes);
-    int cnt = prefix_over_warps(a, hist);
-    layout_experts(a, cnt, local_id, base, warp_tot, tokens);
-    scatter_routes(a, hist, base, local_id, 0, routes);
-    clear_unsorted_local_ids(a, routes, 0, 1);
-}
-
-__global__ void __launch_bounds__(kThreads, 1) sort_count_kernel(SortArgs a) {
-    int* hist = smem_i;
-    const int routes = eff_tokens(a) * a.topk;
-    const int r0 = min((int)blockIdx.x * kChunk, routes);
-    const int r1 = min(r0 + kChunk, routes);
-    count_routes(a, hist, r0, r1);
-    int cnt = prefix_over_warps(a, hist);
-    if ((int)threadIdx.x < a.E) a.ws_cnt[blockIdx.x * a.E + threadIdx.x] = cnt;
-}
-
-__global__ void __launch_bounds__(kThreads, 1) sort_scan_kernel(SortArgs a) {
-    // CTA 0 scans; the others zero-fill moe_buf beside it. The scan is one CTA's worth of latency (tens of
-    // microseconds at 64 K routes), the fill is bandwidth: in the same launch the fill costs nothing extra, in the
-    // count kernel (which is over in microseconds) it would delay the two kernels behind it by its whole length.
-    if (blockIdx.x >= 1) {
-        zero_fill(a, blockIdx.x - 1, gridDim.x - 1);
-        return;
-    }
-    int* local_id = smem_i;
-    int* base = local_id + a.E;
-    int* warp_tot = base + a.E;
-    const int tokens = eff_tokens(a);
-    build_local_ids(a, local_id, warp_tot);
-    int run = 0;
-    const int e = threadIdx.x;
-    if (e < a.E) {
-        // 8 independent loads in flight at a time (the stores in between would otherwise serialise them)
-        for (int c0 = 0; c0 < a.nchunks; c0 += 8) {
-            int v[8];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) v[k] = (c0 + k < a.nchunks) ? __ldcg(a.ws_cnt + (c0 + k) * a.E + e) : 0;
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                if (c0 + k < a.nchunks) a.ws_cnt[(c0 + k) * a.E + e] = run;  // routes of e in earlier chunks
-                run += v[k];
-            }
+    for (int q = 0; q < kChunk / kThreads; ++q) {
+        if (q >= rounds) break;
+        const int i = r0 + q * kThreads + tid;
+        const int s = e[q] >= 0 ? start[e[q]] : -1;
+        if (i < r1 && a.local_topk_ids) a.local_topk_ids[i] = s >= 0 ? before[e[q]] : -1;
+        if (s >= 0) {
+            const int pos = s + prefix_bytes(run_cnt + e[q] * rb, q * kWarps + warp) + rank[q];
+            const int token = i / a.topk;
+            a.sorted_ids[pos] = ((i - token * a.topk) << 24) | token;
+            a.sorted_w[pos] = w[q];
         }
     }
-    layout_experts(a, run, local_id, base, warp_tot, tokens);
-    if (e < a.E) a.ws_base[e] = base[e];
+    // expert ids of the blocks and pad entries: a warp per expert; then the tail past the padded total
+    const int pad_id = (a.topk << 24) | a.M;
+    for (int x = c * kWarps + warp; x < a.E; x += a.nchunks * kWarps) {
+        const int n = after[x], b = base[x];
+        if (b < 0 || n == 0) continue;
+        const int end = b + (n + a.unit - 1) / a.unit * a.unit;
+        for (int k = b / a.unit + lane; k < end / a.unit; k += 32) a.sorted_eids[k] = before[x];
+        for (int p = b + n + lane; p < end; p += 32) {
+            a.sorted_ids[p] = pad_id;
+            a.sorted_w[p] = 0.f;
+        }
+    }
+    const int part = c * kThreads + tid, nparts = a.nchunks * kThreads;
+    for (int k = total / a.unit + part; k < a.max_blocks; k += nparts) a.sorted_eids[k] = -1;
+    for (int p = total + part; p < a.max_padded; p += nparts) {
+        a.sorted_ids[p] = pad_id;
+        a.sorted_w[p] = 0.f;
+    }
+    if (a.local_topk_ids)
+        for (int i = routes + part; i < a.M * a.topk; i += nparts) a.local_topk_ids[i] = -1;
 }
 
-__global__ void __launch_bounds__(kThreads, 1) sort_scatter_kernel(SortArgs a) {
-    int* hist = smem_i;
-    int* local_id = hist + kWarps * a.E;
-    int* base = local_id + a.E;
-    int* warp_tot = base + a.E;
+// Routes per (chunk, expert) for the two-kernel path.
+__global__ void __launch_bounds__(kThreads, 1) sort_count_kernel(SortArgs a) {
+    int* hist = reinterpret_cast<int*>(smem_b);
+    for (int i = threadIdx.x; i < a.E; i += kThreads) hist[i] = 0;
+    pdl_wait();
+    pdl_trigger();
     const int routes = eff_tokens(a) * a.topk;
-    const int r0 = min((int)blockIdx.x * kChunk, routes);
-    const int r1 = min(r0 + kChunk, routes);
-    build_local_ids(a, local_id, warp_tot);
-    count_routes(a, hist, r0, r1);
-    prefix_over_warps(a, hist);
-    if ((int)threadIdx.x < a.E)
-        base[threadIdx.x] = a.ws_base[threadIdx.x] + a.ws_cnt[blockIdx.x * a.E + threadIdx.x];
+    const int r0 = min((int)blockIdx.x * kChunk, routes), r1 = min(r0 + kChunk, routes);
+    int e[kChunk / kThreads];
+#pragma unroll
+    for (int q = 0; q < kChunk / kThreads; ++q) {
+        const int i = r0 + q * kThreads + threadIdx.x;
+        e[q] = i < r1 ? a.ids[i] : -1;
+    }
     __syncthreads();
-    scatter_routes(a, hist, base, local_id, r0, r1);
-    clear_unsorted_local_ids(a, routes, blockIdx.x, gridDim.x);
+#pragma unroll
+    for (int q = 0; q < kChunk / kThreads; ++q)
+        if (e[q] >= 0 && e[q] < a.E) atomicAdd(hist + e[q], 1);
+    __syncthreads();
+    for (int i = threadIdx.x; i < a.E; i += kThreads) a.ws_cnt[(size_t)blockIdx.x * a.E + i] = hist[i];
 }
 
 inline int num_chunks(int64_t routes) { return (int)((routes + kChunk - 1) / kChunk); }
@@ -385,14 +370,21 @@ void launch_moe_sorting(const aiter_tensor_t* topk_ids, const aiter_tensor_t* to
     }
 
     const int64_t routes = M * topk;
-    const size_t smem_full = ((size_t)kWarps * E + 2 * (size_t)E + 40) * sizeof(int);
+    a.nchunks = std::max(1, num_chunks(routes));
+    a.runs = kWarps * (int)((std::min<int64_t>(routes, kChunk) + kThreads - 1) / kThreads);
+    if (a.runs < kWarps) a.runs = kWarps;
+    const size_t smem = (size_t)E * row_bytes(a.runs) + 4 * (size_t)E * sizeof(int) + 32 * sizeof(int2);
+    static bool attr_set[64] = {false};
+    const int dev = topk_ids->device_id;
+    if (dev >= 64 || !attr_set[dev]) {
+        const int most = kMaxExperts * row_bytes(kChunk / 32) + 4 * kMaxExperts * (int)sizeof(int) + 32 * (int)sizeof(int2);
+        B200_CUDA(cudaFuncSetAttribute(sort_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+        B200_CUDA(cudaFuncSetAttribute(sort_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+        if (dev < 64) attr_set[dev] = true;
+    }
     if (routes <= kSingleMaxRoutes) {
-        a.nchunks = 1;
-        B200_CUDA(cudaFuncSetAttribute(sort_single_kernel,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_full));
-        sort_single_kernel<<<1 + zero_ctas, kThreads, smem_full, stream>>>(a);
+        launch_pdl(sort_kernel<false>, a.nchunks + zero_ctas, kThreads, smem, stream, a);
     } else {
-        a.nchunks = num_chunks(routes);
         const int64_t need = sorting_workspace_bytes((int)M, E, (int)topk);
         B200_CHECK(workspace != nullptr && workspace->ptr != nullptr,
                    "workspace of ", need, " bytes is required for this problem size");
@@ -401,16 +393,9 @@ void launch_moe_sorting(const aiter_tensor_t* topk_ids, const aiter_tensor_t* to
         size_t ws_esz = (workspace->dtype_ == AITER_DTYPE_u8 || workspace->dtype_ == AITER_DTYPE_i8) ? 1 : 4;
         B200_CHECK((int64_t)(workspace->numel_ * ws_esz) >= need, "workspace needs ", need, " bytes");
         a.ws_cnt = (int*)workspace->ptr;
-        a.ws_base = a.ws_cnt + (size_t)a.nchunks * E;
-        B200_CUDA(cudaFuncSetAttribute(sort_count_kernel,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_full));
-        B200_CUDA(cudaFuncSetAttribute(sort_scatter_kernel,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_full));
-        sort_count_kernel<<<a.nchunks, kThreads, smem_full, stream>>>(a);
-        sort_scan_kernel<<<1 + zero_ctas, kThreads, (2 * (size_t)E + 40) * sizeof(int), stream>>>(a);
-        sort_scatter_kernel<<<a.nchunks, kThreads, smem_full, stream>>>(a);
+        launch_pdl(sort_count_kernel, a.nchunks, kThreads, (size_t)E * sizeof(int), stream, a);
+        launch_pdl(sort_kernel<true>, a.nchunks + zero_ctas, kThreads, smem, stream, a);
     }
-    B200_CUDA(cudaGetLastError());
 }
 
 // ------------------------------------------------------------------------------------------------

@@ -5,6 +5,9 @@
 // reciprocals instead (csrc/kernels/quant_kernels.cu:121,159-160), which is not.
 //
 // 16 lanes own one 128-element group (8 bf16 = one 16-byte load each), two groups per warp.
+//
+// What bounds these kernels: HBM, 3 bytes per element. That takes several loads in flight per thread and short
+// arithmetic (quant_codes8); with one load per thread and eight IEEE divisions the 1x128 kernel ran at 2.3 TB/s.
 
 #include <algorithm>
 
@@ -19,79 +22,106 @@ namespace b200 {
 namespace {
 
 constexpr int kQuantThreads = 256;
-constexpr int kGroupsPerBlock = kQuantThreads / 16;
 
 // num_rows (optional, device): only the first *num_rows * rows_factor rows are quantised. transposed: the scale of
 // group (row, col-group) goes to scales[col-group * rows_used + row] instead of scales[row * groups_per_row + col-group]
 // (the layout the reference's 1-stage path reads, csrc/kernels/quant_kernels.cu:143-146; rows_used = the dynamic
 // row count when num_rows is given, as there).
-template <bool F16>
+// A CTA covers kQuantThreads * U consecutive 16-byte pieces, U loads in flight per thread.
+// after_wait = false: this launch neither reads nor overwrites anything of the kernel before it on the stream, so it may
+// run beside it (the layer's quantiser beside the sort); its completion still implies that kernel's.
+template <bool F16, int U>
 __global__ void __launch_bounds__(kQuantThreads) quant_1x128_kernel(
-    const uint4* __restrict__ x, uint2* __restrict__ q, float* __restrict__ scales, int64_t groups, int groups_per_row,
-    const int* __restrict__ num_rows, int rows_factor, int transposed) {
-    const int64_t g = (int64_t)blockIdx.x * kGroupsPerBlock + (threadIdx.x >> 4);
-    const int sub = threadIdx.x & 15;
+    const uint4* x, uint2* q, float* scales, int64_t groups, int groups_per_row, const int* num_rows, int rows_factor,
+    int transposed, bool after_wait) {
+    if (after_wait) pdl_wait();
+    pdl_trigger();
+    const int64_t p0 = (int64_t)blockIdx.x * (kQuantThreads * U) + threadIdx.x;
     int64_t rows_used = groups / groups_per_row;
     if (num_rows) rows_used = min(rows_used, (int64_t)*num_rows * rows_factor);
-    const bool live = g < rows_used * groups_per_row;
-    uint4 raw = make_uint4(0, 0, 0, 0);
-    if (live) raw = __ldg(x + g * 16 + sub);
-    uint2 codes;
-    const float scale = quant_group16<F16>(raw, codes);
-    if (live) {
-        q[g * 16 + sub] = codes;
-        if (sub == 0) {
-            const int64_t row = g / groups_per_row, cg = g - row * groups_per_row;
-            scales[transposed ? cg * rows_used + row : g] = scale;
+    const int64_t pieces = rows_used * groups_per_row * 16;
+    uint4 raw[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        raw[u] = make_uint4(0, 0, 0, 0);
+        if (p0 + u * kQuantThreads < pieces) raw[u] = x[p0 + u * kQuantThreads];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int64_t p = p0 + u * kQuantThreads;
+        uint2 codes;
+        const float scale = quant_group16<F16>(raw[u], codes);
+        if (p < pieces) {
+            q[p] = codes;
+            if ((threadIdx.x & 15) == 0) {
+                const int64_t g = p >> 4;
+                if (transposed) {
+                    const int64_t row = g / groups_per_row, cg = g - row * groups_per_row;
+                    scales[cg * rows_used + row] = scale;
+                } else {
+                    scales[g] = scale;
+                }
+            }
         }
     }
+    if (!after_wait) pdl_wait();
 }
 
-// Per-row dynamic FP8 quantisation over the whole row (QuantType.per_Token): one CTA per row, the row is
-// kept in shared memory between the amax pass and the conversion pass. Same rounding sequence as above
-// (aiter/ops/quant.py:64-94 over the last dimension). Rows >= *row_limit (if given) are skipped.
-template <bool F16>
-__global__ void __launch_bounds__(256) quant_per_token_kernel(const uint4* __restrict__ x, uint2* __restrict__ q,
-                                                              float* __restrict__ scales, int cols8,
-                                                              const int* __restrict__ row_limit, int rows_factor) {
-    extern __shared__ uint4 row_s[];
-    __shared__ float red[8];
-    const int64_t row = blockIdx.x;
-    if (row_limit && row >= (int64_t)*row_limit * rows_factor) return;
-    float amax = 0.f;
-    for (int i = threadIdx.x; i < cols8; i += blockDim.x) {
-        const uint4 raw = __ldg(x + row * cols8 + i);
-        row_s[i] = raw;
-        float v[8];
-        unpack8<F16>(raw, v);
+// Per-row dynamic FP8 quantisation over the whole row (QuantType.per_Token): one CTA per row at a time; the row stays in
+// registers (CACHE 16-byte pieces per thread) between the amax pass and the conversion pass; what does not fit there is
+// read again (L1/L2). Same rounding sequence as above (aiter/ops/quant.py:64-94 over the last dimension). Rows at or past
+// *row_limit * rows_factor (if given) are skipped: the grid is a few CTAs per SM that stride over the rows below it, so a
+// sorted buffer's padded tail costs no CTAs.
+constexpr int kRowThreads = 256;
+template <bool F16, int CACHE>
+__global__ void __launch_bounds__(kRowThreads) quant_per_token_kernel(const uint4* x, uint2* q, float* scales, int64_t rows,
+                                                                      int cols8, const int* row_limit, int rows_factor,
+                                                                      bool after_wait) {
+    __shared__ float red[2][kRowThreads / 32];
+    if (after_wait) pdl_wait();
+    pdl_trigger();
+    const int tid = threadIdx.x;
+    if (row_limit) rows = min(rows, (int64_t)*row_limit * rows_factor);
+    int par = 0;
+    for (int64_t row = blockIdx.x; row < rows; row += gridDim.x, par ^= 1) {
+        const uint4* xr = x + row * cols8;
+        uint4 raw[CACHE];
+        float amax = 0.f, v[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) amax = fmaxf(amax, fabsf(v[k]));
-    }
-#pragma unroll
-    for (int d = 16; d >= 1; d >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, d));
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
-    __syncthreads();
-    amax = red[0];
-#pragma unroll
-    for (int k = 1; k < 8; ++k) amax = fmaxf(amax, red[k]);
-    float scale = __fdiv_rn(amax, 448.0f);
-    if (scale == 0.f) scale = 1.f;
-    for (int i = threadIdx.x; i < cols8; i += blockDim.x) {
-        const uint4 raw = row_s[i];
-        float v[8];
-        unpack8<F16>(raw, v);
-        uint32_t w[2];
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(__fdiv_rn(v[4 * k], scale), __fdiv_rn(v[4 * k + 1], scale)),
-                                                         __NV_SATFINITE, __NV_E4M3);
-            const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(__fdiv_rn(v[4 * k + 2], scale), __fdiv_rn(v[4 * k + 3], scale)),
-                                                         __NV_SATFINITE, __NV_E4M3);
-            w[k] = lo | (hi << 16);
+        for (int k = 0; k < CACHE; ++k) {
+            raw[k] = make_uint4(0, 0, 0, 0);
+            if (k * kRowThreads + tid < cols8) raw[k] = xr[k * kRowThreads + tid];
         }
-        q[row * cols8 + i] = make_uint2(w[0], w[1]);
+#pragma unroll
+        for (int k = 0; k < CACHE; ++k) {
+            unpack8<F16>(raw[k], v);
+            amax = amax8(v, amax);
+        }
+        for (int i = CACHE * kRowThreads + tid; i < cols8; i += kRowThreads) {
+            unpack8<F16>(xr[i], v);
+            amax = amax8(v, amax);
+        }
+#pragma unroll
+        for (int d = 16; d >= 1; d >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, d));
+        if ((tid & 31) == 0) red[par][tid >> 5] = amax;
+        __syncthreads();   // one per row: the buffers alternate
+#pragma unroll
+        for (int k = 0; k < kRowThreads / 32; ++k) amax = fmaxf(amax, red[par][k]);
+        float scale = __fdiv_rn(amax, 448.0f);
+        if (scale == 0.f) scale = 1.f;
+#pragma unroll
+        for (int k = 0; k < CACHE; ++k)
+            if (k * kRowThreads + tid < cols8) {
+                unpack8<F16>(raw[k], v);
+                q[row * cols8 + k * kRowThreads + tid] = quant_codes8(v, scale);
+            }
+        for (int i = CACHE * kRowThreads + tid; i < cols8; i += kRowThreads) {
+            unpack8<F16>(xr[i], v);
+            q[row * cols8 + i] = quant_codes8(v, scale);
+        }
+        if (tid == 0) scales[row] = scale;
     }
-    if (threadIdx.x == 0) scales[row] = scale;
+    if (!after_wait) pdl_wait();
 }
 
 // Per-tensor dynamic FP8 quantisation (QuantType.per_Tensor; torch twin per_tensor_quant, aiter/ops/quant.py:318-328:
@@ -100,17 +130,25 @@ __global__ void __launch_bounds__(256) quant_per_token_kernel(const uint4* __res
 // so an integer atomicMax does it), then every row is converted with the one scale, which is also written to
 // scale[0] and, if asked, once per row to row_scales (the GEMM kernels take one activation scale per row).
 template <bool F16>
-__global__ void __launch_bounds__(256) amax_kernel(const uint4* __restrict__ x, int64_t rows, int cols8,
-                                                   const int* __restrict__ row_limit, unsigned int* __restrict__ amax) {
+__global__ void __launch_bounds__(256) amax_kernel(const uint4* x, int64_t rows, int cols8, const int* row_limit,
+                                                   unsigned int* amax) {
+    pdl_wait();
+    pdl_trigger();
     const int64_t limit = row_limit ? min((int64_t)*row_limit, rows) : rows;
-    const int64_t n = limit * cols8;
-    float m = 0.f;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const uint4 raw = __ldg(x + i);
-        float v[8];
-        unpack8<F16>(raw, v);
+    const int64_t n = limit * cols8, step = (int64_t)gridDim.x * blockDim.x;
+    float m = 0.f, v[8];
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += 4 * step) {
+        uint4 raw[4];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) m = fmaxf(m, fabsf(v[k]));
+        for (int k = 0; k < 4; ++k) {
+            raw[k] = make_uint4(0, 0, 0, 0);
+            if (i + k * step < n) raw[k] = x[i + k * step];
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            unpack8<F16>(raw[k], v);
+            m = amax8(v, m);
+        }
     }
 #pragma unroll
     for (int d = 16; d >= 1; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
@@ -118,32 +156,31 @@ __global__ void __launch_bounds__(256) amax_kernel(const uint4* __restrict__ x, 
 }
 
 template <bool F16>
-__global__ void __launch_bounds__(256) quant_per_tensor_kernel(const uint4* __restrict__ x, uint2* __restrict__ q,
-                                                               float* __restrict__ scale_out, float* __restrict__ row_scales,
-                                                               int64_t rows, int cols8, const int* __restrict__ row_limit,
-                                                               const unsigned int* __restrict__ amax) {
+__global__ void __launch_bounds__(256) quant_per_tensor_kernel(const uint4* x, uint2* q, float* scale_out, float* row_scales,
+                                                               int64_t rows, int cols8, const int* row_limit,
+                                                               const unsigned int* amax) {
+    pdl_wait();
+    pdl_trigger();
     const int64_t limit = row_limit ? min((int64_t)*row_limit, rows) : rows;
     const float scale = __fdiv_rn(__uint_as_float(*amax), 448.0f);
     if (blockIdx.x == 0 && threadIdx.x == 0) scale_out[0] = scale;
-    const int64_t n = limit * cols8;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const uint4 raw = __ldg(x + i);
-        float v[8];
-        unpack8<F16>(raw, v);
-        uint32_t w[2];
+    const int64_t n = limit * cols8, step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += 4 * step) {
+        uint4 raw[4];
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(__fdiv_rn(v[4 * k], scale), __fdiv_rn(v[4 * k + 1], scale)),
-                                                         __NV_SATFINITE, __NV_E4M3);
-            const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(__fdiv_rn(v[4 * k + 2], scale), __fdiv_rn(v[4 * k + 3], scale)),
-                                                         __NV_SATFINITE, __NV_E4M3);
-            w[k] = lo | (hi << 16);
+        for (int k = 0; k < 4; ++k) {
+            raw[k] = make_uint4(0, 0, 0, 0);
+            if (i + k * step < n) raw[k] = x[i + k * step];
         }
-        q[i] = make_uint2(w[0], w[1]);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            float v[8];
+            unpack8<F16>(raw[k], v);
+            if (i + k * step < n) q[i + k * step] = quant_codes8(v, scale);
+        }
     }
     if (row_scales)
-        for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += (int64_t)gridDim.x * blockDim.x)
-            row_scales[r] = scale;
+        for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += step) row_scales[r] = scale;
 }
 
 }  // namespace
@@ -157,7 +194,7 @@ static bool input_is_f16(const aiter_tensor_t* input) {
 }
 
 void launch_quant_per_tensor(aiter_tensor_t* out, const aiter_tensor_t* input, aiter_tensor_t* scale, aiter_tensor_t* amax,
-                             aiter_tensor_t* row_scales, const aiter_tensor_t* row_limit, cudaStream_t stream) {
+                             aiter_tensor_t* row_scales, const aiter_tensor_t* row_limit, bool amax_cleared, cudaStream_t stream) {
     const bool f16 = input_is_f16(input);
     check_tensor(input, "input", -1, 2);
     check_tensor(out, "out", AITER_DTYPE_fp8, 2);
@@ -173,60 +210,47 @@ void launch_quant_per_tensor(aiter_tensor_t* out, const aiter_tensor_t* input, a
         B200_CHECK((int64_t)row_scales->numel_ >= rows, "row_scales needs one element per row");
     }
     if (row_limit) check_tensor(row_limit, "row_limit", AITER_DTYPE_i32, -1);
-    B200_CUDA(cudaMemsetAsync(amax->ptr, 0, sizeof(float), stream));
+    if (!amax_cleared) B200_CUDA(cudaMemsetAsync(amax->ptr, 0, sizeof(float), stream));
     if (rows == 0) return;
     const int64_t n = rows * (cols / 8);
     const int grid = (int)std::min<int64_t>((n + 255) / 256, (int64_t)sm_count(input->device_id) * 8);
     const int* lim = row_limit ? (const int*)row_limit->ptr : nullptr;
-    if (f16) {
-        amax_kernel<true><<<grid, 256, 0, stream>>>((const uint4*)input->ptr, rows, (int)(cols / 8), lim, (unsigned int*)amax->ptr);
-        quant_per_tensor_kernel<true><<<grid, 256, 0, stream>>>((const uint4*)input->ptr, (uint2*)out->ptr, (float*)scale->ptr,
-                                                                row_scales ? (float*)row_scales->ptr : nullptr, rows,
-                                                                (int)(cols / 8), lim, (const unsigned int*)amax->ptr);
-    } else {
-        amax_kernel<false><<<grid, 256, 0, stream>>>((const uint4*)input->ptr, rows, (int)(cols / 8), lim, (unsigned int*)amax->ptr);
-        quant_per_tensor_kernel<false><<<grid, 256, 0, stream>>>((const uint4*)input->ptr, (uint2*)out->ptr, (float*)scale->ptr,
-                                                                 row_scales ? (float*)row_scales->ptr : nullptr, rows,
-                                                                 (int)(cols / 8), lim, (const unsigned int*)amax->ptr);
-    }
-    B200_CUDA(cudaGetLastError());
+    float* per_row = row_scales ? (float*)row_scales->ptr : nullptr;
+    launch_pdl(f16 ? amax_kernel<true> : amax_kernel<false>, grid, 256, 0, stream, (const uint4*)input->ptr, rows, (int)(cols / 8),
+               lim, (unsigned int*)amax->ptr);
+    launch_pdl(f16 ? quant_per_tensor_kernel<true> : quant_per_tensor_kernel<false>, grid, 256, 0, stream, (const uint4*)input->ptr,
+               (uint2*)out->ptr, (float*)scale->ptr, per_row, rows, (int)(cols / 8), lim, (const unsigned int*)amax->ptr);
 }
 
 void launch_quant_per_token(aiter_tensor_t* out, const aiter_tensor_t* input, aiter_tensor_t* scales,
-                            const aiter_tensor_t* row_limit, int rows_factor, cudaStream_t stream) {
+                            const aiter_tensor_t* row_limit, int rows_factor, bool after_wait, cudaStream_t stream) {
     const bool f16 = input_is_f16(input);
     check_tensor(input, "input", -1, 2);
     check_tensor(out, "out", AITER_DTYPE_fp8, 2);
     check_tensor(scales, "scales", AITER_DTYPE_fp32, -1);
     const int64_t rows = input->shape[0], cols = input->shape[1];
     B200_CHECK(cols % 8 == 0 && cols >= 8, "row length must be a multiple of 8, got ", cols);
-    B200_CHECK(cols * 2 <= 200 * 1024, "row too long for the shared-memory row cache: ", cols);
     B200_CHECK(out->shape[0] == rows && out->shape[1] == cols, "out must have the shape of input");
     B200_CHECK((int64_t)scales->numel_ >= rows, "scales needs one element per row");
     B200_CHECK(((uintptr_t)input->ptr & 15) == 0 && ((uintptr_t)out->ptr & 7) == 0, "input must be 16-byte and out 8-byte aligned");
     B200_CHECK(rows_factor >= 1, "num_rows_factor must be >= 1, got ", rows_factor);
     if (row_limit) check_tensor(row_limit, "num_rows", AITER_DTYPE_i32, -1);
     if (rows == 0) return;
-    const size_t smem = (size_t)cols * 2;
-    static bool attr_set[64] = {false};
-    const int dev = input->device_id;
-    if (dev >= 64 || !attr_set[dev]) {
-        B200_CUDA(cudaFuncSetAttribute(quant_per_token_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        B200_CUDA(cudaFuncSetAttribute(quant_per_token_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        if (dev < 64) attr_set[dev] = true;
-    }
     const int* lim = row_limit ? (const int*)row_limit->ptr : nullptr;
-    if (f16)
-        quant_per_token_kernel<true><<<(unsigned)rows, 256, smem, stream>>>((const uint4*)input->ptr, (uint2*)out->ptr,
-                                                                             (float*)scales->ptr, (int)(cols / 8), lim, rows_factor);
-    else
-        quant_per_token_kernel<false><<<(unsigned)rows, 256, smem, stream>>>((const uint4*)input->ptr, (uint2*)out->ptr,
-                                                                              (float*)scales->ptr, (int)(cols / 8), lim, rows_factor);
-    B200_CUDA(cudaGetLastError());
+    const int cols8 = (int)(cols / 8);
+    const int grid = (int)std::min<int64_t>(rows, (int64_t)sm_count(input->device_id) * 8);
+    // pieces a thread keeps: the whole row for rows up to 4096 / 16384 elements, 8 of them for longer ones
+    auto go = [&](auto kernel) {
+        launch_pdl(kernel, grid, kRowThreads, 0, stream, (const uint4*)input->ptr, (uint2*)out->ptr, (float*)scales->ptr, rows, cols8,
+                   lim, rows_factor, after_wait);
+    };
+    if (cols8 <= 2 * kRowThreads) f16 ? go(quant_per_token_kernel<true, 2>) : go(quant_per_token_kernel<false, 2>);
+    else f16 ? go(quant_per_token_kernel<true, 8>) : go(quant_per_token_kernel<false, 8>);
 }
 
 void launch_quant_1x128(aiter_tensor_t* out, const aiter_tensor_t* input, aiter_tensor_t* scales,
-                        const aiter_tensor_t* num_rows, int rows_factor, int transpose_scale, cudaStream_t stream) {
+                        const aiter_tensor_t* num_rows, int rows_factor, int transpose_scale, bool after_wait,
+                        cudaStream_t stream) {
     const bool f16 = input_is_f16(input);
     check_tensor(input, "input", -1, -1);
     check_tensor(out, "out", AITER_DTYPE_fp8, -1);
@@ -243,18 +267,18 @@ void launch_quant_1x128(aiter_tensor_t* out, const aiter_tensor_t* input, aiter_
     B200_CHECK(rows_factor >= 1, "num_rows_factor must be >= 1, got ", rows_factor);
     if (num_rows) check_tensor(num_rows, "num_rows", AITER_DTYPE_i32, -1);
     if (groups == 0) return;
-    const int64_t blocks = (groups + kGroupsPerBlock - 1) / kGroupsPerBlock;
-    B200_CHECK(blocks < ((int64_t)1 << 31), "input too large");
     const int* lim = num_rows ? (const int*)num_rows->ptr : nullptr;
-    if (f16)
-        quant_1x128_kernel<true><<<(unsigned)blocks, kQuantThreads, 0, stream>>>(
-            (const uint4*)input->ptr, (uint2*)out->ptr, (float*)scales->ptr, groups, (int)(cols / 128), lim, rows_factor,
-            transpose_scale);
-    else
-        quant_1x128_kernel<false><<<(unsigned)blocks, kQuantThreads, 0, stream>>>(
-            (const uint4*)input->ptr, (uint2*)out->ptr, (float*)scales->ptr, groups, (int)(cols / 128), lim, rows_factor,
-            transpose_scale);
-    B200_CUDA(cudaGetLastError());
+    // four pieces per thread once that still gives every SM a few CTAs, one for small inputs (latency)
+    const int64_t pieces = groups * 16, sms = sm_count(input->device_id);
+    const int per_thread = pieces >= sms * 4 * kQuantThreads * 4 ? 4 : 1;
+    const int64_t blocks = (pieces + kQuantThreads * per_thread - 1) / (kQuantThreads * per_thread);
+    B200_CHECK(blocks < ((int64_t)1 << 31), "input too large");
+    auto go = [&](auto kernel) {
+        launch_pdl(kernel, (unsigned)blocks, kQuantThreads, 0, stream, (const uint4*)input->ptr, (uint2*)out->ptr, (float*)scales->ptr,
+                   groups, (int)(cols / 128), lim, rows_factor, transpose_scale, after_wait);
+    };
+    if (per_thread == 4) f16 ? go(quant_1x128_kernel<true, 4>) : go(quant_1x128_kernel<false, 4>);
+    else f16 ? go(quant_1x128_kernel<true, 1>) : go(quant_1x128_kernel<false, 1>);
 }
 
 }  // namespace b200

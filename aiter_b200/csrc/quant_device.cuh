@@ -31,29 +31,58 @@ __device__ __forceinline__ void unpack8(const uint4& raw, float (&v)[8]) {
     }
 }
 
+// Correctly rounded a / b given rb = RN(1/b): two FMA residual corrections (the first makes the quotient faithful, the
+// second then rounds it correctly), valid while nothing over- or underflows.
+__device__ __forceinline__ float div_rn_by(float a, float b, float rb) {
+    float q = a * rb;
+    q = fmaf(fmaf(-q, b, a), rb, q);
+    return fmaf(fmaf(-q, b, a), rb, q);
+}
+
+// Scales for which div_rn_by stands in for the IEEE division: quotients of magnitude up to 448 that matter (above e4m3's
+// smallest step) keep their residuals normal.
+__device__ __forceinline__ bool scale_is_tame(float scale) { return scale > 1e-30f && scale < 1e30f; }
+
+// Codes RNE_e4m3(v / scale) of eight values: five FMA-pipe operations per quotient from one reciprocal per scale instead of
+// the ~4x longer division sequence, which bound the quantisers at 2.3 TB/s.
+__device__ __forceinline__ uint2 quant_codes8(const float (&v)[8], float scale) {
+    float d[8];
+    if (scale_is_tame(scale)) {
+        const float rs = __frcp_rn(scale);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) d[i] = copysignf(div_rn_by(v[i], scale, rs), v[i]);   // the corrections lose the sign of -0
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) d[i] = __fdiv_rn(v[i], scale);
+    }
+    uint32_t w[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(d[4 * i], d[4 * i + 1]), __NV_SATFINITE, __NV_E4M3);
+        const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(d[4 * i + 2], d[4 * i + 3]), __NV_SATFINITE, __NV_E4M3);
+        w[i] = lo | (hi << 16);
+    }
+    return make_uint2(w[0], w[1]);
+}
+
+__device__ __forceinline__ float amax8(const float (&v)[8], float m = 0.f) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) m = fmaxf(m, fabsf(v[i]));
+    return m;
+}
+
 // 16 consecutive lanes of a warp (an aligned half-warp) hold one 128-element group, 8 elements each. Returns the
 // group's scale (on all 16 lanes) and this lane's 8 codes. Must be called by the whole warp (shuffles).
 template <bool F16>
 __device__ __forceinline__ float quant_group16(const uint4& raw, uint2& codes) {
     float v[8];
     unpack8<F16>(raw, v);
-    float amax = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
+    float amax = amax8(v);
 #pragma unroll
     for (int d = 8; d >= 1; d >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, d));
     float scale = __fdiv_rn(amax, 448.0f);
     if (scale == 0.f) scale = 1.f;
-    uint32_t w[2];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        float2 lo = make_float2(__fdiv_rn(v[4 * i], scale), __fdiv_rn(v[4 * i + 1], scale));
-        float2 hi = make_float2(__fdiv_rn(v[4 * i + 2], scale), __fdiv_rn(v[4 * i + 3], scale));
-        uint32_t a = __nv_cvt_float2_to_fp8x2(lo, __NV_SATFINITE, __NV_E4M3);
-        uint32_t b = __nv_cvt_float2_to_fp8x2(hi, __NV_SATFINITE, __NV_E4M3);
-        w[i] = a | (b << 16);
-    }
-    codes = make_uint2(w[0], w[1]);
+    codes = quant_codes8(v, scale);
     return scale;
 }
 

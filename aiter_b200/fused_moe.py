@@ -457,7 +457,7 @@ def _layer_launches(routes, quant_type, hidden_code):
     """Kernels behind one layer call (for ``_lib.launch_count``): sort, quantiser, two GEMMs, requantiser, final rounding."""
     quant = _lib._KERNELS_PER_CALL["b200_moe_quant_per_tensor"] if quant_type == QuantType.per_Tensor else 1
     a1 = 0 if hidden_code == dtypes.AITER_DTYPE[dtypes.fp8] else quant
-    return (3 if routes > 16384 else 1) + a1 + (0 if quant_type == QuantType.per_1x128 else quant) + 3
+    return (2 if routes > 16384 else 1) + a1 + (0 if quant_type == QuantType.per_1x128 else quant) + 3
 
 
 def fused_moe(
