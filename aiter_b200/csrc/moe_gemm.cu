@@ -13,8 +13,10 @@
 // Per tile and per 128-wide K block:
 //   warp 0      TMA-loads two [128 rows x 128 B] weight boxes (gate+up rows, or 256 output rows)
 //               into a 128B-swizzled shared-memory stage;
-//   warps 4-7   gather the 128 activation rows of the block (cp.async, 16 B chunks, same swizzle);
-//               completion is signalled by cp.async.mbarrier.arrive;
+//   warps 4-7   stage 1: gather the 128 activation rows of the block (cp.async, 16 B chunks, same swizzle), completion
+//               signalled by cp.async.mbarrier.arrive; stage 2: one thread loads them (contiguous) with TMA, 32 rows a box;
+//               32-row quarters that hold padding only are neither loaded nor promoted nor (skip_pads) written;
+//   warp 3      (stage 2: 5) prefetches the weight scales of the CTA's tiles into L2;
 //   warp 1      issues 4 tcgen05.mma (M128 N256 K32, e4m3 -> fp32) into one of two 256-column
 //               TMEM stages, then commits to free the smem stage and to publish the TMEM stage;
 //   warps 8-15  read the TMEM stage (tcgen05.ld) and fold it into fp32 registers with the block
@@ -40,7 +42,6 @@ namespace {
 constexpr int BM = 128;            // sorted rows per tile (== sort unit)
 constexpr int BK = 128;            // K elements (bytes) per pipeline step == scale block
 constexpr int BN = 256;            // UMMA N: 128 gate + 128 up columns, or 256 output columns
-constexpr int kStages = 3;         // shared-memory pipeline depth (4 measured no faster; the space stages stage 2's output)
 constexpr int kABytes = BM * BK;   // 16 KB
 constexpr int kBBytes = BN * BK;   // 32 KB
 constexpr int kThreads = 512;
@@ -65,19 +66,23 @@ constexpr int kProducerSleepNs = 100;  // back-off of the load roles while no st
 constexpr int kEpilogueSleepNs = B200_EPI_SLEEP_NS;   // back-off of the promotion warps while the UMMAs run
 constexpr uint32_t kIdesc = ptx::make_idesc_e4m3_f32(BM, BN);
 
-// shared memory map (offsets from a 1024-byte aligned base)
-constexpr int kOffA = 0;
-constexpr int kOffB = kOffA + kStages * kABytes;
-constexpr int kOffBar = kOffB + kStages * kBBytes;          // mbarriers (8 B each)
-constexpr int kNumBars = 2 * kStages + 4;
-constexpr int kOffTmemSlot = kOffBar + kNumBars * 8;
-constexpr int kOffAbort = kOffTmemSlot + 4;
-constexpr int kOffAmax = (kOffAbort + 4 + 15) & ~15;        // float [2 tiles][2 halves][128 rows]
-constexpr int kOffRowTab = kOffAmax + 2 * 2 * BM * 4;       // uint32 [2 tiles][128 rows]
+// Shared memory map (offsets from a 1024-byte aligned base). Stage 1 has room for four pipeline stages; stage 2 spends the
+// space of the fourth on staging its output rows.
 constexpr int kStageRowBytes = 272;                            // staged output row: 64 floats + 16 B (bank spread)
-constexpr int kOffStage = (kOffRowTab + 2 * BM * 4 + 15) & ~15;   // [8 warps][32 rows][kStageRowBytes] (stage 2)
-constexpr int kSmemUsed = kOffStage + 8 * 32 * kStageRowBytes;
-constexpr int kSmemBytes = kSmemUsed + 1024;                // slack for the 1024-byte alignment
+template <int STAGE>
+struct Smem {
+    static constexpr int kStages = STAGE == 1 ? 4 : 3;
+    static constexpr int kOffA = 0;
+    static constexpr int kOffB = kOffA + kStages * kABytes;
+    static constexpr int kOffBar = kOffB + kStages * kBBytes;   // mbarriers (8 B each)
+    static constexpr int kNumBars = 2 * kStages + 4;
+    static constexpr int kOffTmemSlot = kOffBar + kNumBars * 8;
+    static constexpr int kOffAbort = kOffTmemSlot + 4;
+    static constexpr int kOffAmax = (kOffAbort + 4 + 15) & ~15;   // stage 1: float [2 tiles][2 halves][128 rows]
+    static constexpr int kOffStage = (kOffAmax + (STAGE == 1 ? 2 * 2 * BM * 4 : 0) + 15) & ~15;   // stage 2: [8 warps][32 rows][kStageRowBytes]
+    static constexpr int kBytes = kOffStage + (STAGE == 1 ? 0 : 8 * 32 * kStageRowBytes) + 1024;   // + slack for the alignment
+};
+static_assert(Smem<1>::kBytes <= 232448 && Smem<2>::kBytes <= 232448, "shared memory of a CTA");
 
 struct GemmParams {
     const uint8_t* a;        // stage 1: a1 [M,K] by token; stage 2: a2 [P,K] by sorted row
@@ -100,6 +105,7 @@ struct GemmParams {
     float* a2_scale;         // stage 1 out [P, I/128]
     float* acc;              // stage 2 out [M, H] fp32
     int* status;
+    int skip_pads;           // stage 1: rows of padding are not written (stage 2 does not read them)
     int use_weight;          // multiply this stage's GEMM result by the route weight (sorted_w)
     long long wait_limit;    // SM clocks after which a device-side wait gives up (sets status, the CTA winds down)
     int stall_producer;      // self-test only: the weight producer loads nothing, so every wait downstream runs out
@@ -151,6 +157,25 @@ __device__ __forceinline__ void fold16(float2* acc, const uint32_t* v, float2 s)
         acc[j] = __ffma2_rn(make_float2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1])), s, acc[j]);
 }
 
+// Weight scales of all tiles of this CTA -> L2, a lane per tile (a few hundred bytes each). Without it every tile starts with
+// a DRAM round trip on the promotion warps' path.
+template <int STAGE, bool PT>
+__device__ __forceinline__ void prefetch_weight_scales(const GemmParams& p, int lane, int total_tiles) {
+    const int unit = PT ? 128 : p.KB;          // floats of one 128-row group
+    const int groups = p.n_rows / 128;
+    for (int t = blockIdx.x + lane * gridDim.x; t < total_tiles; t += 32 * gridDim.x) {
+        const int blk = t / p.n_tiles, nt = t - blk * p.n_tiles + p.nt0;
+        const int g0 = STAGE == 1 ? nt : nt * 2;
+        const int gap = STAGE == 1 ? p.inter / 128 : min(1, groups - 1 - g0);   // second 128-row group of the tile
+        const float* w = p.w_scale + (size_t)(p.sorted_eids[blk] * groups + g0) * unit;
+        for (int i = 0; i < unit + 31; i += 32) {   // an address in every 128-byte line, whatever the alignment
+            const float* at = w + min(i, unit - 1);
+            ptx::prefetch_l2(at);
+            ptx::prefetch_l2(at + gap * unit);
+        }
+    }
+}
+
 // PT = false: 1x128 activation scales and 128x128 weight scales (QuantType.per_1x128 / per_128x128).
 // PT = true : one scale per activation row and one per weight output channel (QuantType.per_Token); the
 //             row scale rides on every K step, the channel scales are applied once in the epilogue, and
@@ -159,26 +184,28 @@ __device__ __forceinline__ void fold16(float2* acc, const uint32_t* v, float2 s)
 //             unrolled epilogue doubles in size and the SiLU path measurably slows down.
 template <int STAGE, bool PT, int ACT>
 __global__ void __launch_bounds__(kThreads, 1)
-moe_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const GemmParams p) {
+moe_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_a, const GemmParams p) {
+    using S = Smem<STAGE>;
+    constexpr int kStages = S::kStages;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const uint32_t sbase = ptx::smem_u32(smem);
-    const uint32_t sA = sbase + kOffA, sB = sbase + kOffB;
-    const uint32_t bar0 = sbase + kOffBar;
+    const uint32_t sA = sbase + S::kOffA, sB = sbase + S::kOffB;
+    const uint32_t bar0 = sbase + S::kOffBar;
     auto full_bar = [&](int s) { return bar0 + 8u * s; };
     auto empty_bar = [&](int s) { return bar0 + 8u * (kStages + s); };
     auto tfull_bar = [&](int s) { return bar0 + 8u * (2 * kStages + s); };
     auto tempty_bar = [&](int s) { return bar0 + 8u * (2 * kStages + 2 + s); };
-    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + kOffTmemSlot);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + kOffAbort);
-    float* amax_x = reinterpret_cast<float*>(smem + kOffAmax);
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + S::kOffTmemSlot);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + S::kOffAbort);
+    float* amax_x = reinterpret_cast<float*>(smem + S::kOffAmax);
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
     const int lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
-            ptx::mbar_init(full_bar(s), BM + 1);   // 128 gather threads + the TMA thread
+            ptx::mbar_init(full_bar(s), STAGE == 1 ? BM + 1 : 2);   // 128 gather threads (stage 2: one) + the weight thread
             ptx::mbar_init(empty_bar(s), 1);       // one tcgen05.commit
         }
         for (int s = 0; s < 2; ++s) {
@@ -188,6 +215,7 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const GemmParams p) 
         *abort_flag = 0;
         ptx::fence_mbar_init();
         ptx::prefetch_tensormap(&tmap_w);
+        if (STAGE == 2) ptx::prefetch_tensormap(&tmap_a);
     }
     if (warp == 2) {
         ptx::tmem_alloc(ptx::smem_u32(const_cast<uint32_t*>(tmem_slot)), kTmemCols);
@@ -251,9 +279,9 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const GemmParams p) 
                     if (!PT || kb == 0)
                         if (!(ok = ptx::mbar_wait(tempty_bar(ts), tph ^ 1u, abort_flag, p.wait_limit))) break;
                     if (!(ok = ptx::mbar_wait(full_bar(s), ph, abort_flag, p.wait_limit))) break;
-                    // the activation rows were written by cp.async (generic proxy); order them
+                    // stage 1's activation rows were written by cp.async (generic proxy); order them
                     // before the tensor core's async-proxy reads
-                    ptx::fence_proxy_async();
+                    if (STAGE == 1) ptx::fence_proxy_async();
                     ptx::tc_fence_after();
                     const uint64_t da = ptx::make_kmajor_sw128_desc(sA + s * kABytes);
                     const uint64_t db = ptx::make_kmajor_sw128_desc(sB + s * kBBytes);
@@ -265,63 +293,94 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const GemmParams p) 
                     if (!PT || kb == p.KB - 1) ptx::umma_commit(tfull_bar(ts));
                 }
             }
+        } else if (STAGE == 1 && warp == 3 && !(PT && p.w_scale_by_expert)) {
+            prefetch_weight_scales<STAGE, PT>(p, lane, total_tiles);
         }
     } else if (warp < kEpiWarp0) {
         // -------------------------------------------------------------------- activation gather
         ptx::setmaxnreg_dec<kRegsGather>();
-        const int r = threadIdx.x - kGatherWarp0 * 32;   // row whose scale / row offset this thread owns
-        // Copy mapping: 8 consecutive lanes fetch the eight 16-byte chunks of one 128-byte row segment,
-        // so a warp-wide cp.async touches 4 whole cache lines (not 32 partial ones). Pass i of a
-        // thread covers row gw*32 + i*4 + lane/8.
-        const int gw = r >> 5, sub = (r & 31) >> 3;
-        const uint32_t chunk = (uint32_t)(r & 7);
-        uint32_t* row_tab = reinterpret_cast<uint32_t*>(smem + kOffRowTab);   // [2][128] source rows
         uint32_t it = 0;
-        uint32_t tile_par = 0;
         bool ok = true;
-        int sid_next = 0;   // sorted id of this thread's row in the next tile, fetched one tile ahead
-        if (STAGE == 1 && (int)blockIdx.x < total_tiles)
-            sid_next = p.sorted_ids[((int)blockIdx.x / p.n_tiles) * BM + r];
-        for (int t = blockIdx.x; ok && t < total_tiles; t += gridDim.x, tile_par ^= 1u) {
-            const int blk = t / p.n_tiles, nt = t - blk * p.n_tiles + p.nt0;
-            const int prow = blk * BM + r;
-            uint32_t my_row;                 // source row of tile row r, or 0xFFFFFFFF for padding
-            if (STAGE == 1) {
+        if (STAGE == 2) {
+            // Sorted rows are contiguous: one thread fetches them with TMA, 32 rows a box, and leaves out the boxes that
+            // hold padding only (decode: three of four; the tensor core then computes on what the buffer held before, in
+            // rows nobody reads). Rows of a tile's padding are never read from HBM or L2 for their own sake.
+            if (warp == kGatherWarp0) {
+                int ids[4] = {0, 0, 0, 0};   // sorted ids of the next tile's rows (one per quarter and lane)
+                auto fetch = [&](int t) {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) ids[q] = p.sorted_ids[(t / p.n_tiles) * BM + q * 32 + lane];
+                };
+                if ((int)blockIdx.x < total_tiles) fetch(blockIdx.x);
+                for (int t = blockIdx.x; ok && t < total_tiles; t += gridDim.x) {
+                    const int row0 = (t / p.n_tiles) * BM;
+                    uint32_t live = 0;
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) live |= (__any_sync(0xffffffffu, (ids[q] & 0xFFFFFF) < tokens) ? 1u : 0u) << q;
+                    if (t + (int)gridDim.x < total_tiles) fetch(t + gridDim.x);
+                    if (lane == 0) {
+                        for (int kb = 0; kb < p.KB; ++kb, ++it) {
+                            const int s = it % kStages;
+                            const uint32_t ph = (it / kStages) & 1u;
+                            if (!(ok = ptx::mbar_wait<kTmaSleepNs>(empty_bar(s), ph ^ 1u, abort_flag, p.wait_limit))) break;
+                            ptx::mbar_arrive_expect_tx(full_bar(s), __popc(live) * (kABytes / 4));
+#pragma unroll
+                            for (int q = 0; q < 4; ++q)
+                                if ((live >> q) & 1u)
+                                    ptx::tma_load_2d(sA + s * kABytes + q * (kABytes / 4), &tmap_a, kb * BK, row0 + q * 32, full_bar(s));
+                        }
+                    }
+                    ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+                }
+            } else if (warp == kGatherWarp0 + 1 && !(PT && p.w_scale_by_expert)) {
+                prefetch_weight_scales<STAGE, PT>(p, lane, total_tiles);
+            }
+        } else {
+            const int r = threadIdx.x - kGatherWarp0 * 32;   // row of the tile whose sorted id this thread holds
+            // Copy mapping: 8 consecutive lanes fetch the eight 16-byte chunks of one 128-byte row segment, so a warp-wide
+            // cp.async touches 4 whole cache lines (not 32 partial ones). A warp copies its own 32 rows: pass i of a thread
+            // covers row i*4 + lane/8 of them.
+            const int gw = r >> 5, sub = lane >> 3;
+            const uint32_t chunk = (uint32_t)(lane & 7);
+            int sid_next = 0;   // sorted id of this thread's row in the next tile, fetched one tile ahead
+            if ((int)blockIdx.x < total_tiles) sid_next = p.sorted_ids[((int)blockIdx.x / p.n_tiles) * BM + r];
+            for (int t = blockIdx.x; ok && t < total_tiles; t += gridDim.x) {
                 const int tok = sid_next & 0xFFFFFF;
-                my_row = tok < tokens ? (uint32_t)tok : 0xFFFFFFFFu;
-                if (t + (int)gridDim.x < total_tiles)
-                    sid_next = p.sorted_ids[((t + (int)gridDim.x) / p.n_tiles) * BM + r];
-            } else {
-                my_row = (uint32_t)prow;
-            }
-            row_tab[tile_par * BM + r] = my_row;
-            ptx::named_barrier(2, BM);       // the 128 gather threads; table of the previous tile is
-                                             // untouched (other parity), so one barrier per tile suffices
-            // source of pass i in 16-byte units from p.a (32 bits cover 64 GB), validity as a bit mask, and the
-            // two swizzled destination offsets (even / odd pass): few registers, this role runs with 56
-            uint32_t src16[8], vmask = 0;
+                const uint32_t my_row = tok < tokens ? (uint32_t)tok : 0xFFFFFFFFu;   // 0xFFFFFFFF: padding
+                if (t + (int)gridDim.x < total_tiles) sid_next = p.sorted_ids[((t + (int)gridDim.x) / p.n_tiles) * BM + r];
+                // 32 rows of padding are not copied at all: their results stay in TMEM lanes that nobody reads
+                const bool warp_live = __any_sync(0xffffffffu, tok < tokens);
+                // source of pass i in 16-byte units from p.a (32 bits cover 64 GB), validity as a bit mask, and the
+                // two swizzled destination offsets (even / odd pass): few registers, this role runs with 56
+                uint32_t src16[8], vmask = 0;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const uint32_t sr = row_tab[tile_par * BM + gw * 32 + i * 4 + sub];
-                const bool live = sr != 0xFFFFFFFFu;   // pads: zero-filled rows
-                vmask |= (live ? 1u : 0u) << i;
-                src16[i] = (live ? sr : 0u) * (uint32_t)(p.K >> 4) + chunk;
-            }
-            const uint32_t row0 = (uint32_t)(gw * 32 + sub);   // row of pass i: row0 + 4 i, so (row & 7) = sub or 4 + sub
-            const uint32_t d_even = row0 * BK + ((chunk ^ (uint32_t)sub) << 4);
-            const uint32_t d_odd = row0 * BK + ((chunk ^ (uint32_t)(4 + sub)) << 4);
-            for (int kb = 0; kb < p.KB; ++kb, ++it) {
-                const int s = it % kStages;
-                const uint32_t ph = (it / kStages) & 1u;
-                if (!(ok = ptx::mbar_wait<kProducerSleepNs>(empty_bar(s), ph ^ 1u, abort_flag, p.wait_limit))) break;
-                const uint32_t dst = sA + s * kABytes;
+                for (int i = 0; i < 8; ++i) {
+                    const uint32_t sr = __shfl_sync(0xffffffffu, my_row, i * 4 + sub);
+                    const bool live = sr != 0xFFFFFFFFu;   // pads beside live rows: zero-filled
+                    vmask |= (live ? 1u : 0u) << i;
+                    src16[i] = (live ? sr : 0u) * (uint32_t)(p.K >> 4) + chunk;
+                }
+                const uint32_t row0 = (uint32_t)(gw * 32 + sub);   // row of pass i: row0 + 4 i, so (row & 7) = sub or 4 + sub
+                const uint32_t d_even = row0 * BK + ((chunk ^ (uint32_t)sub) << 4);
+                const uint32_t d_odd = row0 * BK + ((chunk ^ (uint32_t)(4 + sub)) << 4);
+                for (int kb = 0; kb < p.KB; ++kb, ++it) {
+                    const int s = it % kStages;
+                    const uint32_t ph = (it / kStages) & 1u;
+                    if (!(ok = ptx::mbar_wait<kProducerSleepNs>(empty_bar(s), ph ^ 1u, abort_flag, p.wait_limit))) break;
+                    if (!warp_live) {
+                        ptx::mbar_arrive(full_bar(s));
+                        continue;
+                    }
+                    const uint32_t dst = sA + s * kABytes;
 #pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    ptx::cp_async16(dst + ((i & 1) ? d_odd : d_even) + i * 4 * BK, p.a + ((size_t)src16[i] << 4) + (size_t)kb * BK,
-                                    ((vmask >> i) & 1u) ? 16u : 0u);
-                // the arrival is delivered by the copy engine when this thread's copies have landed,
-                // so the thread can go on to the next stage at once (all kStages stay in flight)
-                ptx::cp_async_mbar_arrive(full_bar(s));
+                    for (int i = 0; i < 8; ++i)
+                        ptx::cp_async16(dst + ((i & 1) ? d_odd : d_even) + i * 4 * BK, p.a + ((size_t)src16[i] << 4) + (size_t)kb * BK,
+                                        ((vmask >> i) & 1u) ? 16u : 0u);
+                    // the arrival is delivered by the copy engine when this thread's copies have landed,
+                    // so the thread can go on to the next stage at once (all kStages stay in flight)
+                    ptx::cp_async_mbar_arrive(full_bar(s));
+                }
+                ok = __all_sync(0xffffffffu, ok) != 0;   // the next tile starts with shuffles
             }
         }
         ptx::cp_async_commit();
@@ -422,7 +481,8 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const GemmParams p) 
             }
             if (!ok) break;
 
-            if (PT && !p.w_scale_by_expert) {
+            const bool warp_out = warp_live || (STAGE == 1 && !p.skip_pads);   // this warp has rows to write
+            if (PT && !p.w_scale_by_expert && warp_out) {
                 // weight scales per output channel: column j of the first group is weight row
                 // e*n_rows + c0 + j, of the second group c1 + j (all lanes read the same addresses)
                 const int e = p.sorted_eids[blk];
@@ -441,6 +501,7 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const GemmParams p) 
             }
 
             if (STAGE == 1 && PT) {
+                if (!warp_out) continue;
                 // SiLU(gate)*up -> bf16, written in sorted-row order; the row-wise quantisation follows
                 uint32_t w[32];
 #pragma unroll
@@ -459,11 +520,14 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const GemmParams p) 
                     }
                 }
                 uint4* dst = reinterpret_cast<uint4*>(p.a2 + ((size_t)prow * p.inter + nt * 128 + half * 64) * 2);
+                if (valid || !p.skip_pads) {
 #pragma unroll
-                for (int j = 0; j < 8; ++j) dst[j] = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+                    for (int j = 0; j < 8; ++j) dst[j] = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+                }
             } else if (STAGE == 1) {
                 // SiLU(gate)*up in fp32 -> bf16 (RNE) -> 1x128 requant, as the oracle does:
                 // aiter/fused_moe.py:3668-3681 then aiter/ops/quant.py:64-94 on the bf16 values.
+                if (!warp_out) continue;
                 float amax = 0.f;
 #pragma unroll
                 for (int j0 = 0; j0 < 32; j0 += 4) {   // acc[j] is overwritten by the two activations it feeds
@@ -484,7 +548,7 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const GemmParams p) 
                 }
                 float* ax = amax_x + tile_par * (2 * BM);
                 ax[half * BM + r] = amax;
-                ptx::named_barrier(1, kEpiThreads);
+                ptx::named_barrier(1 + q, 64);   // the two warps that hold these 32 rows
                 amax = fmaxf(amax, ax[(half ^ 1) * BM + r]);
                 float scale = __fdiv_rn(amax, 448.0f);
                 if (scale == 0.f) scale = 1.f;
@@ -511,9 +575,12 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const GemmParams p) 
                     }
                 }
                 uint4* dst = reinterpret_cast<uint4*>(p.a2 + (size_t)prow * p.inter + nt * 128 + half * 64);
+                const bool store = valid || !p.skip_pads;
+                if (store) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) dst[j] = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
-                if (half == 0) p.a2_scale[(size_t)prow * (p.inter / 128) + nt] = scale;
+                    for (int j = 0; j < 4; ++j) dst[j] = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+                }
+                if (half == 0 && store) p.a2_scale[(size_t)prow * (p.inter / 128) + nt] = scale;
             } else {
                 // out[token] += weight * row  (aiter/fused_moe.py:3802-3811) as fp32 reductions in L2; the
                 // weight is already in the accumulators (it rode on the per-step scales).
@@ -524,7 +591,7 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const GemmParams p) 
                 // red.global.v4 from registers or as bulk reductions (plain stores: ~35 B/clock), i.e. ~6k clocks
                 // per tile that the MMA warp, at most two K steps ahead, waits out; hiding them needs a buffer
                 // for the whole 128 KB tile, which neither shared nor tensor memory has room for.
-                const uint32_t srow = sbase + kOffStage + (uint32_t)((warp - kEpiWarp0) * 32 + lane) * kStageRowBytes;
+                const uint32_t srow = sbase + S::kOffStage + (uint32_t)((warp - kEpiWarp0) * 32 + lane) * kStageRowBytes;
                 const int n_groups = (nt * 256 + 128 < p.n_rows) ? 2 : 1;
                 if (valid) {
                     float* orow = p.acc + (size_t)tok * p.acc_ld + (nt - p.nt0) * 256 + half * 64;
@@ -583,30 +650,32 @@ EncodeTiledFn encode_tiled_fn() {
     return fn;
 }
 
-// 2-D view [rows, K] of an fp8 weight tensor [E, n_rows, K]; boxes of 128 rows x 128 bytes, 128B swizzle. Encoding a map
+// 2-D view [rows, K] of an fp8 matrix (weights [E, n_rows, K] in boxes of 128 rows x 128 bytes, stage 2's activations in
+// boxes of 32 rows), 128B swizzle. Encoding a map
 // costs a few microseconds of host time, so the last maps are kept (per thread) and reused while pointer and shape
 // repeat, as they do from layer call to layer call.
-CUtensorMap make_weight_map(const void* ptr, uint64_t rows, uint64_t K) {
+CUtensorMap make_map(const void* ptr, uint64_t rows, uint64_t K, uint32_t box_rows) {
     struct Entry {
         const void* ptr;
         uint64_t rows, K;
+        uint32_t box_rows;
         CUtensorMap map;
     };
     constexpr int kEntries = 16;
     static thread_local Entry cache[kEntries];
     static thread_local int next = 0, used = 0;
     for (int i = 0; i < used; ++i)
-        if (cache[i].ptr == ptr && cache[i].rows == rows && cache[i].K == K) return cache[i].map;
+        if (cache[i].ptr == ptr && cache[i].rows == rows && cache[i].K == K && cache[i].box_rows == box_rows) return cache[i].map;
     CUtensorMap m;
     cuuint64_t dims[2] = {K, rows};
     cuuint64_t strides[1] = {K};
-    cuuint32_t box[2] = {128, 128};
+    cuuint32_t box[2] = {128, box_rows};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = encode_tiled_fn()(&m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(ptr), dims, strides,
                                    box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     B200_CHECK(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled failed with code ", (int)r);
-    cache[next] = Entry{ptr, rows, K, m};
+    cache[next] = Entry{ptr, rows, K, box_rows, m};
     next = (next + 1) % kEntries;
     if (used < kEntries) ++used;
     return m;
@@ -618,12 +687,12 @@ long long g_wait_limit = ptx::kWaitLimitCycles;
 int g_stall_producer = 0;
 
 template <int STAGE, bool PT, int ACT = 0>
-void launch_gemm(const CUtensorMap& tmap, const GemmParams& p, int64_t max_tiles, int dev, cudaStream_t stream,
+void launch_gemm(const CUtensorMap& tmap, const CUtensorMap& tmap_a, const GemmParams& p, int64_t max_tiles, int dev, cudaStream_t stream,
                  int sm_margin = 0) {
     static bool attr_set[64] = {false};
     if (dev >= 64 || !attr_set[dev]) {
         B200_CUDA(cudaFuncSetAttribute(moe_gemm_kernel<STAGE, PT, ACT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       kSmemBytes));
+                                       Smem<STAGE>::kBytes));
         cudaFuncAttributes fa;
         B200_CUDA(cudaFuncGetAttributes(&fa, moe_gemm_kernel<STAGE, PT, ACT>));
         B200_CHECK((int64_t)fa.numRegs * kThreads >= kRegDemand, "GEMM kernel was compiled with ", fa.numRegs,
@@ -641,7 +710,7 @@ void launch_gemm(const CUtensorMap& tmap, const GemmParams& p, int64_t max_tiles
     // Overlapping the launch with the kernel before it pays while the layer is short. With tens of tiles per SM the few
     // microseconds are nothing, and at the power limit the early CTAs cost more than they give (1-2 % at 65 K routes).
     const bool overlap = max_tiles <= 64 * grid;
-    launch_kernel(overlap, moe_gemm_kernel<STAGE, PT, ACT>, (unsigned)grid, kThreads, kSmemBytes, stream, tmap, q);
+    launch_kernel(overlap, moe_gemm_kernel<STAGE, PT, ACT>, (unsigned)grid, kThreads, Smem<STAGE>::kBytes, stream, tmap, tmap_a, q);
 }
 
 }  // namespace
@@ -655,7 +724,7 @@ void launch_moe_stage1(const aiter_tensor_t* a1, const aiter_tensor_t* a1_scale,
                        const aiter_tensor_t* w1_scale, const aiter_tensor_t* sorted_ids,
                        const aiter_tensor_t* sorted_eids, const aiter_tensor_t* num_valid, aiter_tensor_t* a2,
                        aiter_tensor_t* a2_scale, aiter_tensor_t* status, int quant_type,
-                       const aiter_tensor_t* sorted_w, int activation, cudaStream_t stream) {
+                       const aiter_tensor_t* sorted_w, int activation, bool skip_pads, cudaStream_t stream) {
     B200_CHECK(activation == 0 || activation == 1, "activation must be Silu (0) or Gelu (1), got ", activation);
     if (sorted_w) {
         check_tensor(sorted_w, "sorted_weights", AITER_DTYPE_fp32, 1);
@@ -722,13 +791,14 @@ void launch_moe_stage1(const aiter_tensor_t* a1, const aiter_tensor_t* a1_scale,
     p.a2_scale = pt ? nullptr : (float*)a2_scale->ptr;
     p.status = (int*)status->ptr;
     p.sorted_w = sorted_w ? (const float*)sorted_w->ptr : nullptr;
+    p.skip_pads = skip_pads;
     p.use_weight = sorted_w != nullptr;   // doweight_stage1 (aiter/fused_moe.py:3651-3652)
-    CUtensorMap tmap = make_weight_map(w1->ptr, (uint64_t)(E * N2), (uint64_t)H);
+    CUtensorMap tmap = make_map(w1->ptr, (uint64_t)(E * N2), (uint64_t)H, 128);
     const int64_t max_tiles = ((int64_t)sorted_ids->numel_ / BM) * p.n_tiles;
-    if (pt && activation == 1) launch_gemm<1, true, 1>(tmap, p, max_tiles, a1->device_id, stream);
-    else if (pt) launch_gemm<1, true, 0>(tmap, p, max_tiles, a1->device_id, stream);
-    else if (activation == 1) launch_gemm<1, false, 1>(tmap, p, max_tiles, a1->device_id, stream);
-    else launch_gemm<1, false, 0>(tmap, p, max_tiles, a1->device_id, stream);
+    if (pt && activation == 1) launch_gemm<1, true, 1>(tmap, tmap, p, max_tiles, a1->device_id, stream);
+    else if (pt) launch_gemm<1, true, 0>(tmap, tmap, p, max_tiles, a1->device_id, stream);
+    else if (activation == 1) launch_gemm<1, false, 1>(tmap, tmap, p, max_tiles, a1->device_id, stream);
+    else launch_gemm<1, false, 0>(tmap, tmap, p, max_tiles, a1->device_id, stream);
 }
 
 void launch_moe_stage2(const aiter_tensor_t* a2, const aiter_tensor_t* a2_scale, const aiter_tensor_t* w2,
@@ -804,10 +874,11 @@ void launch_moe_stage2(const aiter_tensor_t* a2, const aiter_tensor_t* a2_scale,
     p.acc = (float*)acc->ptr + (full_width ? col_begin : 0);
     p.status = (int*)status->ptr;
     p.use_weight = doweight != 0;
-    CUtensorMap tmap = make_weight_map(w2->ptr, (uint64_t)(E * H), (uint64_t)I);
+    CUtensorMap tmap = make_map(w2->ptr, (uint64_t)(E * H), (uint64_t)I, 128);
+    CUtensorMap tmap_a = make_map(a2->ptr, (uint64_t)P, (uint64_t)I, 32);
     const int64_t max_tiles = ((int64_t)sorted_ids->numel_ / BM) * p.n_tiles;
-    if (pt) launch_gemm<2, true>(tmap, p, max_tiles, a2->device_id, stream, sm_margin);
-    else launch_gemm<2, false>(tmap, p, max_tiles, a2->device_id, stream, sm_margin);
+    if (pt) launch_gemm<2, true>(tmap, tmap_a, p, max_tiles, a2->device_id, stream, sm_margin);
+    else launch_gemm<2, false>(tmap, tmap_a, p, max_tiles, a2->device_id, stream, sm_margin);
 }
 
 }  // namespace b200

@@ -71,12 +71,16 @@ __global__ void __launch_bounds__(kQuantThreads) quant_1x128_kernel(
 // registers (CACHE 16-byte pieces per thread) between the amax pass and the conversion pass; what does not fit there is
 // read again (L1/L2). Same rounding sequence as above (aiter/ops/quant.py:64-94 over the last dimension). Rows at or past
 // *row_limit * rows_factor (if given) are skipped: the grid is a few CTAs per SM that stride over the rows below it, so a
-// sorted buffer's padded tail costs no CTAs.
+// sorted buffer's padded tail costs no CTAs. sorted_ids (if given; row_limit is then the sort's {rows, tokens} pair): rows of
+// a sorted buffer that hold padding are skipped, neither read nor written (a decode batch has ~16 of them per live row).
+__device__ __forceinline__ bool is_padding(const int* sorted_ids, const int* num_valid, int M, int64_t row) {
+    return sorted_ids && (sorted_ids[row] & 0xFFFFFF) >= min(num_valid[1], M);
+}
 constexpr int kRowThreads = 256;
 template <bool F16, int CACHE>
 __global__ void __launch_bounds__(kRowThreads) quant_per_token_kernel(const uint4* x, uint2* q, float* scales, int64_t rows,
                                                                       int cols8, const int* row_limit, int rows_factor,
-                                                                      bool after_wait) {
+                                                                      const int* sorted_ids, int M, bool after_wait) {
     __shared__ float red[2][kRowThreads / 32];
     if (after_wait) pdl_wait();
     pdl_trigger();
@@ -84,6 +88,7 @@ __global__ void __launch_bounds__(kRowThreads) quant_per_token_kernel(const uint
     if (row_limit) rows = min(rows, (int64_t)*row_limit * rows_factor);
     int par = 0;
     for (int64_t row = blockIdx.x; row < rows; row += gridDim.x, par ^= 1) {
+        if (is_padding(sorted_ids, row_limit, M, row)) continue;
         const uint4* xr = x + row * cols8;
         uint4 raw[CACHE];
         float amax = 0.f, v[8];
@@ -129,12 +134,27 @@ __global__ void __launch_bounds__(kRowThreads) quant_per_token_kernel(const uint
 // the maximum over the rows below *row_limit goes to amax[0] (non-negative floats order like their bit patterns,
 // so an integer atomicMax does it), then every row is converted with the one scale, which is also written to
 // scale[0] and, if asked, once per row to row_scales (the GEMM kernels take one activation scale per row).
+// With sorted_ids a CTA takes whole rows, so that padding rows can be left out; else the buffer is one flat range.
 template <bool F16>
 __global__ void __launch_bounds__(256) amax_kernel(const uint4* x, int64_t rows, int cols8, const int* row_limit,
-                                                   unsigned int* amax) {
+                                                   const int* sorted_ids, int M, unsigned int* amax) {
     pdl_wait();
     pdl_trigger();
     const int64_t limit = row_limit ? min((int64_t)*row_limit, rows) : rows;
+    if (sorted_ids) {
+        float m = 0.f, v[8];
+        for (int64_t row = blockIdx.x; row < limit; row += gridDim.x) {
+            if (is_padding(sorted_ids, row_limit, M, row)) continue;
+            for (int i = threadIdx.x; i < cols8; i += 256) {
+                unpack8<F16>(x[row * cols8 + i], v);
+                m = amax8(v, m);
+            }
+        }
+#pragma unroll
+        for (int d = 16; d >= 1; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
+        if ((threadIdx.x & 31) == 0 && m > 0.f) atomicMax(amax, __float_as_uint(m));
+        return;
+    }
     const int64_t n = limit * cols8, step = (int64_t)gridDim.x * blockDim.x;
     float m = 0.f, v[8];
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += 4 * step) {
@@ -158,12 +178,23 @@ __global__ void __launch_bounds__(256) amax_kernel(const uint4* x, int64_t rows,
 template <bool F16>
 __global__ void __launch_bounds__(256) quant_per_tensor_kernel(const uint4* x, uint2* q, float* scale_out, float* row_scales,
                                                                int64_t rows, int cols8, const int* row_limit,
-                                                               const unsigned int* amax) {
+                                                               const int* sorted_ids, int M, const unsigned int* amax) {
     pdl_wait();
     pdl_trigger();
     const int64_t limit = row_limit ? min((int64_t)*row_limit, rows) : rows;
     const float scale = __fdiv_rn(__uint_as_float(*amax), 448.0f);
     if (blockIdx.x == 0 && threadIdx.x == 0) scale_out[0] = scale;
+    if (sorted_ids) {
+        float v[8];
+        for (int64_t row = blockIdx.x; row < limit; row += gridDim.x) {
+            if (is_padding(sorted_ids, row_limit, M, row)) continue;
+            for (int i = threadIdx.x; i < cols8; i += 256) {
+                unpack8<F16>(x[row * cols8 + i], v);
+                q[row * cols8 + i] = quant_codes8(v, scale);
+            }
+        }
+        return;
+    }
     const int64_t n = limit * cols8, step = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += 4 * step) {
         uint4 raw[4];
@@ -194,7 +225,7 @@ static bool input_is_f16(const aiter_tensor_t* input) {
 }
 
 void launch_quant_per_tensor(aiter_tensor_t* out, const aiter_tensor_t* input, aiter_tensor_t* scale, aiter_tensor_t* amax,
-                             aiter_tensor_t* row_scales, const aiter_tensor_t* row_limit, bool amax_cleared, cudaStream_t stream) {
+                             aiter_tensor_t* row_scales, const aiter_tensor_t* row_limit, bool amax_cleared, const int* sorted_ids, int M, cudaStream_t stream) {
     const bool f16 = input_is_f16(input);
     check_tensor(input, "input", -1, 2);
     check_tensor(out, "out", AITER_DTYPE_fp8, 2);
@@ -212,18 +243,20 @@ void launch_quant_per_tensor(aiter_tensor_t* out, const aiter_tensor_t* input, a
     if (row_limit) check_tensor(row_limit, "row_limit", AITER_DTYPE_i32, -1);
     if (!amax_cleared) B200_CUDA(cudaMemsetAsync(amax->ptr, 0, sizeof(float), stream));
     if (rows == 0) return;
-    const int64_t n = rows * (cols / 8);
+    const int64_t n = sorted_ids ? rows * 256 : rows * (cols / 8);   // a CTA per row, or per 256 pieces
     const int grid = (int)std::min<int64_t>((n + 255) / 256, (int64_t)sm_count(input->device_id) * 8);
     const int* lim = row_limit ? (const int*)row_limit->ptr : nullptr;
     float* per_row = row_scales ? (float*)row_scales->ptr : nullptr;
     launch_pdl(f16 ? amax_kernel<true> : amax_kernel<false>, grid, 256, 0, stream, (const uint4*)input->ptr, rows, (int)(cols / 8),
-               lim, (unsigned int*)amax->ptr);
+               lim, sorted_ids, M, (unsigned int*)amax->ptr);
     launch_pdl(f16 ? quant_per_tensor_kernel<true> : quant_per_tensor_kernel<false>, grid, 256, 0, stream, (const uint4*)input->ptr,
-               (uint2*)out->ptr, (float*)scale->ptr, per_row, rows, (int)(cols / 8), lim, (const unsigned int*)amax->ptr);
+               (uint2*)out->ptr, (float*)scale->ptr, per_row, rows, (int)(cols / 8), lim, sorted_ids, M,
+               (const unsigned int*)amax->ptr);
 }
 
 void launch_quant_per_token(aiter_tensor_t* out, const aiter_tensor_t* input, aiter_tensor_t* scales,
-                            const aiter_tensor_t* row_limit, int rows_factor, bool after_wait, cudaStream_t stream) {
+                            const aiter_tensor_t* row_limit, int rows_factor, bool after_wait, const int* sorted_ids, int M,
+                            cudaStream_t stream) {
     const bool f16 = input_is_f16(input);
     check_tensor(input, "input", -1, 2);
     check_tensor(out, "out", AITER_DTYPE_fp8, 2);
@@ -242,7 +275,7 @@ void launch_quant_per_token(aiter_tensor_t* out, const aiter_tensor_t* input, ai
     // pieces a thread keeps: the whole row for rows up to 4096 / 16384 elements, 8 of them for longer ones
     auto go = [&](auto kernel) {
         launch_pdl(kernel, grid, kRowThreads, 0, stream, (const uint4*)input->ptr, (uint2*)out->ptr, (float*)scales->ptr, rows, cols8,
-                   lim, rows_factor, after_wait);
+                   lim, rows_factor, sorted_ids, M, after_wait);
     };
     if (cols8 <= 2 * kRowThreads) f16 ? go(quant_per_token_kernel<true, 2>) : go(quant_per_token_kernel<false, 2>);
     else f16 ? go(quant_per_token_kernel<true, 8>) : go(quant_per_token_kernel<false, 8>);

@@ -32,7 +32,8 @@ __device__ __forceinline__ void unpack8(const uint4& raw, float (&v)[8]) {
 }
 
 // Correctly rounded a / b given rb = RN(1/b): two FMA residual corrections (the first makes the quotient faithful, the
-// second then rounds it correctly), valid while nothing over- or underflows.
+// second then rounds it correctly), valid while nothing over- or underflows (P. Markstein, "Computation of elementary functions
+// on the IBM RISC System/6000 processor", 1990, theorem on quotient rounding).
 __device__ __forceinline__ float div_rn_by(float a, float b, float rb) {
     float q = a * rb;
     q = fmaf(fmaf(-q, b, a), rb, q);
