@@ -25,10 +25,10 @@ void launch_quant_1x128(aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*,
 void launch_quant_per_token(aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*, const aiter_tensor_t*, int, bool,
                             const int*, int, cudaStream_t);
 void launch_quant_per_tensor(aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*, aiter_tensor_t*, aiter_tensor_t*,
-                             const aiter_tensor_t*, bool, const int*, int, cudaStream_t);
+                             const aiter_tensor_t*, bool, bool, const int*, int, cudaStream_t);
 void launch_moe_stage1(const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*,
                        const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*,
-                       aiter_tensor_t*, aiter_tensor_t*, int, const aiter_tensor_t*, int, bool, cudaStream_t);
+                       aiter_tensor_t*, aiter_tensor_t*, int, const aiter_tensor_t*, int, bool, unsigned*, cudaStream_t);
 void launch_moe_stage2(const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*,
                        const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*,
                        aiter_tensor_t*, aiter_tensor_t*, int, int, int, int, int, cudaStream_t);
@@ -186,7 +186,7 @@ B200_EXPORT int b200_moe_stage1(const aiter_tensor_t* a1, const aiter_tensor_t* 
         B200_CHECK(a1 != nullptr, "a1 must not be NULL");
         DeviceGuard g(a1->device_id);
         launch_moe_stage1(a1, a1_scale, w1, w1_scale, sorted_token_ids, sorted_expert_ids, num_valid_ids, a2,
-                          a2_scale, status, quant_type, sorted_weights, activation, false, (cudaStream_t)stream);
+                          a2_scale, status, quant_type, sorted_weights, activation, false, nullptr, (cudaStream_t)stream);
     });
 }
 
@@ -260,7 +260,7 @@ B200_EXPORT int b200_moe_quant_per_tensor(aiter_tensor_t* out, const aiter_tenso
     return safe_call([&] {
         B200_CHECK(input != nullptr, "input must not be NULL");
         DeviceGuard g(input->device_id);
-        launch_quant_per_tensor(out, input, scale, amax, row_scales, row_limit, false, nullptr, 0, (cudaStream_t)stream);
+        launch_quant_per_tensor(out, input, scale, amax, row_scales, row_limit, false, false, nullptr, 0, (cudaStream_t)stream);
     });
 }
 

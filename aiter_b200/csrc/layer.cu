@@ -15,10 +15,10 @@ void launch_quant_1x128(aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*,
 void launch_quant_per_token(aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*, const aiter_tensor_t*, int, bool,
                             const int*, int, cudaStream_t);
 void launch_quant_per_tensor(aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*, aiter_tensor_t*, aiter_tensor_t*,
-                             const aiter_tensor_t*, bool, const int*, int, cudaStream_t);
+                             const aiter_tensor_t*, bool, bool, const int*, int, cudaStream_t);
 void launch_moe_stage1(const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*,
                        const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*,
-                       aiter_tensor_t*, aiter_tensor_t*, int, const aiter_tensor_t*, int, bool, cudaStream_t);
+                       aiter_tensor_t*, aiter_tensor_t*, int, const aiter_tensor_t*, int, bool, unsigned*, cudaStream_t);
 void launch_moe_stage2(const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*,
                        const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*,
                        aiter_tensor_t*, aiter_tensor_t*, int, int, int, int, int, cudaStream_t);
@@ -113,7 +113,7 @@ void launch_fused_moe(const b200_fused_moe_args& a, cudaStream_t stream) {
         a1_s = tensor(a.a1_scale, F32, dev, a.a1_scale_numel);
     } else {
         a1 = tensor(ws + at.a1, FP8, dev, M, H);
-        if (per_tensor) launch_quant_per_tensor(&a1, &hidden, &one, &amax, nullptr, nullptr, true, nullptr, 0, stream), a1_s = one;
+        if (per_tensor) launch_quant_per_tensor(&a1, &hidden, &one, &amax, nullptr, nullptr, true, false, nullptr, 0, stream), a1_s = one;
         else if (rowwise) launch_quant_per_token(&a1, &hidden, &a1_s, nullptr, 1, false, nullptr, 0, stream);
         else launch_quant_1x128(&a1, &hidden, &a1_s, nullptr, 1, 0, false, stream);
     }
@@ -126,11 +126,12 @@ void launch_fused_moe(const b200_fused_moe_args& a, cudaStream_t stream) {
     const aiter_tensor_t* w_stage1 = a.doweight_stage1 ? &s_w : nullptr;
     if (rowwise) {
         aiter_tensor_t half = tensor(ws + at.a2_half, AITER_DTYPE_bf16, dev, at.P, I);
-        launch_moe_stage1(&a1, &a1_s, &w1, &w1_s, &s_ids, &s_e, &nv, &half, nullptr, &status, gemm_qt, w_stage1, (int)a.activation, true, stream);
-        if (per_tensor) launch_quant_per_tensor(&a2, &half, &one2, &amax2, nullptr, &nv, true, (const int*)s_ids.ptr, (int)M, stream), a2_s = one2;
+        launch_moe_stage1(&a1, &a1_s, &w1, &w1_s, &s_ids, &s_e, &nv, &half, nullptr, &status, gemm_qt, w_stage1, (int)a.activation, true,
+                          per_tensor ? (unsigned*)amax2.ptr : nullptr, stream);
+        if (per_tensor) launch_quant_per_tensor(&a2, &half, &one2, &amax2, nullptr, &nv, true, true, (const int*)s_ids.ptr, (int)M, stream), a2_s = one2;
         else launch_quant_per_token(&a2, &half, &a2_s, &nv, 1, true, (const int*)s_ids.ptr, (int)M, stream);
     } else {
-        launch_moe_stage1(&a1, &a1_s, &w1, &w1_s, &s_ids, &s_e, &nv, &a2, &a2_s, &status, gemm_qt, w_stage1, (int)a.activation, true, stream);
+        launch_moe_stage1(&a1, &a1_s, &w1, &w1_s, &s_ids, &s_e, &nv, &a2, &a2_s, &status, gemm_qt, w_stage1, (int)a.activation, true, nullptr, stream);
     }
     launch_moe_stage2(&a2, &a2_s, &w2, &w2_s, &s_ids, &s_w, &s_e, &nv, &acc, &status, 0, 0, 0, gemm_qt, a.doweight_stage1 ? 0 : 1, stream);
     aiter_tensor_t out = tensor(a.out, (int)a.out_dtype, dev, M, H);

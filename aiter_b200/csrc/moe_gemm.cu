@@ -105,6 +105,7 @@ struct GemmParams {
     float* a2_scale;         // stage 1 out [P, I/128]
     float* acc;              // stage 2 out [M, H] fp32
     int* status;
+    unsigned* amax;          // PT stage 1: maximum magnitude written, as fp32 bits (cleared before the launch), or null
     int skip_pads;           // stage 1: rows of padding are not written (stage 2 does not read them)
     int use_weight;          // multiply this stage's GEMM result by the route weight (sorted_w)
     long long wait_limit;    // SM clocks after which a device-side wait gives up (sets status, the CTA winds down)
@@ -519,6 +520,16 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
                         w[j0 + i] = *reinterpret_cast<uint32_t*>(&hb);
                     }
                 }
+                if (p.amax) {
+                    // per_Tensor requantisation: the maximum is taken here, where the values are in registers, instead of
+                    // by a kernel that reads them all again (fmaxf and __hmax2 both skip NaN)
+                    __nv_bfloat162 m2 = __floats2bfloat162_rn(0.f, 0.f);
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) m2 = __hmax2(m2, __habs2(*reinterpret_cast<__nv_bfloat162*>(&w[j])));
+                    const float m = valid ? fmaxf(__low2float(m2), __high2float(m2)) : 0.f;
+                    const unsigned top = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+                    if (lane == 0 && top != 0u) atomicMax(p.amax, top);
+                }
                 uint4* dst = reinterpret_cast<uint4*>(p.a2 + ((size_t)prow * p.inter + nt * 128 + half * 64) * 2);
                 if (valid || !p.skip_pads) {
 #pragma unroll
@@ -724,7 +735,8 @@ void launch_moe_stage1(const aiter_tensor_t* a1, const aiter_tensor_t* a1_scale,
                        const aiter_tensor_t* w1_scale, const aiter_tensor_t* sorted_ids,
                        const aiter_tensor_t* sorted_eids, const aiter_tensor_t* num_valid, aiter_tensor_t* a2,
                        aiter_tensor_t* a2_scale, aiter_tensor_t* status, int quant_type,
-                       const aiter_tensor_t* sorted_w, int activation, bool skip_pads, cudaStream_t stream) {
+                       const aiter_tensor_t* sorted_w, int activation, bool skip_pads, unsigned* amax,
+                       cudaStream_t stream) {
     B200_CHECK(activation == 0 || activation == 1, "activation must be Silu (0) or Gelu (1), got ", activation);
     if (sorted_w) {
         check_tensor(sorted_w, "sorted_weights", AITER_DTYPE_fp32, 1);
@@ -792,6 +804,7 @@ void launch_moe_stage1(const aiter_tensor_t* a1, const aiter_tensor_t* a1_scale,
     p.status = (int*)status->ptr;
     p.sorted_w = sorted_w ? (const float*)sorted_w->ptr : nullptr;
     p.skip_pads = skip_pads;
+    p.amax = amax;
     p.use_weight = sorted_w != nullptr;   // doweight_stage1 (aiter/fused_moe.py:3651-3652)
     CUtensorMap tmap = make_map(w1->ptr, (uint64_t)(E * N2), (uint64_t)H, 128);
     const int64_t max_tiles = ((int64_t)sorted_ids->numel_ / BM) * p.n_tiles;

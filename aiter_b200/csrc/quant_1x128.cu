@@ -134,27 +134,12 @@ __global__ void __launch_bounds__(kRowThreads) quant_per_token_kernel(const uint
 // the maximum over the rows below *row_limit goes to amax[0] (non-negative floats order like their bit patterns,
 // so an integer atomicMax does it), then every row is converted with the one scale, which is also written to
 // scale[0] and, if asked, once per row to row_scales (the GEMM kernels take one activation scale per row).
-// With sorted_ids a CTA takes whole rows, so that padding rows can be left out; else the buffer is one flat range.
 template <bool F16>
 __global__ void __launch_bounds__(256) amax_kernel(const uint4* x, int64_t rows, int cols8, const int* row_limit,
-                                                   const int* sorted_ids, int M, unsigned int* amax) {
+                                                   unsigned int* amax) {
     pdl_wait();
     pdl_trigger();
     const int64_t limit = row_limit ? min((int64_t)*row_limit, rows) : rows;
-    if (sorted_ids) {
-        float m = 0.f, v[8];
-        for (int64_t row = blockIdx.x; row < limit; row += gridDim.x) {
-            if (is_padding(sorted_ids, row_limit, M, row)) continue;
-            for (int i = threadIdx.x; i < cols8; i += 256) {
-                unpack8<F16>(x[row * cols8 + i], v);
-                m = amax8(v, m);
-            }
-        }
-#pragma unroll
-        for (int d = 16; d >= 1; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
-        if ((threadIdx.x & 31) == 0 && m > 0.f) atomicMax(amax, __float_as_uint(m));
-        return;
-    }
     const int64_t n = limit * cols8, step = (int64_t)gridDim.x * blockDim.x;
     float m = 0.f, v[8];
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += 4 * step) {
@@ -184,7 +169,7 @@ __global__ void __launch_bounds__(256) quant_per_tensor_kernel(const uint4* x, u
     const int64_t limit = row_limit ? min((int64_t)*row_limit, rows) : rows;
     const float scale = __fdiv_rn(__uint_as_float(*amax), 448.0f);
     if (blockIdx.x == 0 && threadIdx.x == 0) scale_out[0] = scale;
-    if (sorted_ids) {
+    if (sorted_ids) {   // a CTA takes whole rows, so that padding rows can be left out
         float v[8];
         for (int64_t row = blockIdx.x; row < limit; row += gridDim.x) {
             if (is_padding(sorted_ids, row_limit, M, row)) continue;
@@ -225,7 +210,8 @@ static bool input_is_f16(const aiter_tensor_t* input) {
 }
 
 void launch_quant_per_tensor(aiter_tensor_t* out, const aiter_tensor_t* input, aiter_tensor_t* scale, aiter_tensor_t* amax,
-                             aiter_tensor_t* row_scales, const aiter_tensor_t* row_limit, bool amax_cleared, const int* sorted_ids, int M, cudaStream_t stream) {
+                             aiter_tensor_t* row_scales, const aiter_tensor_t* row_limit, bool amax_cleared, bool amax_done, const int* sorted_ids,
+                             int M, cudaStream_t stream) {
     const bool f16 = input_is_f16(input);
     check_tensor(input, "input", -1, 2);
     check_tensor(out, "out", AITER_DTYPE_fp8, 2);
@@ -247,8 +233,9 @@ void launch_quant_per_tensor(aiter_tensor_t* out, const aiter_tensor_t* input, a
     const int grid = (int)std::min<int64_t>((n + 255) / 256, (int64_t)sm_count(input->device_id) * 8);
     const int* lim = row_limit ? (const int*)row_limit->ptr : nullptr;
     float* per_row = row_scales ? (float*)row_scales->ptr : nullptr;
-    launch_pdl(f16 ? amax_kernel<true> : amax_kernel<false>, grid, 256, 0, stream, (const uint4*)input->ptr, rows, (int)(cols / 8),
-               lim, sorted_ids, M, (unsigned int*)amax->ptr);
+    if (!amax_done)
+        launch_pdl(f16 ? amax_kernel<true> : amax_kernel<false>, grid, 256, 0, stream, (const uint4*)input->ptr, rows, (int)(cols / 8),
+               lim, (unsigned int*)amax->ptr);
     launch_pdl(f16 ? quant_per_tensor_kernel<true> : quant_per_tensor_kernel<false>, grid, 256, 0, stream, (const uint4*)input->ptr,
                (uint2*)out->ptr, (float*)scale->ptr, per_row, rows, (int)(cols / 8), lim, sorted_ids, M,
                (const unsigned int*)amax->ptr);
