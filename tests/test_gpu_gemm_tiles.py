@@ -1,5 +1,5 @@
 """The GEMM kernels at the edges of their tiles: output widths that leave half an output tile, blocks with
-dead 32-row quarters, tiles shared between CTAs along K, every scale type, against the oracle."""
+dead 32-row quarters, few tiles with long K, every scale type, against the oracle."""
 import pytest
 import torch
 
@@ -31,7 +31,7 @@ def _deq(q, s, quant):
 @pytest.mark.parametrize("quant", ["block", "token", "tensor"])
 @pytest.mark.parametrize("H,I,E,rows", [(128, 128, 1, [3]), (256, 128, 3, [1, 31, 33]), (384, 256, 4, [97, 0, 128, 129]),
                                         (640, 384, 5, [64, 65, 0, 260, 1]), (1408, 128, 2, [32, 96]),
-                                        # tiles shared between CTAs: 39 of 56 K steps in stage 1, 160 of 16; 12 of 20 in stage 2
+                                        # long K with fewer tiles than SMs; a second, partly filled round of tiles; few tiles in stage 2
                                         (7168, 384, 13, [1, 40, 130, 2, 3, 64, 7, 5, 1, 9, 33, 1, 2]),
                                         (2048, 1024, 20, [1 + 7 * i for i in range(20)]), (512, 2560, 6, [1, 128, 5, 70, 2, 33])])
 def test_layer_at_tile_edges(quant, H, I, E, rows):
