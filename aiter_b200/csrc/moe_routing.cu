@@ -107,7 +107,11 @@ __device__ __forceinline__ float select_topk(uint32_t (&key)[VPL], const float (
     return wsum;
 }
 
-// Two largest of a run of values and of a second such pair
+// A score as it counts for its group: NaN counts for nothing (fmaxf returns the operand that is a number). The two largest of
+// a run are merged by fminf / fmaxf, which would otherwise take the partner of a NaN twice.
+__device__ __forceinline__ float in_group(float v) { return fmaxf(v, kNegInf); }
+
+// Two largest of a run of values and of a second such pair (no NaN among them)
 __device__ __forceinline__ void merge_top2(float& b1, float& b2, float o1, float o2) {
     b2 = fmaxf(fminf(b1, o1), fmaxf(b2, o2));
     b1 = fmaxf(b1, o1);
@@ -138,12 +142,12 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) biased_grouped_topk_kerne
     const int span = gsize / VPL;   // lanes per group
     if (gsize % VPL == 0 && (span & (span - 1)) == 0) {
         // a group is a power-of-two run of lanes: all groups at once in log2(span) butterfly rounds
-        float b1 = choice[0], b2 = kNegInf;
+        float b1 = in_group(choice[0]), b2 = kNegInf;
 #pragma unroll
-        for (int j = 1; j < VPL; ++j) merge_top2(b1, b2, choice[j], kNegInf);
+        for (int j = 1; j < VPL; ++j) merge_top2(b1, b2, in_group(choice[j]), kNegInf);
         for (int d = 1; d < span; d <<= 1)
             merge_top2(b1, b2, __shfl_xor_sync(0xffffffffu, b1, d), __shfl_xor_sync(0xffffffffu, b2, d));
-        const float gs = (gsize >= 2) ? b1 + b2 : b1;
+        const float gs = in_group((gsize >= 2) ? b1 + b2 : b1);   // inf - inf of two biases
         const int mine = lane / span;
         int better = 0;
         for (int g = 0; g < n_group; ++g) {
@@ -158,11 +162,11 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) biased_grouped_topk_kerne
             float b1 = kNegInf, b2 = kNegInf;
 #pragma unroll
             for (int j = 0; j < VPL; ++j)
-                if (e0 + j >= g * gsize && e0 + j < (g + 1) * gsize) merge_top2(b1, b2, choice[j], kNegInf);
+                if (e0 + j >= g * gsize && e0 + j < (g + 1) * gsize) merge_top2(b1, b2, in_group(choice[j]), kNegInf);
 #pragma unroll
             for (int d = 1; d < 32; d <<= 1)
                 merge_top2(b1, b2, __shfl_xor_sync(0xffffffffu, b1, d), __shfl_xor_sync(0xffffffffu, b2, d));
-            if (lane == g) gs_mine = (gsize >= 2) ? b1 + b2 : b1;
+            if (lane == g) gs_mine = in_group((gsize >= 2) ? b1 + b2 : b1);
         }
         int better = 0;
         for (int g = 0; g < n_group; ++g) {

@@ -100,3 +100,20 @@ def test_routing_errors():
         aiter_b200.biased_grouped_topk(x, torch.zeros(48, device=DEV), w, ids, 5, 2, True)
     with pytest.raises(RuntimeError, match="fp32 or bf16"):
         aiter_b200.topk_softmax(w, ids, None, x.to(torch.float16), True)
+
+
+def test_nan_does_not_raise_a_groups_score():
+    """A NaN score counts for nothing in its group's score (the sum of the two largest others) and is never chosen."""
+    logits = torch.full((3, 256), -9.0)
+    logits[:, 32:160:32] = 0.5            # groups 1..4: two experts at sigmoid(0.5), group score 1.245
+    logits[:, 33:160:32] = 0.5
+    logits[:, 1] = 5.0                    # group 0: one expert at 0.993; counted twice it would beat the others
+    logits[1, 200], logits[2, 8] = float("nan"), float("nan")
+    logits[0, 0], logits[1, 0], logits[2, 2] = float("nan"), float("nan"), float("nan")
+    bias = torch.zeros(256)
+    w_ref, ids_ref = moe_oracle.biased_grouped_topk_ref(logits.nan_to_num(nan=-1e4), bias, 8, True, 8, 4, 2.5)
+    assert not (ids_ref < 32).any()
+    w = torch.empty((3, 8), dtype=torch.float32, device=DEV)
+    ids = torch.empty((3, 8), dtype=torch.int32, device=DEV)
+    aiter_b200.biased_grouped_topk(logits.to(DEV), bias.to(DEV), w, ids, 8, 4, True, 2.5)
+    compare(w, ids, w_ref, ids_ref, "NaN beside scores")
