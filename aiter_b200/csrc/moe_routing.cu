@@ -73,8 +73,9 @@ __device__ __forceinline__ uint32_t order_key(float v) {
 }
 
 // Picks the k largest of key[] (value, then lower index) one at a time; entry j of a lane is expert index(j), ascending in
-// j; key 0 = not there or already taken. Lane i < k keeps pick i in (my_id, my_w), with the weight wsrc[] of the winning
-// expert. Returns the sum of the k weights, added in the order of the picks.
+// j; key 0 = not there, NaN or already taken. Lane i < k keeps pick i in (my_id, my_w), with the weight wsrc[] of the winning
+// expert. Where nothing is left to pick the id is INT_MAX, which the sort drops, and the weight 0. Returns the sum of the k
+// weights, added in the order of the picks.
 template <int VPL, typename Index>
 __device__ __forceinline__ float select_topk(uint32_t (&key)[VPL], const float (&wsrc)[VPL], int k, int lane, Index index,
                                              int& my_id, float& my_w) {
@@ -83,7 +84,7 @@ __device__ __forceinline__ float select_topk(uint32_t (&key)[VPL], const float (
         uint32_t best = key[0];
 #pragma unroll
         for (int j = 1; j < VPL; ++j) best = max(best, key[j]);
-        best = __reduce_max_sync(0xffffffffu, best);
+        best = max(__reduce_max_sync(0xffffffffu, best), 1u);   // no score has key 1: at 0 nothing matches
         int mine = 0x7fffffff;
         float w = 0.f;
 #pragma unroll

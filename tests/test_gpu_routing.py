@@ -117,3 +117,27 @@ def test_nan_does_not_raise_a_groups_score():
     ids = torch.empty((3, 8), dtype=torch.int32, device=DEV)
     aiter_b200.biased_grouped_topk(logits.to(DEV), bias.to(DEV), w, ids, 8, 4, True, 2.5)
     compare(w, ids, w_ref, ids_ref, "NaN beside scores")
+
+
+@pytest.mark.parametrize("E", [30, 128, 256])
+def test_token_without_a_score_gets_no_expert(E):
+    """Where every score is NaN there is nothing to choose: the ids are outside [0, E), which the sort drops, and the other
+    tokens of the batch are routed as ever."""
+    logits = torch.randn((5, E), generator=torch.Generator().manual_seed(E))
+    clean = logits.clone()
+    logits[3] = float("nan")
+    for grouped in (False, True):
+        got = []
+        for x in (clean, logits):
+            w = torch.empty((5, 4), dtype=torch.float32, device=DEV)
+            ids = torch.empty((5, 4), dtype=torch.int32, device=DEV)
+            if grouped:
+                # both groups kept: the experts of a dropped group would compete with the value 0
+                aiter_b200.biased_grouped_topk(x.to(DEV), torch.zeros(E, device=DEV), w, ids, 2, 2, True, 1.0)
+            else:
+                aiter_b200.topk_softmax(w, ids, None, x.to(DEV), True)
+            got.append((w.cpu(), ids.cpu()))
+        (w0, i0), (w1, i1) = got
+        keep = torch.tensor([0, 1, 2, 4])
+        assert torch.equal(i0[keep], i1[keep]) and torch.equal(w0[keep], w1[keep])
+        assert bool(((i1[3] < 0) | (i1[3] >= E)).all()), i1[3]
