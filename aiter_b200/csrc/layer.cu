@@ -18,10 +18,10 @@ void launch_quant_per_tensor(aiter_tensor_t*, const aiter_tensor_t*, aiter_tenso
                              const aiter_tensor_t*, bool, bool, const int*, int, cudaStream_t);
 void launch_moe_stage1(const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*,
                        const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*,
-                       aiter_tensor_t*, aiter_tensor_t*, int, const aiter_tensor_t*, int, bool, unsigned*, cudaStream_t);
+                       aiter_tensor_t*, aiter_tensor_t*, int, const aiter_tensor_t*, int, bool, unsigned*, bool, cudaStream_t);
 void launch_moe_stage2(const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*,
                        const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*,
-                       aiter_tensor_t*, aiter_tensor_t*, int, int, int, int, int, cudaStream_t);
+                       aiter_tensor_t*, aiter_tensor_t*, int, int, int, int, int, bool, cudaStream_t);
 void launch_finalize(aiter_tensor_t*, const aiter_tensor_t*, cudaStream_t);
 
 namespace {
@@ -127,13 +127,13 @@ void launch_fused_moe(const b200_fused_moe_args& a, cudaStream_t stream) {
     if (rowwise) {
         aiter_tensor_t half = tensor(ws + at.a2_half, AITER_DTYPE_bf16, dev, at.P, I);
         launch_moe_stage1(&a1, &a1_s, &w1, &w1_s, &s_ids, &s_e, &nv, &half, nullptr, &status, gemm_qt, w_stage1, (int)a.activation, true,
-                          per_tensor ? (unsigned*)amax2.ptr : nullptr, stream);
+                          per_tensor ? (unsigned*)amax2.ptr : nullptr, per_tensor, stream);
         if (per_tensor) launch_quant_per_tensor(&a2, &half, &one2, &amax2, nullptr, &nv, true, true, (const int*)s_ids.ptr, (int)M, stream), a2_s = one2;
         else launch_quant_per_token(&a2, &half, &a2_s, &nv, 1, true, (const int*)s_ids.ptr, (int)M, stream);
     } else {
-        launch_moe_stage1(&a1, &a1_s, &w1, &w1_s, &s_ids, &s_e, &nv, &a2, &a2_s, &status, gemm_qt, w_stage1, (int)a.activation, true, nullptr, stream);
+        launch_moe_stage1(&a1, &a1_s, &w1, &w1_s, &s_ids, &s_e, &nv, &a2, &a2_s, &status, gemm_qt, w_stage1, (int)a.activation, true, nullptr, false, stream);
     }
-    launch_moe_stage2(&a2, &a2_s, &w2, &w2_s, &s_ids, &s_w, &s_e, &nv, &acc, &status, 0, 0, 0, gemm_qt, a.doweight_stage1 ? 0 : 1, stream);
+    launch_moe_stage2(&a2, &a2_s, &w2, &w2_s, &s_ids, &s_w, &s_e, &nv, &acc, &status, 0, 0, 0, gemm_qt, a.doweight_stage1 ? 0 : 1, per_tensor, stream);
     aiter_tensor_t out = tensor(a.out, (int)a.out_dtype, dev, M, H);
     launch_finalize(&out, &acc, stream);
 }

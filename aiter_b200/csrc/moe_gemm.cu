@@ -736,7 +736,7 @@ void launch_moe_stage1(const aiter_tensor_t* a1, const aiter_tensor_t* a1_scale,
                        const aiter_tensor_t* w1_scale, const aiter_tensor_t* sorted_ids,
                        const aiter_tensor_t* sorted_eids, const aiter_tensor_t* num_valid, aiter_tensor_t* a2,
                        aiter_tensor_t* a2_scale, aiter_tensor_t* status, int quant_type,
-                       const aiter_tensor_t* sorted_w, int activation, bool skip_pads, unsigned* amax,
+                       const aiter_tensor_t* sorted_w, int activation, bool skip_pads, unsigned* amax, bool per_tensor,
                        cudaStream_t stream) {
     B200_CHECK(activation == 0 || activation == 1, "activation must be Silu (0) or Gelu (1), got ", activation);
     if (sorted_w) {
@@ -764,9 +764,11 @@ void launch_moe_stage1(const aiter_tensor_t* a1, const aiter_tensor_t* a1_scale,
     B200_CHECK(H % 128 == 0, "model_dim must be a multiple of 128, got ", H);
     const int64_t I = N2 / 2;
     if (pt) {
-        B200_CHECK((int64_t)a1_scale->numel_ == M || a1_scale->numel_ == 1, "a1_scale must have one element per token for per_Token");
-        B200_CHECK((int64_t)w1_scale->numel_ == E * N2 || (int64_t)w1_scale->numel_ == E,
-                   "w1_scale must have E*2*inter_dim elements for per_Token (or one per expert)");
+        // one scale for all rows / one per expert is the layout of per_Tensor only: the count alone does not select it
+        B200_CHECK((int64_t)a1_scale->numel_ == M || (per_tensor && a1_scale->numel_ == 1),
+                   "a1_scale must have one element per token for per_Token (one for per_Tensor)");
+        B200_CHECK((int64_t)w1_scale->numel_ == E * N2 || (per_tensor && (int64_t)w1_scale->numel_ == E),
+                   "w1_scale must have E*2*inter_dim elements for per_Token (E for per_Tensor)");
     } else {
         B200_CHECK((int64_t)a1_scale->numel_ == M * (H / 128), "a1_scale must have M*model_dim/128 elements");
         B200_CHECK((int64_t)w1_scale->numel_ == E * (N2 / 128) * (H / 128),
@@ -819,7 +821,8 @@ void launch_moe_stage2(const aiter_tensor_t* a2, const aiter_tensor_t* a2_scale,
                        const aiter_tensor_t* w2_scale, const aiter_tensor_t* sorted_ids,
                        const aiter_tensor_t* sorted_w, const aiter_tensor_t* sorted_eids,
                        const aiter_tensor_t* num_valid, aiter_tensor_t* acc, aiter_tensor_t* status,
-                       int col_begin, int col_end, int sm_margin, int quant_type, int doweight, cudaStream_t stream) {
+                       int col_begin, int col_end, int sm_margin, int quant_type, int doweight, bool per_tensor,
+                       cudaStream_t stream) {
     B200_CHECK(quant_type == 4 || quant_type == 5 || quant_type == 2,
                "quant_type must be per_1x128 (4), per_128x128 (5) or per_Token (2), got ", quant_type);
     const bool pt = quant_type == 2;
@@ -849,9 +852,10 @@ void launch_moe_stage2(const aiter_tensor_t* a2, const aiter_tensor_t* a2_scale,
     B200_CHECK(sm_margin >= 0, "sm_margin must not be negative");
     B200_CHECK(I % 128 == 0 && H % 128 == 0, "inter_dim and model_dim must be multiples of 128");
     if (pt) {
-        B200_CHECK((int64_t)a2_scale->numel_ >= P || a2_scale->numel_ == 1, "a2_scale must have one element per sorted row for per_Token");
-        B200_CHECK((int64_t)w2_scale->numel_ == E * H || (int64_t)w2_scale->numel_ == E,
-                   "w2_scale must have E*model_dim elements for per_Token (or one per expert)");
+        B200_CHECK((int64_t)a2_scale->numel_ >= P || (per_tensor && a2_scale->numel_ == 1),
+                   "a2_scale must have one element per sorted row for per_Token (one for per_Tensor)");
+        B200_CHECK((int64_t)w2_scale->numel_ == E * H || (per_tensor && (int64_t)w2_scale->numel_ == E),
+                   "w2_scale must have E*model_dim elements for per_Token (E for per_Tensor)");
         B200_CHECK(((uintptr_t)w2_scale->ptr & 15) == 0 || (int64_t)w2_scale->numel_ == E, "w2_scale must be 16-byte aligned");
     } else {
         B200_CHECK((int64_t)a2_scale->numel_ >= P * (I / 128), "a2_scale must have P*inter_dim/128 elements");

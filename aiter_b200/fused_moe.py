@@ -319,6 +319,11 @@ def fused_moe_stages(hidden_states, w1, w2, topk_weight, topk_ids, expert_mask, 
     w_stage1 = sorted_weights if doweight_stage1 else None   # aiter/fused_moe.py:3651-3652
     dw2 = 0 if doweight_stage1 else 1
     qt = int(QuantType.per_Token if per_token else QuantType.per_1x128)
+    if per_tensor:
+        w1_scale = w1_scale.reshape(E, -1).expand(E, 2 * inter_dim).contiguous()
+        w2_scale = w2_scale.reshape(E, -1).expand(E, model_dim).contiguous()
+        if a1_scale is not None:
+            a1_scale = a1_scale.reshape(-1).expand(M)
     if hidden_states.dtype == dtypes.fp8:
         a1, a1_s = hidden_states.contiguous(), a1_scale.contiguous()
     elif per_tensor:

@@ -142,8 +142,8 @@ typedef struct b200_fused_moe_args {
     const void* a1_scale;          /* fp32, with fp8 hidden: [M,H/128], [M] (per_Token) or [1] (per_Tensor) */
     const void* w1;                /* [E,2I,H] fp8 */
     const void* w2;                /* [E,H,I] fp8 */
-    const void* w1_scale;          /* fp32, w1_scale_numel elements */
-    const void* w2_scale;          /* fp32, w2_scale_numel elements */
+    const void* w1_scale;          /* fp32: [E,2I/128,H/128], [E,2I] (per_Token) or [E] (per_Tensor) */
+    const void* w2_scale;          /* fp32: [E,H/128,I/128], [E,H] (per_Token) or [E] (per_Tensor) */
     const void* topk_weight;       /* [M,topk] fp32 */
     const void* topk_ids;          /* [M,topk] i32 */
     const void* expert_mask;       /* optional [global_E] i32 */

@@ -431,3 +431,31 @@ def test_registered_operator_matches_function():
                                           c["w1_scale"], c["w2_scale"], None, None, None)
     s = moe_oracle.error_stats(out, ref.cpu())
     assert s["n_diff"] <= 1e-3 * s["numel"] and s["max_abs_over_rms"] <= MAX_ABS_OVER_RMS, s
+
+
+@pytest.mark.parametrize("where", ["layer", "stages"])
+def test_scale_counts_of_another_quantisation_raise(where):
+    """Row / channel scales with the element count of one scale per expert or per tensor are an error, not a broadcast."""
+    c = to_dev(inputs.make_config("cfg0_pt", seed=0))
+    E = c["w1_q"].shape[0]
+    a1, a1s = aiter_b200.get_hip_quant(QT.per_Token)(c["x"], quant_dtype=torch.float8_e4m3fn)
+    good = dict(x=a1, a1_scale=a1s, w1_scale=c["w1_scale"], w2_scale=c["w2_scale"])
+
+    def call(**over):
+        k = {**good, **over}
+        fm.kernel_bench_events = [] if where == "stages" else None
+        try:
+            return aiter_b200.fused_moe(k["x"], c["w1_q"], c["w2_q"], c["topk_weight"], c["topk_ids"], quant_type=QT.per_Token,
+                                        w1_scale=k["w1_scale"], w2_scale=k["w2_scale"], a1_scale=k["a1_scale"])
+        finally:
+            fm.kernel_bench_events = None
+
+    call()
+    one = torch.ones((E, 1), device=DEV)
+    with pytest.raises(RuntimeError, match="w1_scale must have"):
+        call(w1_scale=one)
+    with pytest.raises(RuntimeError, match="w2_scale must have"):
+        call(w2_scale=one)
+    with pytest.raises(RuntimeError, match="a1_scale must have"):
+        call(a1_scale=a1s[:1])
+    aiter_b200.check_device_status()
