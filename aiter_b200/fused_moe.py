@@ -428,6 +428,10 @@ def _layer(hidden_states, w1, w2, topk_weight, topk_ids, expert_mask, w1_scale, 
                           ("w1_scale", w1_scale, dtypes.fp32), ("w2_scale", w2_scale, dtypes.fp32), ("a1_scale", a1_scale, dtypes.fp32)):
         if t is not None and (t.dtype != code or not t.is_cuda or t.numel() < 1):
             raise RuntimeError(f"{name} must be a non-empty {code} CUDA tensor")
+    if expert_mask is not None and (expert_mask.dim() != 1 or not expert_mask.is_contiguous()):
+        raise RuntimeError("local_expert_mask must be contiguous and have one dimension")
+    if num_local_tokens is not None and not num_local_tokens.is_contiguous():
+        raise RuntimeError("num_local_tokens must be contiguous")
     if not (w1.is_cuda and w2.is_cuda and topk_weight.is_cuda and topk_ids.is_cuda):
         raise RuntimeError("fused_moe: tensors must live on a CUDA device (there is no CPU path)")
     if w1.shape != (E, 2 * I, H):
@@ -439,8 +443,6 @@ def _layer(hidden_states, w1, w2, topk_weight, topk_ids, expert_mask, w1_scale, 
         a1_scale = None
     elif a1_scale is not None:
         a1_scale = a1_scale.contiguous()
-    if expert_mask is not None:
-        expert_mask = expert_mask.contiguous()
     global_E = E if expert_mask is None else expert_mask.numel()
     code = dtypes.AITER_DTYPE[hidden_states.dtype]
     nbytes = _layer_workspace_bytes(M, H, I, global_E, topk, int(quant_type), code)

@@ -459,3 +459,16 @@ def test_scale_counts_of_another_quantisation_raise(where):
     with pytest.raises(RuntimeError, match="a1_scale must have"):
         call(a1_scale=a1s[:1])
     aiter_b200.check_device_status()
+
+
+def test_mask_and_token_count_forms_that_raise():
+    """An expert mask is one contiguous row of int32, the token count a contiguous int32 tensor: other forms are refused."""
+    c = to_dev(inputs.make_config("cfg0", seed=0))
+    E = c["w1_q"].shape[0]
+    ones = torch.ones(2 * E, dtype=torch.int32, device=DEV)
+    run(c, expert_mask=ones[:E])
+    for mask in (ones[:E].view(1, E), ones[::2]):
+        with pytest.raises(RuntimeError, match="local_expert_mask"):
+            run(c, expert_mask=mask)
+    with pytest.raises(RuntimeError, match="num_local_tokens"):
+        run(c, num_local_tokens=ones[::2])
