@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(kRowThreads) quant_per_token_kernel(const uint
     const int tid = threadIdx.x;
     if (row_limit) rows = min(rows, (int64_t)*row_limit * rows_factor);
     int par = 0;
-    for (int64_t row = blockIdx.x; row < rows; row += gridDim.x, par ^= 1) {
+    for (int64_t row = blockIdx.x; row < rows; row += gridDim.x) {
         if (is_padding(sorted_ids, row_limit, M, row)) continue;
         const uint4* xr = x + row * cols8;
         uint4 raw[CACHE];
@@ -109,7 +109,9 @@ __global__ void __launch_bounds__(kRowThreads) quant_per_token_kernel(const uint
 #pragma unroll
         for (int d = 16; d >= 1; d >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, d));
         if ((tid & 31) == 0) red[par][tid >> 5] = amax;
-        __syncthreads();   // one per row: the buffers alternate
+        // One barrier per row: the buffers alternate with the rows that pass it, skipped rows not counted, so a buffer is
+        // written again only behind the barrier of the row in between, which every reader of this row has reached by then.
+        __syncthreads();
 #pragma unroll
         for (int k = 0; k < kRowThreads / 32; ++k) amax = fmaxf(amax, red[par][k]);
         float scale = __fdiv_rn(amax, 448.0f);
@@ -125,6 +127,7 @@ __global__ void __launch_bounds__(kRowThreads) quant_per_token_kernel(const uint
             q[row * cols8 + i] = quant_codes8(v, scale);
         }
         if (tid == 0) scales[row] = scale;
+        par ^= 1;
     }
     if (!after_wait) pdl_wait();
 }

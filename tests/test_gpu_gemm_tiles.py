@@ -60,3 +60,9 @@ def test_layer_at_tile_edges(quant, H, I, E, rows):
     # bf16 result (2^-9 relative) plus single e4m3 codes of a2 that round the other way: the bars of the layer tests
     s = moe_oracle.error_stats(out, ref.to(torch.bfloat16))
     assert not s["has_nan"] and s["frac_within"] >= 0.995 and s["max_abs_over_rms"] <= 0.06, s
+
+
+def test_padding_between_live_rows_of_one_cta():
+    """Row scales: the requantiser's CTAs (8 an SM) stride over 7680 sorted rows of which they skip the padding, so a CTA meets
+    live and padding rows in every order."""
+    test_layer_at_tile_edges("token", 128, 640, 60, [(1, 40, 70, 128)[(i * i + i // 7) % 4] for i in range(60)])
