@@ -395,7 +395,7 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
         const int r = q * 32 + lane;                    // row of the tile == TMEM lane
         const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
         uint32_t it = 0;
-        uint32_t tile_par = 0;
+        uint32_t ax_par = 0;   // stage 1: buffer of the next exchange of row maxima
         bool ok = true;
         // row info of the next tile is fetched one tile ahead, so its latency is off the path between
         // two tiles (where the MMA warp can only run two K steps ahead of these warps)
@@ -407,7 +407,7 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
             eid_next = p.sorted_eids[(int)blockIdx.x / p.n_tiles];
             if (p.use_weight) wgt_next = p.sorted_w[prow0];
         }
-        for (int t = blockIdx.x; ok && t < total_tiles; t += gridDim.x, tile_par ^= 1u) {
+        for (int t = blockIdx.x; ok && t < total_tiles; t += gridDim.x) {
             const int blk = t / p.n_tiles, nt = t - blk * p.n_tiles + p.nt0;
             const int prow = blk * BM + r;
             const int tok = tok_next, eid = eid_next;
@@ -558,7 +558,11 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
                         amax = fmaxf(amax, fmaxf(fabsf(h0), fabsf(h1)));
                     }
                 }
-                float* ax = amax_x + tile_par * (2 * BM);
+                // The two buffers alternate with the exchanges, tiles that this pair of warps skips not counted: a buffer is
+                // written again only behind the barrier of the exchange in between, which the other warp reaches after its
+                // read. (With one K block per tile nothing else keeps the two warps within a tile of each other.)
+                float* ax = amax_x + ax_par * (2 * BM);
+                ax_par ^= 1u;
                 ax[half * BM + r] = amax;
                 ptx::named_barrier(1 + q, 64);   // the two warps that hold these 32 rows
                 amax = fmaxf(amax, ax[(half ^ 1) * BM + r]);

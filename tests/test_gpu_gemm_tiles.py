@@ -66,3 +66,8 @@ def test_padding_between_live_rows_of_one_cta():
     """Row scales: the requantiser's CTAs (8 an SM) stride over 7680 sorted rows of which they skip the padding, so a CTA meets
     live and padding rows in every order."""
     test_layer_at_tile_edges("token", 128, 640, 60, [(1, 40, 70, 128)[(i * i + i // 7) % 4] for i in range(60)])
+
+
+def test_dead_quarters_between_live_ones_with_one_k_block():
+    """Block scales, K = 128 in stage 1: a CTA has four tiles, in which a 32-row quarter is live and dead in every order."""
+    test_layer_at_tile_edges("block", 128, 1280, 60, [(1, 40, 70, 128)[(i * i + i // 7) % 4] for i in range(60)])
