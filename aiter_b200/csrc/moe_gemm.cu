@@ -108,6 +108,7 @@ struct GemmParams {
     int* status;
     unsigned* amax;          // PT stage 1: maximum magnitude written, as fp32 bits (cleared before the launch), or null
     int skip_pads;           // stage 1: rows of padding are not written (stage 2 does not read them)
+    int hold_successor;      // stage 2: the next kernel of the stream is not placed before this one is over
     int use_weight;          // multiply this stage's GEMM result by the route weight (sorted_w)
     long long wait_limit;    // SM clocks after which a device-side wait gives up (sets status, the CTA winds down)
     int stall_producer;      // self-test only: the weight producer loads nothing, so every wait downstream runs out
@@ -228,7 +229,9 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
     ptx::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     pdl_wait();      // everything above overlaps the kernels before this one
-    pdl_trigger();
+    // A launch that leaves SMs free for another stream's kernels must not hand them to its own successor: CTAs of the next
+    // column range would sit there until this range is over.
+    if (STAGE == 1 || !p.hold_successor) pdl_trigger();
 
     const int num_valid = p.num_valid[0];
     const int tokens = min(p.num_valid[1], p.M);
@@ -723,6 +726,7 @@ void launch_gemm(const CUtensorMap& tmap, const CUtensorMap& tmap_a, const GemmP
     GemmParams q = p;
     q.wait_limit = g_wait_limit;
     q.stall_producer = g_stall_producer;
+    q.hold_successor = sm_margin > 0;
     // Overlapping the launch with the kernel before it pays while the layer is short. With tens of tiles per SM the few
     // microseconds are nothing, and at the power limit the early CTAs cost more than they give (1-2 % at 65 K routes).
     const bool overlap = max_tiles <= 64 * grid;

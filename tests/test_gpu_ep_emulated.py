@@ -119,3 +119,48 @@ def test_dispatch_push_combine_emulated_ranks(world, routing, E, topk, placement
             touched = (owner_of_expert[rows] == r).any(dim=1)
             arrived = ~torch.isnan(recv[o][r]).any(dim=1)
             assert torch.equal(touched, arrived), f"rows pushed from rank {r} to rank {o} differ from the routing"
+
+
+def test_range_launches_leave_their_margin_free():
+    """Stage-2 launches of column ranges leave ``sm_margin`` SMs to kernels of other streams while they run: the next range,
+    queued behind, must not sit on them. Small kernels of a second stream get through during the first of two launches."""
+    M, H, I, E, topk = 8192, 7168, 2048, 16, 8
+    dev = torch.device(DEV)
+    g = torch.Generator(device=DEV).manual_seed(0)
+    ids = torch.randint(0, E, (M, topk), generator=g, dtype=torch.int32, device=dev)
+    wts = torch.rand((M, topk), generator=g, device=dev)
+    sid, sw, se, nv, acc = aiter_b200.moe_sorting(ids, wts, E, H, torch.float32, 128)
+    P = sid.numel()
+    a2 = torch.zeros((P, I), dtype=torch.uint8, device=dev).view(torch.float8_e4m3fn)
+    w2 = torch.zeros((E, H, I), dtype=torch.uint8, device=dev).view(torch.float8_e4m3fn)
+    a2s, w2s = torch.ones((P, I // 128), device=dev), torch.ones((E, H // 128, I // 128), device=dev)
+    status = torch.zeros(1, dtype=torch.int32, device=dev)
+    side, tick = torch.cuda.Stream(dev), torch.zeros(1, device=dev)
+
+    def launch(c):
+        _lib.call("b200_moe_stage2", a2, a2s, w2, w2s, sid, sw, se, nv, acc, status, c * H // 2, (c + 1) * H // 2, 16,
+                  int(aiter_b200.QuantType.per_1x128), 1, device=dev)
+
+    def run(beside):
+        ev = [torch.cuda.Event(enable_timing=True) for _ in range(3)]
+        torch.cuda.synchronize()
+        ev[0].record()
+        side.wait_event(ev[0])
+        launch(0)
+        launch(1)
+        ev[1].record()
+        if beside:
+            with torch.cuda.stream(side):
+                for _ in range(10):
+                    tick.add_(1.0)
+                ev[2].record(side)
+        torch.cuda.synchronize()
+        return ev[0].elapsed_time(ev[1]), ev[0].elapsed_time(ev[2]) if beside else 0.0
+
+    run(True)
+    total = run(False)[0]
+    beside = sorted(run(True)[1] for _ in range(5))[2]
+    print(f"two launches {total:.3f} ms, the other stream's kernels done after {beside:.3f} ms")
+    # one launch is half of the total; ten small kernels need some tens of microseconds
+    assert total > 1.0 and beside < 0.4 * total
+    assert int(status.item()) == 0
