@@ -40,9 +40,10 @@ __device__ __forceinline__ float div_rn_by(float a, float b, float rb) {
     return fmaf(fmaf(-q, b, a), rb, q);
 }
 
-// Scales for which div_rn_by stands in for the IEEE division: quotients of magnitude up to 448 that matter (above e4m3's
-// smallest step) keep their residuals normal.
-__device__ __forceinline__ bool scale_is_tame(float scale) { return scale > 1e-30f && scale < 1e30f; }
+// Scales for which div_rn_by stands in for the IEEE division. The residual a - q*b is a multiple of ulp(q) * ulp(b); for a
+// quotient of at least 2^-10 (smaller ones are code 0) that is 2^-33 * ulp(b), which fp32 holds exactly, as a subnormal if
+// need be, down to ulp(b) = 2^-116. 1e-24 (ulp 2^-103) leaves three decades; the upper limit keeps 1/b normal.
+__device__ __forceinline__ bool scale_is_tame(float scale) { return scale > 1e-24f && scale < 1e30f; }
 
 // Codes RNE_e4m3(v / scale) of eight values: five FMA-pipe operations per quotient from one reciprocal per scale instead of
 // the ~4x longer division sequence, which bound the quantisers at 2.3 TB/s.

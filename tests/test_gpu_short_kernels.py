@@ -65,3 +65,21 @@ def test_row_and_tensor_quant_edges(rows, cols, limit):
     q, s = aiter_b200.per_tensor_quant_hip(x.to(DEV), quant_dtype=FP8)
     q_ref, s_ref = moe_oracle.quant_per_tensor(x)
     assert torch.equal(q.cpu().view(torch.uint8), q_ref.view(torch.uint8)) and float(s) == float(s_ref)
+
+
+@pytest.mark.parametrize("qt", [QT.per_1x128, QT.per_Token, QT.per_Tensor])
+def test_quant_codes_at_extreme_scales(qt):
+    """Codes are the correctly rounded quotients over the whole range of scales: around both limits between the two ways of
+    dividing, where residuals are subnormal, and with quotients on and beside the middles between two codes."""
+    g = torch.Generator().manual_seed(7)
+    oracle = {QT.per_1x128: moe_oracle.quant_1x128, QT.per_Token: moe_oracle.quant_per_token,
+              QT.per_Tensor: moe_oracle.quant_per_tensor}[qt]
+    m = torch.randint(128, 256, (64, 128), generator=g).float() * 2.0 ** torch.randint(-18, 1, (64, 128), generator=g)
+    x = m * torch.where(torch.rand((64, 128), generator=g) < 0.5, -1.0, 1.0)
+    x[:, 0] = 448.0 * torch.randint(128, 256, (64,), generator=g) / 256     # scales of few bits: quotients hit the middles
+    for top in (2.0 ** -120, 448e-30, 4.48e-27, 448e-24, 2.0 ** -70, 1.0, 2.0 ** 90, 448e30):
+        t = (x.double() * (top / 448.0)).to(torch.bfloat16)
+        q, s = aiter_b200.get_hip_quant(qt)(t.to(DEV), quant_dtype=FP8)
+        q_ref, s_ref = oracle(t)
+        assert torch.equal(s.cpu().view(-1).view(torch.int32), s_ref.reshape(-1).view(torch.int32)), top
+        assert torch.equal(q.cpu().view(torch.uint8), q_ref.view(torch.uint8)), top
