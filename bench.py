@@ -685,12 +685,21 @@ def main():
     sampler = ClockSampler(local_rank)
     if rank == 0:
         sampler.start()
-    if world == 1:
-        fm.kernel_bench_events = []   # per-kernel event marks of the timed steps (warm-up marks are dropped below)
     t_dev = timed(step_dev, args.steps, args.warmup, sync, profile=args.cuda_profiler_range)
-    stage_marks, fm.kernel_bench_events = fm.kernel_bench_events, None
-    t_e2e_total = timed_e2e_pipelined(layer, (hx, htw, hti), hout2, dev, args.steps, min(args.warmup, 3), sync,
+    device_allocs = []   # device allocations of the process at the start and at the end of the end-to-end loop
+
+    def e2e_sync():
+        sync()
+        device_allocs.append(torch.cuda.memory_stats(dev).get("num_device_alloc", 0))
+    t_e2e_total = timed_e2e_pipelined(layer, (hx, htw, hti), hout2, dev, args.steps, min(args.warmup, 3), e2e_sync,
                                       static_out=captured is not None)
+    stage_marks = None
+    if world == 1:
+        # per-kernel device times: a loop of its own, because event marks make the layer launch its stages one by one
+        # instead of in the one native call that the two loops above time
+        fm.kernel_bench_events = []
+        timed(step_dev, args.steps, args.warmup, sync)
+        stage_marks, fm.kernel_bench_events = fm.kernel_bench_events, None
     # the two host copies of a step timed alone (what bounds e2e when they are slower than the layer)
     def copy_ms(pairs, reps=3):
         torch.cuda.synchronize()
@@ -731,6 +740,7 @@ def main():
                 "h2d_bytes_per_step": int(hx.numel() * 2 + htw.numel() * 4 + hti.numel() * 4) * world,
                 "d2h_bytes_per_step": int(hout.numel() * 2) * world,
                 "h2d_ms_alone": round(h2d_ms, 4), "d2h_ms_alone": round(d2h_ms, 4),
+                "device_allocs_in_loop": device_allocs[1] - device_allocs[0],
                 "how": "pinned host -> device copy of x, topk_weight, topk_ids and device -> pinned host copy of the bf16 "
                        "result every step, on two copy streams overlapping the neighbouring steps' compute"},
         "clocks": clocks,
@@ -742,7 +752,7 @@ def main():
         line["cpu_affinity_rank0"] = cpu_affinity
 
     if world == 1:
-        # per-kernel device time averaged over the timed steps themselves (events recorded inside the timed loop)
+        # per-kernel device time averaged over the steps of the marked loop
         per_call = len(stage_marks) // (args.steps + args.warmup)
         kb_acc = {}
         for c in range(args.warmup, args.steps + args.warmup):
@@ -751,6 +761,7 @@ def main():
                 kb_acc.setdefault(n0, []).append(e0.elapsed_time(e1))
         kb = {k: sum(v) / len(v) for k, v in kb_acc.items()}
         line["kernels_ms"] = {k: round(v, 4) for k, v in kb.items()}
+        line["kernels_how"] = "a second loop of the same steps with event marks between the stages, launched one by one"
         s1 = 4.0 * M_PREFILL * TOPK * H * I / (kb["stage1"] * 1e-3) / 1e12
         s2 = 2.0 * M_PREFILL * TOPK * H * I / (kb["stage2"] * 1e-3) / 1e12
         line["roofline"] = {"bound": "tensor", "kernel": "stage-1 GEMM (gate/up + SiLU*up + requant)", "achieved": s1,
