@@ -75,10 +75,14 @@ inline void check_tensor(const aiter_tensor_t* t, const char* name, int dtype, i
 }
 
 // Programmatic dependent launch: the grid may be placed while its predecessor on the stream still runs; the kernel calls
-// pdl_wait() before it touches anything an earlier kernel wrote or reads. Convention of this library: a kernel triggers
-// its successor (pdl_trigger) only after its own pdl_wait() in at least one CTA, so when a kernel starts, everything up to
-// the predecessor of its predecessor is complete; and every kernel calls pdl_wait() somewhere, so a grid's completion
-// implies the completion of all before it. Saves the 1-2 us between two dependent short kernels and hides their start-up.
+// pdl_wait() before it touches anything an earlier kernel wrote or reads. Every kernel calls pdl_wait() somewhere, so a
+// grid's completion implies the completion of all before it. Most trigger their successor (pdl_trigger) after their own
+// wait; then, when the successor starts, everything before the triggering kernel is complete, and only that kernel may still
+// run. What works before its own wait relies on this and names the kernel it may run beside: the fill of the two-kernel sort
+// (its predecessor is always the count kernel, whose sorting CTAs trigger after their wait) and the layer's activation
+// quantiser (its predecessor is always the sort). That quantiser triggers BEFORE its wait, so whatever is launched behind it
+// must wait before it touches anything (stage 1 and the per_Tensor kernels do). A stage-2 launch that leaves SMs idle does not
+// trigger at all: its successor starts when it is over. Saves the 1-2 us between two dependent short kernels and hides their start-up.
 template <typename... Params, typename... Args>
 inline void launch_kernel(bool overlap, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                           Args&&... args) {

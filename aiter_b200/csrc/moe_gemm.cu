@@ -17,7 +17,8 @@
 //               signalled by cp.async.mbarrier.arrive; stage 2: one thread loads them (contiguous) with TMA, 32 rows a box;
 //               32-row quarters that hold padding only are neither loaded nor promoted nor (skip_pads) written - a decode
 //               block has a few live rows of 128 (Mixtral-shaped layer at 32 tokens: 298 -> 276 us);
-//   warp 3      (stage 2: 5) prefetches the weight scales of the CTA's tiles into L2;
+//   warp 3      (stage 2: 5) prefetches the weight scales of the CTA's tiles into L2 (a DRAM round trip less at the start of a
+//               tile; by itself within the noise, +-0.5 %, from M=1 to 8192);
 //   warp 1      issues 4 tcgen05.mma (M128 N256 K32, e4m3 -> fp32) into one of two 256-column
 //               TMEM stages, then commits to free the smem stage and to publish the TMEM stage;
 //   warps 8-15  read the TMEM stage (tcgen05.ld) and fold it into fp32 registers with the block
@@ -68,7 +69,8 @@ constexpr int kEpilogueSleepNs = B200_EPI_SLEEP_NS;   // back-off of the promoti
 constexpr uint32_t kIdesc = ptx::make_idesc_e4m3_f32(BM, BN);
 
 // Shared memory map (offsets from a 1024-byte aligned base). Stage 1 has room for four pipeline stages; stage 2 spends the
-// space of the fourth on staging its output rows.
+// space of the fourth on staging its output rows. Stage 1 with three stages instead: decode layers 0.7 to 2.3 % slower (M=1
+// 50.4 against 49.3 us, Mixtral-shaped M=32 277.1 against 272.5), prefill layers the same within 0.6 %.
 constexpr int kStageRowBytes = 272;                            // staged output row: 64 floats + 16 B (bank spread)
 template <int STAGE>
 struct Smem {
@@ -466,8 +468,9 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
                 // they need half the issue slots of scalar FMAs, and with scalar FMAs the two promotion
                 // warps that share a scheduler with the UMMA-issuing warp starve it (measured: the UMMA
                 // rate halves).
-                // Eight 16-column chunks (16, not 32: sixteen fewer live registers keep this loop, which sits at
-                // the register limit, free of spills - a few spilled values here cost more than 50 %). Sixteen
+                // Eight 16-column chunks (16, not 32: sixteen fewer live registers keep the accumulators of this loop,
+                // which sits at the register limit, in registers - spilling a few of them cost more than 50 %; ptxas
+                // now reports 3 to 13 words a thread spilled, whose cost was not measured by itself). Sixteen
                 // 8-column chunks in two buffers, the next load in flight during the FMAs, measured 3 % slower.
                 uint32_t v[16];
                 if (warp_live) {

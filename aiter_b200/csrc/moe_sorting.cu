@@ -282,6 +282,8 @@ inline int num_chunks(int64_t routes) { return (int)((routes + kChunk - 1) / kCh
 
 }  // namespace
 
+// One counter per chunk and expert, and one more row that nothing uses: the size is part of the ABI (callers may have stored
+// it, and the static scratch below is stated in bytes).
 int64_t sorting_workspace_bytes(int tokens, int num_experts, int topk) {
     int64_t routes = (int64_t)tokens * topk;
     if (routes <= kSingleMaxRoutes) return 0;
@@ -442,8 +444,8 @@ void launch_moe_sorting_noalloc(const aiter_tensor_t* topk_ids, const aiter_tens
                "problem too large for the built-in scratch: ", M * topk, " routes (tokens*topk), the limit is ",
                (int64_t)kStaticMaxChunks * kChunk, " with up to ", kMaxExperts, " experts (", static_scratch_bytes(),
                " bytes held by the library); use b200_moe_sorting_fwd with a caller-provided workspace instead");
-    // Nothing in the scratch has to start at zero: the count kernel writes every counter it covers
-    // and the scan kernel every base before anything reads them.
+    // Nothing in the scratch has to start at zero: the count kernel writes every counter before the
+    // scatter kernel reads it.
     aiter_tensor_t ws{};
     ws.ptr = static_scratch_ptr(topk_ids->device_id);
     ws.numel_ = (size_t)static_scratch_bytes();

@@ -1,7 +1,7 @@
 // Per-row, per-128-column dynamic FP8 e4m3 quantisation (bandwidth kernel).
 // Rounding sequence of the reference's torch oracle (aiter/ops/quant.py:64-94):
-//   amax -> scale = amax / 448 (IEEE division; 0 -> 1) -> code = RNE_e4m3(x / scale) (IEEE division)
-// so the codes and scales are bit-identical to it.  The reference's HIP kernel multiplies by
+//   amax -> scale = amax / 448 (IEEE division; 0 -> 1) -> code = RNE_e4m3(x / scale), the quotient correctly
+// rounded (quant_codes8), so the codes and scales are bit-identical to it.  The reference's HIP kernel multiplies by
 // reciprocals instead (csrc/kernels/quant_kernels.cu:121,159-160), which is not.
 //
 // 16 lanes own one 128-element group (8 bf16 = one 16-byte load each), two groups per warp.
@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(kRowThreads) quant_per_token_kernel(const uint
 }
 
 // Per-tensor dynamic FP8 quantisation (QuantType.per_Tensor; torch twin per_tensor_quant, aiter/ops/quant.py:318-328:
-// scale = max|x| / 448 and codes = RNE_e4m3(x / scale), both IEEE divisions, no zero guard). Two passes:
+// scale = max|x| / 448 and codes = RNE_e4m3(x / scale), both correctly rounded, no zero guard). Two passes:
 // the maximum over the rows below *row_limit goes to amax[0] (non-negative floats order like their bit patterns,
 // so an integer atomicMax does it), then every row is converted with the one scale, which is also written to
 // scale[0] and, if asked, once per row to row_scales (the GEMM kernels take one activation scale per row).

@@ -302,7 +302,7 @@ def fused_moe_stages(hidden_states, w1, w2, topk_weight, topk_ids, expert_mask, 
 
     _mark(timers, "sort")
     # stage 2 accumulates fp32 sums: the sort's zero-filled moe_buf, asked for as [M, model_dim] fp32, is that
-    # accumulator (its spare CTAs clear it beside the scan, so no fill kernel of its own runs); the column-range
+    # accumulator (its spare CTAs clear it beside the sorting ones, so no fill kernel of its own runs); the column-range
     # variant has another layout and clears its own
     sorted_ids, sorted_weights, sorted_expert_ids, num_valid_ids, acc_buf = _moe_sorting_impl(
         topk_ids, topk_weight, global_E, model_dim, dtypes.fp32, GEMM_BLOCK_M, expert_mask,

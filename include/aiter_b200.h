@@ -189,7 +189,8 @@ int b200_moe_stage1(const aiter_tensor_t* a1, const aiter_tensor_t* a1_scale,
  *   [col_begin, col_end) are filled), zero on entry; receives sum over routes of weight * (a2 . w2)
  *   for the output columns [col_begin, col_end) (multiples of 256; col_end <= 0 means model_dim). Launching
  *   the columns in several ranges lets a caller hand finished ranges to a collective while the next is computed;
- *   sm_margin SMs are then left idle by this launch so that the collective's kernels can run beside it.
+ *   sm_margin SMs are then left idle by this launch so that the collective's kernels can run beside it (the next kernel
+ *   of the stream is not placed there either while this one runs).
  *   quant_type 2 (per_Token): a2_scale [P], w2_scale [E,H]. doweight 0 leaves the route weight out
  *   (it was applied in stage 1). */
 int b200_moe_stage2(const aiter_tensor_t* a2, const aiter_tensor_t* a2_scale,
