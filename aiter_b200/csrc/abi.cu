@@ -17,7 +17,7 @@ std::string& last_error() {
 int64_t sorting_workspace_bytes(int tokens, int num_experts, int topk);
 void launch_moe_sorting(const aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*, aiter_tensor_t*,
                         aiter_tensor_t*, aiter_tensor_t*, aiter_tensor_t*, int, int, const aiter_tensor_t*,
-                        const aiter_tensor_t*, aiter_tensor_t*, aiter_tensor_t*, cudaStream_t);
+                        const aiter_tensor_t*, aiter_tensor_t*, aiter_tensor_t*, const BlockLists*, cudaStream_t);
 void launch_moe_sorting_noalloc(const aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*, aiter_tensor_t*,
                                 aiter_tensor_t*, aiter_tensor_t*, aiter_tensor_t*, int, int, const aiter_tensor_t*,
                                 const aiter_tensor_t*, aiter_tensor_t*, cudaStream_t);
@@ -28,10 +28,10 @@ void launch_quant_per_tensor(aiter_tensor_t*, const aiter_tensor_t*, aiter_tenso
                              const aiter_tensor_t*, bool, bool, const int*, int, cudaStream_t);
 void launch_moe_stage1(const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*,
                        const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*,
-                       aiter_tensor_t*, aiter_tensor_t*, int, const aiter_tensor_t*, int, bool, unsigned*, bool, cudaStream_t);
+                       aiter_tensor_t*, aiter_tensor_t*, int, const aiter_tensor_t*, int, bool, unsigned*, bool, SortedStage*, cudaStream_t);
 void launch_moe_stage2(const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*,
                        const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*,
-                       aiter_tensor_t*, aiter_tensor_t*, int, int, int, int, int, bool, cudaStream_t);
+                       aiter_tensor_t*, aiter_tensor_t*, int, int, int, int, int, bool, SortedStage*, cudaStream_t);
 
 int64_t fused_moe_workspace_bytes(int64_t, int64_t, int64_t, int64_t, int64_t, int, int);
 void launch_fused_moe(const b200_fused_moe_args&, cudaStream_t);
@@ -134,7 +134,7 @@ B200_EXPORT int b200_moe_sorting_fwd(const aiter_tensor_t* topk_ids, const aiter
         DeviceGuard g(topk_ids->device_id);
         launch_moe_sorting(topk_ids, topk_weights, sorted_token_ids, sorted_weights, sorted_expert_ids,
                            num_valid_ids, moe_buf, num_experts, unit_size, local_expert_mask, num_local_tokens,
-                           workspace, local_topk_ids, (cudaStream_t)stream);
+                           workspace, local_topk_ids, nullptr, (cudaStream_t)stream);
     });
 }
 
@@ -186,7 +186,8 @@ B200_EXPORT int b200_moe_stage1(const aiter_tensor_t* a1, const aiter_tensor_t* 
         B200_CHECK(a1 != nullptr, "a1 must not be NULL");
         DeviceGuard g(a1->device_id);
         launch_moe_stage1(a1, a1_scale, w1, w1_scale, sorted_token_ids, sorted_expert_ids, num_valid_ids, a2,
-                          a2_scale, status, quant_type, sorted_weights, activation, false, nullptr, false, (cudaStream_t)stream);
+                          a2_scale, status, quant_type, sorted_weights, activation, false, nullptr, false, nullptr,
+                          (cudaStream_t)stream);
     });
 }
 
@@ -200,7 +201,7 @@ B200_EXPORT int b200_moe_stage2(const aiter_tensor_t* a2, const aiter_tensor_t* 
         DeviceGuard g(a2->device_id);
         launch_moe_stage2(a2, a2_scale, w2, w2_scale, sorted_token_ids, sorted_weights, sorted_expert_ids,
                           num_valid_ids, acc, status, col_begin, col_end, sm_margin, quant_type, doweight, false,
-                          (cudaStream_t)stream);
+                          nullptr, (cudaStream_t)stream);
     });
 }
 

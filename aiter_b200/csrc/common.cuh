@@ -84,29 +84,65 @@ inline void check_tensor(const aiter_tensor_t* t, const char* name, int dtype, i
 // must wait before it touches anything (stage 1 and the per_Tensor kernels do). A stage-2 launch that leaves SMs idle does not
 // trigger at all: its successor starts when it is over. Saves the 1-2 us between two dependent short kernels and hides their start-up.
 template <typename... Params, typename... Args>
-inline void launch_kernel(bool overlap, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+inline void launch_kernel(bool overlap, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster,
                           Args&&... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
     cfg.attrs = attr;
-    cfg.numAttrs = overlap ? 1 : 0;
+    if (overlap) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = (unsigned)cluster;
+        attr[cfg.numAttrs].val.clusterDim.y = 1;
+        attr[cfg.numAttrs++].val.clusterDim.z = 1;
+    }
     B200_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...));
 }
 template <typename... Params, typename... Args>
 inline void launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
-    launch_kernel(true, kernel, grid, block, smem, stream, std::forward<Args>(args)...);
+    launch_kernel(true, kernel, grid, block, smem, stream, 1, std::forward<Args>(args)...);
 }
 
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 #endif
+
+// Row blocks of a sorted buffer (128 rows each), split for the GEMM stages: two neighbouring blocks of one expert are a pair,
+// the last block of an expert with an odd number of them is single. Written by the sort, all pointers on the device.
+struct BlockLists {
+    int* counts = nullptr;    // {pairs, singles}
+    int* pairs = nullptr;     // first block of each pair
+    int* singles = nullptr;
+    int64_t max_pairs = 0, max_singles = 0;   // bounds the host knows
+};
+
+// One GEMM stage over activation rows in sorted order (moe_gemm_sorted.cu)
+struct SortedStage {
+    const void* rows;          // [P, K] fp8
+    const float* a_scale;      // [ceil(K/512)][ld][4]; rowwise: [P], or [1] with a_scale_ld 0
+    const void* w;
+    const float* w_scale;
+    void* out;                 // stage 1: [P, I] bf16; stage 2: acc [M, H]
+    const int* sorted_ids;
+    const float* sorted_w;
+    const int* sorted_eids;
+    const int* num_valid;
+    unsigned* amax;
+    int* status;
+    BlockLists lists;
+    int64_t M, H, I, E, P;     // E: experts of the weights
+    int ld;                    // row pitch of block scales
+    int a_scale_ld, w_scale_by_expert, use_weight, activation, device;
+    bool rowwise;
+};
 
 struct DeviceGuard {
     int prev = -1;

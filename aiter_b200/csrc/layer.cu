@@ -3,6 +3,8 @@
 // What it is for: from Python every entry point costs 10-25 us of host time (argument marshalling, allocator, stream
 // lookup), and a decode layer's kernels are over in 50 us: at M=1 the eager layer took 177 us of which the GPU worked 56.
 
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace b200 {
@@ -10,7 +12,7 @@ namespace b200 {
 int64_t sorting_workspace_bytes(int tokens, int num_experts, int topk);
 void launch_moe_sorting(const aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*, aiter_tensor_t*,
                         aiter_tensor_t*, aiter_tensor_t*, aiter_tensor_t*, int, int, const aiter_tensor_t*,
-                        const aiter_tensor_t*, aiter_tensor_t*, aiter_tensor_t*, cudaStream_t);
+                        const aiter_tensor_t*, aiter_tensor_t*, aiter_tensor_t*, const BlockLists*, cudaStream_t);
 void launch_quant_1x128(aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*, const aiter_tensor_t*, int, int, bool, cudaStream_t);
 void launch_quant_per_token(aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*, const aiter_tensor_t*, int, bool,
                             const int*, int, cudaStream_t);
@@ -18,10 +20,11 @@ void launch_quant_per_tensor(aiter_tensor_t*, const aiter_tensor_t*, aiter_tenso
                              const aiter_tensor_t*, bool, bool, const int*, int, cudaStream_t);
 void launch_moe_stage1(const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*,
                        const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*,
-                       aiter_tensor_t*, aiter_tensor_t*, int, const aiter_tensor_t*, int, bool, unsigned*, bool, cudaStream_t);
+                       aiter_tensor_t*, aiter_tensor_t*, int, const aiter_tensor_t*, int, bool, unsigned*, bool, SortedStage*, cudaStream_t);
 void launch_moe_stage2(const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*,
                        const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*, const aiter_tensor_t*,
-                       aiter_tensor_t*, aiter_tensor_t*, int, int, int, int, int, bool, cudaStream_t);
+                       aiter_tensor_t*, aiter_tensor_t*, int, int, int, int, int, bool, SortedStage*, cudaStream_t);
+void launch_gather_rows(const void*, const float*, void*, float*, const int*, const int*, int64_t, int64_t, int64_t, cudaStream_t);
 void launch_finalize(aiter_tensor_t*, const aiter_tensor_t*, cudaStream_t);
 
 namespace {
@@ -29,12 +32,24 @@ namespace {
 constexpr int kQuantPerTensor = 1, kQuantPerToken = 2;   // QuantType of the reference (csrc/include/aiter_enum.h:16-26)
 constexpr int64_t kUnit = 128;                           // sort unit == row tile of the GEMM kernels
 
+// Which layers work their row blocks in pairs (moe_gemm_sorted.cu). Both sides timed in turn, 16 experts, 4 of them a token, in us
+// (pairs / one block a CTA). Pairs want two full blocks of most experts: Qwen3-shaped at 62 / 125 / 250 / 1024 rows an expert 618 / 619,
+// 807 / 812, 1195 / 1241, 3804 / 4178; DeepSeek-V3-shaped at 75 / 150 / 256 rows 2455 / 2454, 3496 / 3594, 5069 / 5313. And stage 2
+// wants K steps that hide the reductions of a tile, 128 inner dimensions each: block scales, H 2048 and 7168, I 512 247 / 250 and
+// 858 / 844, I 1024 375 / 399 and 1190 / 1316. With row scales stage 1 is worked in pairs too, and the copy of its rows into sorted
+// order has to pay: H 2048 and 7168, I 2048 667 / 641 and 774 / 689, I 4096 1061 / 1149 and 1242 / 1257; H 1024, I 4096 715 / 715.
+bool works_in_pairs(int64_t M, int64_t H, int64_t I, int64_t E, int64_t topk, bool rowwise) {
+    return M * topk >= 144 * E && M * topk > kUnit && (rowwise ? I >= 4096 && H >= 2048 : I >= 1024);
+}
+
 // Workspace map: every buffer starts on a 256-byte boundary. Offsets depend on sizes only.
 struct Layout {
-    int64_t P, sorted_ids, sorted_w, sorted_eids, num_valid, sort_ws, acc, a1, a1_scale, a2, a2_scale, a2_half, words, total;
+    bool pairs;
+    int64_t max_pairs, max_singles, lists, P, ld, sorted_ids, sorted_w, sorted_eids, num_valid, sort_ws, acc, a1, a1_scale, a2, a2_scale, a2_half, words, rows, rows_scale, total;
     Layout(int64_t M, int64_t H, int64_t I, int64_t E, int64_t topk, int qt, bool fp8_in) {
         const bool rowwise = qt == kQuantPerToken || qt == kQuantPerTensor;
         P = M * topk + E * kUnit - topk;
+        ld = (P + 31) / 32 * 32;                 // row of a transposed scale array
         int64_t at = 0;
         auto take = [&](int64_t bytes) {
             const int64_t o = at;
@@ -45,14 +60,20 @@ struct Layout {
         sorted_w = take(P * 4);
         sorted_eids = take((P + kUnit - 1) / kUnit * 4);
         num_valid = take(8);
+        max_pairs = M * topk / (kUnit + 1);      // a pair needs more than one block's rows
+        max_singles = std::min(E, M * topk);     // at most one per expert
+        pairs = works_in_pairs(M, H, I, E, topk, rowwise);
+        lists = take(pairs ? (2 + max_pairs + max_singles) * 4 : 0);
         sort_ws = take(sorting_workspace_bytes((int)M, (int)E, (int)topk));
         a1_scale = take(M * (rowwise ? 1 : H / 128) * 4);
-        a2_scale = take(P * (rowwise ? 1 : I / 128) * 4);
+        a2_scale = take(ld * (rowwise ? 1 : (I + 511) / 512 * 4) * 4);
         words = take(256);                       // per_Tensor: a maximum and a scale word per quantisation
         acc = take(M * H * 4);
         a1 = take(fp8_in ? 0 : M * H);
         a2 = take(P * I);
         a2_half = take(rowwise ? P * I * 2 : 0);  // stage-1 activation before the row requantisation
+        rows_scale = take(pairs && rowwise ? P * 4 : 0);
+        rows = take(pairs && rowwise ? P * H : 0);   // activation rows in sorted order
         total = at;
     }
 };
@@ -100,8 +121,14 @@ void launch_fused_moe(const b200_fused_moe_args& a, cudaStream_t stream) {
     aiter_tensor_t mask = tensor(a.expert_mask, I32, dev, a.global_E), live = tensor(a.num_local_tokens, I32, dev, 1);
     const int64_t sort_bytes = sorting_workspace_bytes((int)M, (int)a.global_E, (int)a.topk);
     aiter_tensor_t sort_ws = tensor(ws + at.sort_ws, AITER_DTYPE_u8, dev, sort_bytes);
+    BlockLists lists;
+    lists.counts = (int*)(ws + at.lists);
+    lists.pairs = lists.counts + 2;
+    lists.singles = lists.pairs + at.max_pairs;
+    lists.max_pairs = at.max_pairs;
+    lists.max_singles = at.max_singles;
     launch_moe_sorting(&ids, &wts, &s_ids, &s_w, &s_e, &nv, &cleared, (int)a.global_E, (int)kUnit, a.expert_mask ? &mask : nullptr,
-                       a.num_local_tokens ? &live : nullptr, sort_bytes ? &sort_ws : nullptr, nullptr, stream);
+                       a.num_local_tokens ? &live : nullptr, sort_bytes ? &sort_ws : nullptr, nullptr, at.pairs ? &lists : nullptr, stream);
 
     aiter_tensor_t hidden = tensor(a.hidden, (int)a.hidden_dtype, dev, M, H);
     aiter_tensor_t a1 = hidden, a1_s = rowwise ? tensor(ws + at.a1_scale, F32, dev, M) : tensor(ws + at.a1_scale, F32, dev, M, H / 128);
@@ -124,16 +151,37 @@ void launch_fused_moe(const b200_fused_moe_args& a, cudaStream_t stream) {
     aiter_tensor_t a2_s = rowwise ? tensor(ws + at.a2_scale, F32, dev, at.P) : tensor(ws + at.a2_scale, F32, dev, at.P, I / 128);
     const int gemm_qt = rowwise ? kQuantPerToken : qt;   // one scale per tensor runs through the row-scale kernels
     const aiter_tensor_t* w_stage1 = a.doweight_stage1 ? &s_w : nullptr;
+    SortedStage stage{};
+    SortedStage* in_order = at.pairs ? &stage : nullptr;
+    if (at.pairs) {
+        stage.sorted_ids = (const int*)s_ids.ptr;
+        stage.sorted_w = (const float*)s_w.ptr;
+        stage.sorted_eids = (const int*)s_e.ptr;
+        stage.num_valid = (const int*)nv.ptr;
+        stage.status = (int*)a.status;
+        stage.lists = lists;
+        stage.M = M, stage.H = H, stage.I = I, stage.E = E, stage.P = at.P, stage.ld = (int)at.ld;
+        stage.device = dev;
+        stage.rowwise = rowwise;
+    }
+    if (at.pairs && rowwise) {
+        const bool per_row = (int64_t)a1_s.numel_ == M;   // else one for all
+        float* scales = (float*)(ws + at.rows_scale);
+        launch_gather_rows(a1.ptr, per_row ? (const float*)a1_s.ptr : nullptr, ws + at.rows, scales, stage.sorted_ids, stage.num_valid, M, H, at.P, stream);
+        stage.rows = ws + at.rows;
+        stage.a_scale = per_row ? scales : (const float*)a1_s.ptr;
+        stage.a_scale_ld = per_row;
+    }
     if (rowwise) {
         aiter_tensor_t half = tensor(ws + at.a2_half, AITER_DTYPE_bf16, dev, at.P, I);
         launch_moe_stage1(&a1, &a1_s, &w1, &w1_s, &s_ids, &s_e, &nv, &half, nullptr, &status, gemm_qt, w_stage1, (int)a.activation, true,
-                          per_tensor ? (unsigned*)amax2.ptr : nullptr, per_tensor, stream);
+                          per_tensor ? (unsigned*)amax2.ptr : nullptr, per_tensor, in_order, stream);
         if (per_tensor) launch_quant_per_tensor(&a2, &half, &one2, &amax2, nullptr, &nv, true, true, (const int*)s_ids.ptr, (int)M, stream), a2_s = one2;
         else launch_quant_per_token(&a2, &half, &a2_s, &nv, 1, true, (const int*)s_ids.ptr, (int)M, stream);
     } else {
-        launch_moe_stage1(&a1, &a1_s, &w1, &w1_s, &s_ids, &s_e, &nv, &a2, &a2_s, &status, gemm_qt, w_stage1, (int)a.activation, true, nullptr, false, stream);
+        launch_moe_stage1(&a1, &a1_s, &w1, &w1_s, &s_ids, &s_e, &nv, &a2, &a2_s, &status, gemm_qt, w_stage1, (int)a.activation, true, nullptr, false, in_order, stream);
     }
-    launch_moe_stage2(&a2, &a2_s, &w2, &w2_s, &s_ids, &s_w, &s_e, &nv, &acc, &status, 0, 0, 0, gemm_qt, a.doweight_stage1 ? 0 : 1, per_tensor, stream);
+    launch_moe_stage2(&a2, &a2_s, &w2, &w2_s, &s_ids, &s_w, &s_e, &nv, &acc, &status, 0, 0, 0, gemm_qt, a.doweight_stage1 ? 0 : 1, per_tensor, in_order, stream);
     aiter_tensor_t out = tensor(a.out, (int)a.out_dtype, dev, M, H);
     launch_finalize(&out, &acc, stream);
 }

@@ -31,14 +31,18 @@
 // All mbarrier waits are bounded (sm100_ptx.cuh); if one runs out, status[0] is set and the kernel
 // winds down: every role leaves its loops, the CTA meets at the tail and frees its TMEM.
 
-#include <cuda_fp8.h>
-#include <cuda_bf16.h>
-
-#include "common.cuh"
-#include "quant_device.cuh"
-#include "sm100_ptx.cuh"
+#include "moe_gemm_device.cuh"
 
 namespace b200 {
+
+void launch_sorted_stage1(const SortedStage&, cudaStream_t);
+void launch_sorted_stage2(const SortedStage&, cudaStream_t);
+
+// Process-wide settings of the wait self-test (b200_moe_debug_config): the limit of every device-side wait in SM
+// clocks, and whether the weight producer is stalled. Defaults: the built-in limit, no stall.
+long long g_wait_limit = ptx::kWaitLimitCycles;
+int g_stall_producer = 0;
+
 namespace {
 
 constexpr int BM = 128;            // sorted rows per tile (== sort unit)
@@ -105,7 +109,8 @@ struct GemmParams {
     int n_rows;              // weight rows per expert: 2I (stage 1) or H (stage 2)
     int inter;               // I
     uint8_t* a2;             // stage 1 out [P, I] fp8
-    float* a2_scale;         // stage 1 out [P, I/128]
+    float* a2_scale;         // stage 1 out [P, I/128], or (a2_scale_ld > 0) [ceil(I/512)][a2_scale_ld][4]
+    int a2_scale_ld;
     float* acc;              // stage 2 out [M, H] fp32
     int* status;
     unsigned* amax;          // PT stage 1: maximum magnitude written, as fp32 bits (cleared before the launch), or null
@@ -115,52 +120,6 @@ struct GemmParams {
     long long wait_limit;    // SM clocks after which a device-side wait gives up (sets status, the CTA winds down)
     int stall_producer;      // self-test only: the weight producer loads nothing, so every wait downstream runs out
 };
-
-// torch: silu(x) = x / (1 + exp(-x)) in fp32, then * up (aiter/fused_moe.py:3676).
-// The quotient is formed from an approximate reciprocal and one FMA residual correction (error below
-// one fp32 ulp, like the exp it depends on) instead of the ~4x longer IEEE division sequence.
-__device__ __forceinline__ float silu_mul_fast(float g, float u) {   // valid for g >= -80
-    const float d = 1.0f + expf(-g);
-    const float y = ptx::rcp_approx(d);
-    const float q = g * y;
-    return fmaf(fmaf(-q, d, g), y, q) * u;
-}
-__device__ __forceinline__ float silu_mul_exact(float g, float u) { return __fdiv_rn(g, 1.0f + expf(-g)) * u; }
-
-// torch: gelu(x) = 0.5 * x * (1 + erf(x / sqrt(2))) (the reference's get_torch_act(Gelu) = F.gelu), then * up
-__device__ __forceinline__ float gelu_mul(float g, float u) {
-    return 0.5f * g * (1.0f + erff(g * 0.70710678118654752440f)) * u;
-}
-
-// act(g) * u for N values. The SiLU fast path is straight-line code, so the N dependency chains (exp,
-// reciprocal, two FMAs: ~150 clocks each) interleave; the exact path for exp(-g) near overflow sits behind
-// ONE branch per group. With a branch per value every chain is a basic block of its own and the epilogue runs
-// at the latency of one chain per value (measured: 9.5k of 11.6k clocks per tile).
-template <int ACT, int N>
-__device__ __forceinline__ void act_mul_n(const float (&g)[N], const float (&u)[N], float (&h)[N]) {
-    if (ACT == 1) {
-#pragma unroll
-        for (int i = 0; i < N; ++i) h[i] = gelu_mul(g[i], u[i]);
-        return;
-    }
-    float gmin = g[0];
-#pragma unroll
-    for (int i = 1; i < N; ++i) gmin = fminf(gmin, g[i]);
-#pragma unroll
-    for (int i = 0; i < N; ++i) h[i] = silu_mul_fast(g[i], u[i]);
-    if (gmin < -80.0f) {
-#pragma unroll
-        for (int i = 0; i < N; ++i)
-            if (g[i] < -80.0f) h[i] = silu_mul_exact(g[i], u[i]);
-    }
-}
-
-// acc[0..7] += v[0..15] * s with packed fp32x2 FMAs (one instruction per column pair)
-__device__ __forceinline__ void fold16(float2* acc, const uint32_t* v, float2 s) {
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-        acc[j] = __ffma2_rn(make_float2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1])), s, acc[j]);
-}
 
 // Weight scales of all tiles of this CTA -> L2, a lane per tile (a few hundred bytes each). Without it every tile starts with
 // a DRAM round trip on the promotion warps' path.
@@ -602,7 +561,8 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
 #pragma unroll
                     for (int j = 0; j < 4; ++j) dst[j] = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
                 }
-                if (half == 0 && store) p.a2_scale[(size_t)prow * (p.inter / 128) + nt] = scale;
+                if (half == 0 && store)
+                    p.a2_scale[p.a2_scale_ld ? ((size_t)(nt >> 2) * p.a2_scale_ld + prow) * 4 + (nt & 3) : (size_t)prow * (p.inter / 128) + nt] = scale;
             } else {
                 // out[token] += weight * row  (aiter/fused_moe.py:3802-3811) as fp32 reductions in L2; the
                 // weight is already in the accumulators (it rode on the per-step scales).
@@ -654,60 +614,6 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
 }
 
 // ------------------------------------------------------------------------------------- host
-using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
-                                   CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
-                                   CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_tiled_fn() {
-    static EncodeTiledFn fn = nullptr;
-    if (!fn) {
-        void* sym = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        B200_CUDA(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &qres));
-        B200_CHECK(sym != nullptr && qres == cudaDriverEntryPointSuccess,
-                   "cuTensorMapEncodeTiled is not available in this driver");
-        fn = reinterpret_cast<EncodeTiledFn>(sym);
-    }
-    return fn;
-}
-
-// 2-D view [rows, K] of an fp8 matrix (weights [E, n_rows, K] in boxes of 128 rows x 128 bytes, stage 2's activations in
-// boxes of 32 rows), 128B swizzle. Encoding a map
-// costs a few microseconds of host time, so the last maps are kept (per thread) and reused while pointer and shape
-// repeat, as they do from layer call to layer call.
-CUtensorMap make_map(const void* ptr, uint64_t rows, uint64_t K, uint32_t box_rows) {
-    struct Entry {
-        const void* ptr;
-        uint64_t rows, K;
-        uint32_t box_rows;
-        CUtensorMap map;
-    };
-    constexpr int kEntries = 16;
-    static thread_local Entry cache[kEntries];
-    static thread_local int next = 0, used = 0;
-    for (int i = 0; i < used; ++i)
-        if (cache[i].ptr == ptr && cache[i].rows == rows && cache[i].K == K && cache[i].box_rows == box_rows) return cache[i].map;
-    CUtensorMap m;
-    cuuint64_t dims[2] = {K, rows};
-    cuuint64_t strides[1] = {K};
-    cuuint32_t box[2] = {128, box_rows};
-    cuuint32_t estr[2] = {1, 1};
-    CUresult r = encode_tiled_fn()(&m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(ptr), dims, strides,
-                                   box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    B200_CHECK(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled failed with code ", (int)r);
-    cache[next] = Entry{ptr, rows, K, box_rows, m};
-    next = (next + 1) % kEntries;
-    if (used < kEntries) ++used;
-    return m;
-}
-
-// Process-wide settings of the wait self-test (b200_moe_debug_config): the limit of every device-side wait in SM
-// clocks, and whether the weight producer is stalled. Defaults: the built-in limit, no stall.
-long long g_wait_limit = ptx::kWaitLimitCycles;
-int g_stall_producer = 0;
-
 template <int STAGE, bool PT, int ACT = 0>
 void launch_gemm(const CUtensorMap& tmap, const CUtensorMap& tmap_a, const GemmParams& p, int64_t max_tiles, int dev, cudaStream_t stream,
                  int sm_margin = 0) {
@@ -733,7 +639,7 @@ void launch_gemm(const CUtensorMap& tmap, const CUtensorMap& tmap_a, const GemmP
     // Overlapping the launch with the kernel before it pays while the layer is short. With tens of tiles per SM the few
     // microseconds are nothing, and at the power limit the early CTAs cost more than they give (1-2 % at 65 K routes).
     const bool overlap = max_tiles <= 64 * grid;
-    launch_kernel(overlap, moe_gemm_kernel<STAGE, PT, ACT>, (unsigned)grid, kThreads, Smem<STAGE>::kBytes, stream, tmap, tmap_a, q);
+    launch_kernel(overlap, moe_gemm_kernel<STAGE, PT, ACT>, (unsigned)grid, kThreads, Smem<STAGE>::kBytes, stream, 1, tmap, tmap_a, q);
 }
 
 }  // namespace
@@ -748,7 +654,7 @@ void launch_moe_stage1(const aiter_tensor_t* a1, const aiter_tensor_t* a1_scale,
                        const aiter_tensor_t* sorted_eids, const aiter_tensor_t* num_valid, aiter_tensor_t* a2,
                        aiter_tensor_t* a2_scale, aiter_tensor_t* status, int quant_type,
                        const aiter_tensor_t* sorted_w, int activation, bool skip_pads, unsigned* amax, bool per_tensor,
-                       cudaStream_t stream) {
+                       SortedStage* sorted, cudaStream_t stream) {
     B200_CHECK(activation == 0 || activation == 1, "activation must be Silu (0) or Gelu (1), got ", activation);
     if (sorted_w) {
         check_tensor(sorted_w, "sorted_weights", AITER_DTYPE_fp32, 1);
@@ -797,6 +703,17 @@ void launch_moe_stage1(const aiter_tensor_t* a1, const aiter_tensor_t* a1_scale,
     B200_CHECK(((uintptr_t)a1->ptr & 15) == 0 && ((uintptr_t)w1->ptr & 15) == 0 && ((uintptr_t)a2->ptr & 15) == 0 &&
                    (((uintptr_t)w1_scale->ptr & 15) == 0 || (int64_t)w1_scale->numel_ == E),   // read one by one if per expert
                "a1, w1, w1_scale and a2 must be 16-byte aligned");
+    if (sorted && pt) {   // rows and their scales lie in sorted order there; the rest is as checked above
+        sorted->w = w1->ptr;
+        sorted->w_scale = (const float*)w1_scale->ptr;
+        sorted->w_scale_by_expert = pt && (int64_t)w1_scale->numel_ != E * N2;
+        sorted->out = a2->ptr;
+        sorted->use_weight = sorted_w != nullptr;
+        sorted->activation = activation;
+        sorted->amax = amax;
+        launch_sorted_stage1(*sorted, stream);
+        return;
+    }
 
     GemmParams p{};
     p.a = (const uint8_t*)a1->ptr;
@@ -815,6 +732,7 @@ void launch_moe_stage1(const aiter_tensor_t* a1, const aiter_tensor_t* a1_scale,
     p.inter = (int)I;
     p.a2 = (uint8_t*)a2->ptr;
     p.a2_scale = pt ? nullptr : (float*)a2_scale->ptr;
+    p.a2_scale_ld = sorted ? sorted->ld : 0;
     p.status = (int*)status->ptr;
     p.sorted_w = sorted_w ? (const float*)sorted_w->ptr : nullptr;
     p.skip_pads = skip_pads;
@@ -833,7 +751,7 @@ void launch_moe_stage2(const aiter_tensor_t* a2, const aiter_tensor_t* a2_scale,
                        const aiter_tensor_t* sorted_w, const aiter_tensor_t* sorted_eids,
                        const aiter_tensor_t* num_valid, aiter_tensor_t* acc, aiter_tensor_t* status,
                        int col_begin, int col_end, int sm_margin, int quant_type, int doweight, bool per_tensor,
-                       cudaStream_t stream) {
+                       SortedStage* sorted, cudaStream_t stream) {
     B200_CHECK(quant_type == 4 || quant_type == 5 || quant_type == 2,
                "quant_type must be per_1x128 (4), per_128x128 (5) or per_Token (2), got ", quant_type);
     const bool pt = quant_type == 2;
@@ -881,6 +799,18 @@ void launch_moe_stage2(const aiter_tensor_t* a2, const aiter_tensor_t* a2_scale,
     B200_CHECK(E * H < ((int64_t)1 << 31) && M < (1 << 24), "problem too large");
     B200_CHECK(((uintptr_t)a2->ptr & 15) == 0 && ((uintptr_t)w2->ptr & 15) == 0 && ((uintptr_t)acc->ptr & 15) == 0,
                "a2, w2 and acc must be 16-byte aligned");
+    if (sorted) {
+        sorted->w = w2->ptr;
+        sorted->w_scale = (const float*)w2_scale->ptr;
+        sorted->w_scale_by_expert = pt && (int64_t)w2_scale->numel_ != E * H;
+        sorted->rows = a2->ptr;
+        sorted->a_scale = (const float*)a2_scale->ptr;
+        sorted->a_scale_ld = !pt ? sorted->ld : (int64_t)a2_scale->numel_ >= P ? 1 : 0;
+        sorted->out = acc->ptr;
+        sorted->use_weight = doweight != 0;
+        launch_sorted_stage2(*sorted, stream);
+        return;
+    }
 
     GemmParams p{};
     p.a = (const uint8_t*)a2->ptr;

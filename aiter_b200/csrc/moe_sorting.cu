@@ -52,6 +52,9 @@ struct SortArgs {
     int M, topk, E, unit;
     int max_padded, max_blocks;
     int nchunks;           // CTAs that sort
+    int* counts;           // {pairs, singles} of blocks, or null (BlockLists)
+    int* pairs;
+    int* singles;
     int runs;              // 32-route runs per chunk: 32 times the rounds of kThreads routes a CTA makes
 };
 
@@ -119,7 +122,7 @@ __device__ __forceinline__ int prefix_bytes(const unsigned char* row, int n) {
 }
 
 extern __shared__ __align__(16) unsigned char smem_b[];
-// smem of the sorting CTAs: run_cnt[E][row_bytes] | before[E] | after[E] | start[E] | base[E] | warp_tot[32]
+// smem of the sorting CTAs: run_cnt[E][row_bytes] | before[E] | after[E] | start[E] | base[E] | pairs_at[E] | warp_tot[32] | warp_tot2[32]
 __host__ __device__ inline int row_bytes(int runs) { return runs + 16; }   // + 16: rows start in different banks
 
 // FROM_WS: the routes of the other chunks come from the counts in the workspace; else they are counted here.
@@ -139,7 +142,8 @@ __global__ void __launch_bounds__(kThreads, 1) sort_kernel(SortArgs a) {
     int* after = before + a.E;                                         // ... in later chunks
     int* start = after + a.E;    // position of this chunk's first route of e, -1: expert dropped
     int* base = start + a.E;     // first position of e
-    int2* warp_tot = reinterpret_cast<int2*>(base + a.E);
+    int* pairs_at = base + a.E;  // pairs of blocks of the experts before e
+    int2* warp_tot = reinterpret_cast<int2*>(pairs_at + ((a.E + 1) & ~1));
     for (int i = tid; i < a.E * rb / 16; i += kThreads) reinterpret_cast<uint4*>(run_cnt)[i] = make_uint4(0, 0, 0, 0);
     for (int i = tid; i < a.E; i += kThreads) before[i] = after[i] = 0;
     pdl_wait();
@@ -210,6 +214,16 @@ __global__ void __launch_bounds__(kThreads, 1) sort_kernel(SortArgs a) {
     lid = keep ? 1 : 0;
     at = padded;
     block_scan2_excl(lid, at, warp_tot, total);   // local expert id, first position
+    if (a.counts) {
+        int np = padded / a.unit / 2, ns = padded / a.unit & 1, singles;
+        const int mine = np;
+        block_scan2_excl(np, ns, warp_tot + 32, singles);
+        if (tid < a.E) pairs_at[tid] = np;
+        if (c == 0 && tid == a.E - 1) {
+            a.counts[0] = np + mine;
+            a.counts[1] = singles;
+        }
+    }
     if (tid < a.E) {
         start[tid] = keep ? at + before[tid] : -1;
         base[tid] = keep ? at : -1;
@@ -241,6 +255,11 @@ __global__ void __launch_bounds__(kThreads, 1) sort_kernel(SortArgs a) {
         if (b < 0 || n == 0) continue;
         const int end = b + (n + a.unit - 1) / a.unit * a.unit;
         for (int k = b / a.unit + lane; k < end / a.unit; k += 32) a.sorted_eids[k] = before[x];
+        if (a.counts) {
+            const int first = b / a.unit, blocks = (end - b) / a.unit, at = pairs_at[x];
+            for (int k = lane; k < blocks / 2; k += 32) a.pairs[at + k] = first + 2 * k;
+            if ((blocks & 1) && lane == 0) a.singles[first - 2 * at] = first + blocks - 1;   // blocks before, less those in pairs
+        }
         for (int p = b + n + lane; p < end; p += 32) {
             a.sorted_ids[p] = pad_id;
             a.sorted_w[p] = 0.f;
@@ -295,7 +314,7 @@ void launch_moe_sorting(const aiter_tensor_t* topk_ids, const aiter_tensor_t* to
                         aiter_tensor_t* sorted_eids, aiter_tensor_t* num_valid,
                         aiter_tensor_t* moe_buf, int E, int unit, const aiter_tensor_t* mask,
                         const aiter_tensor_t* num_local, aiter_tensor_t* workspace,
-                        aiter_tensor_t* local_topk_ids, cudaStream_t stream) {
+                        aiter_tensor_t* local_topk_ids, const BlockLists* lists, cudaStream_t stream) {
     check_tensor(topk_ids, "topk_ids", AITER_DTYPE_i32, 2);
     check_tensor(topk_weights, "topk_weights", -1, 2);
     B200_CHECK(topk_weights->dtype_ == AITER_DTYPE_fp32, "topk_weights must be FP32 (float32)");
@@ -351,6 +370,11 @@ void launch_moe_sorting(const aiter_tensor_t* topk_ids, const aiter_tensor_t* to
     a.unit = unit;
     a.max_padded = (int)max_padded;
     a.max_blocks = (int)max_blocks;
+    if (lists) {
+        a.counts = lists->counts;
+        a.pairs = lists->pairs;
+        a.singles = lists->singles;
+    }
 
     int zero_ctas = 0;
     if (moe_buf && moe_buf->numel_ > 0) {
@@ -375,11 +399,11 @@ void launch_moe_sorting(const aiter_tensor_t* topk_ids, const aiter_tensor_t* to
     a.nchunks = std::max(1, num_chunks(routes));
     a.runs = kWarps * (int)((std::min<int64_t>(routes, kChunk) + kThreads - 1) / kThreads);
     if (a.runs < kWarps) a.runs = kWarps;
-    const size_t smem = (size_t)E * row_bytes(a.runs) + 4 * (size_t)E * sizeof(int) + 32 * sizeof(int2);
+    const size_t smem = (size_t)E * row_bytes(a.runs) + (5 * (size_t)E + 2) * sizeof(int) + 64 * sizeof(int2);
     static bool attr_set[64] = {false};
     const int dev = topk_ids->device_id;
     if (dev >= 64 || !attr_set[dev]) {
-        const int most = kMaxExperts * row_bytes(kChunk / 32) + 4 * kMaxExperts * (int)sizeof(int) + 32 * (int)sizeof(int2);
+        const int most = kMaxExperts * row_bytes(kChunk / 32) + (5 * kMaxExperts + 2) * (int)sizeof(int) + 64 * (int)sizeof(int2);
         B200_CUDA(cudaFuncSetAttribute(sort_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
         B200_CUDA(cudaFuncSetAttribute(sort_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
         if (dev < 64) attr_set[dev] = true;
@@ -455,7 +479,7 @@ void launch_moe_sorting_noalloc(const aiter_tensor_t* topk_ids, const aiter_tens
     ws.dtype_ = AITER_DTYPE_u8;
     ws.device_id = topk_ids->device_id;
     launch_moe_sorting(topk_ids, topk_weights, sorted_ids, sorted_w, sorted_eids, num_valid, moe_buf, E, unit,
-                       mask, num_local, need > 0 ? &ws : nullptr, local_topk_ids, stream);
+                       mask, num_local, need > 0 ? &ws : nullptr, local_topk_ids, nullptr, stream);
 }
 
 }  // namespace b200
