@@ -81,7 +81,9 @@ inline void check_tensor(const aiter_tensor_t* t, const char* name, int dtype, i
 // run. What works before its own wait relies on this and names the kernel it may run beside: the fill of the two-kernel sort
 // (its predecessor is always the count kernel, whose sorting CTAs trigger after their wait) and the layer's activation
 // quantiser (its predecessor is always the sort). That quantiser triggers BEFORE its wait, so whatever is launched behind it
-// must wait before it touches anything (stage 1 and the per_Tensor kernels do). A stage-2 launch that leaves SMs idle does not
+// must wait before it touches anything (stage 1 and the per_Tensor kernels do). The launch over the single blocks of a stage, whose
+// predecessor is always the launch over its pairs, waits at its end only and triggers before, so the same holds for its successors
+// (the requantisers, stage 2's pairs, the final rounding). A stage-2 launch that leaves SMs idle does not
 // trigger at all: its successor starts when it is over. Saves the 1-2 us between two dependent short kernels and hides their start-up.
 template <typename... Params, typename... Args>
 inline void launch_kernel(bool overlap, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster,

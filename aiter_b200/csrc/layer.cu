@@ -32,8 +32,8 @@ namespace {
 constexpr int kQuantPerTensor = 1, kQuantPerToken = 2;   // QuantType of the reference (csrc/include/aiter_enum.h:16-26)
 constexpr int64_t kUnit = 128;                           // sort unit == row tile of the GEMM kernels
 
-// Which layers work their row blocks in pairs (moe_gemm_sorted.cu). Both sides timed in turn, 16 experts, 4 of them a token, in us
-// (pairs / one block a CTA). Pairs want two full blocks of most experts: Qwen3-shaped at 62 / 125 / 250 / 1024 rows an expert 618 / 619,
+// Which layers work their row blocks in pairs (moe_gemm_sorted.cu). Both sides timed in turn, in us (pairs / one block a CTA); those
+// named by H and I have 16 experts, 4 of them a token, and 8192 tokens (3000 where H x I is above 8 M). Pairs want two full blocks of most experts: Qwen3-shaped at 62 / 125 / 250 / 1024 rows an expert 618 / 619,
 // 807 / 812, 1195 / 1241, 3804 / 4178; DeepSeek-V3-shaped at 75 / 150 / 256 rows 2455 / 2454, 3496 / 3594, 5069 / 5313. And stage 2
 // wants K steps that hide the reductions of a tile, 128 inner dimensions each: block scales, H 2048 and 7168, I 512 247 / 250 and
 // 858 / 844, I 1024 375 / 399 and 1190 / 1316. With row scales stage 1 is worked in pairs too, and the copy of its rows into sorted
