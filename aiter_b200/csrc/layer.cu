@@ -10,6 +10,7 @@
 namespace b200 {
 
 int64_t sorting_workspace_bytes(int tokens, int num_experts, int topk);
+int sorting_launches(int64_t routes);
 void launch_moe_sorting(const aiter_tensor_t*, const aiter_tensor_t*, aiter_tensor_t*, aiter_tensor_t*,
                         aiter_tensor_t*, aiter_tensor_t*, aiter_tensor_t*, int, int, const aiter_tensor_t*,
                         const aiter_tensor_t*, aiter_tensor_t*, aiter_tensor_t*, const BlockLists*, cudaStream_t);
@@ -99,6 +100,18 @@ aiter_tensor_t tensor(const void* ptr, int dtype, int dev, int64_t d0, int64_t d
 
 int64_t fused_moe_workspace_bytes(int64_t M, int64_t H, int64_t I, int64_t E, int64_t topk, int qt, int hidden_dtype) {
     return Layout(M, H, I, E, topk, qt, hidden_dtype == AITER_DTYPE_fp8).total;
+}
+
+// Kernels that launch_fused_moe below enqueues for these sizes.
+int fused_moe_launches(int64_t M, int64_t H, int64_t I, int64_t E, int64_t topk, int qt, int hidden_dtype) {
+    const bool per_tensor = qt == kQuantPerTensor, rowwise = per_tensor || qt == kQuantPerToken;
+    const bool pairs = works_in_pairs(M, H, I, E, topk, rowwise);
+    int n = sorting_launches(M * topk);
+    if (hidden_dtype != AITER_DTYPE_fp8) n += per_tensor ? 2 : 1;   // maximum, codes
+    n += pairs && rowwise ? 3 : 1;                                  // stage 1: rows in order, pairs, single blocks
+    n += rowwise ? 1 : 0;                                           // requantisation
+    n += pairs ? 2 : 1;                                             // stage 2
+    return n + 1;                                                   // final rounding
 }
 
 void launch_fused_moe(const b200_fused_moe_args& a, cudaStream_t stream) {

@@ -309,6 +309,8 @@ int64_t sorting_workspace_bytes(int tokens, int num_experts, int topk) {
     return ((int64_t)num_chunks(routes) * num_experts + num_experts) * (int64_t)sizeof(int);
 }
 
+int sorting_launches(int64_t routes) { return routes <= kSingleMaxRoutes ? 1 : 2; }
+
 void launch_moe_sorting(const aiter_tensor_t* topk_ids, const aiter_tensor_t* topk_weights,
                         aiter_tensor_t* sorted_ids, aiter_tensor_t* sorted_w,
                         aiter_tensor_t* sorted_eids, aiter_tensor_t* num_valid,

@@ -404,8 +404,10 @@ _LAYER_ARGS = struct.Struct("@13P16q")
 
 
 @functools.lru_cache(maxsize=1024)
-def _layer_workspace_bytes(M, H, I, E, topk, qt, hidden_code):
-    return int(_lib.lib().b200_fused_moe_workspace_size(M, H, I, E, topk, qt, hidden_code))
+def _layer_sizes(*sizes):
+    """Workspace bytes and kernel launches of a layer call; sizes: M, H, I, global_E, topk, quant type, hidden dtype code."""
+    handle = _lib.lib()
+    return int(handle.b200_fused_moe_workspace_size(*sizes)), int(handle.b200_fused_moe_launches(*sizes))
 
 
 def _ptr(t):
@@ -415,8 +417,9 @@ def _ptr(t):
 def _layer(hidden_states, w1, w2, topk_weight, topk_ids, expert_mask, w1_scale, w2_scale, a1_scale, num_local_tokens, dtype,
            quant_type, activation, doweight_stage1):
     """The layer through the one-call entry point: one workspace, one FFI crossing. Arguments as ``fused_moe`` checked
-    them; the tensors' sizes are checked natively. Same kernels and results as ``fused_moe_stages``, which remains for
-    callers that need the stages apart (event marks, column ranges, fp32 sums, intermediates)."""
+    them; the tensors' sizes are checked natively. Same arithmetic as ``fused_moe_stages``, which remains for callers that
+    need the stages apart (event marks, column ranges, fp32 sums, intermediates); large batches run GEMM kernels of their
+    own here (csrc/moe_gemm_sorted.cu)."""
     device = hidden_states.device
     index = hidden_states.get_device()
     M, topk = topk_ids.shape
@@ -445,7 +448,7 @@ def _layer(hidden_states, w1, w2, topk_weight, topk_ids, expert_mask, w1_scale, 
         a1_scale = a1_scale.contiguous()
     global_E = E if expert_mask is None else expert_mask.numel()
     code = dtypes.AITER_DTYPE[hidden_states.dtype]
-    nbytes = _layer_workspace_bytes(M, H, I, global_E, topk, int(quant_type), code)
+    nbytes, launches = _layer_sizes(M, H, I, global_E, topk, int(quant_type), code)
     workspace = torch.empty(nbytes, dtype=dtypes.u8, device=device)
     out = torch.empty((M, H), dtype=dtype, device=device)
     args = _LAYER_ARGS.pack(
@@ -456,15 +459,8 @@ def _layer(hidden_states, w1, w2, topk_weight, topk_ids, expert_mask, w1_scale, 
         code, dtypes.AITER_DTYPE[dtype], int(quant_type), int(activation), int(doweight_stage1), index)
     if _lib._fn("b200_fused_moe")(args, _lib.current_stream(index)) != 0:
         _lib.raise_last_error("b200_fused_moe")
-    _lib.launch_count += _layer_launches(M * topk, quant_type, code)
+    _lib.launch_count += launches
     return out
-
-
-def _layer_launches(routes, quant_type, hidden_code):
-    """Kernels behind one layer call (for ``_lib.launch_count``): sort, quantiser, two GEMMs, requantiser, final rounding."""
-    quant = _lib._KERNELS_PER_CALL["b200_moe_quant_per_tensor"] if quant_type == QuantType.per_Tensor else 1
-    a1 = 0 if hidden_code == dtypes.AITER_DTYPE[dtypes.fp8] else quant
-    return (2 if routes > 16384 else 1) + a1 + (0 if quant_type == QuantType.per_1x128 else quant) + 3
 
 
 def fused_moe(

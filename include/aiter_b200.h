@@ -134,8 +134,9 @@ int b200_moe_quant_per_tensor(aiter_tensor_t* out, const aiter_tensor_t* input, 
                               void* stream);
 
 /* The whole layer of aiter.fused_moe in one call: sort -> activation quantisation -> stage 1 -> (row requantisation)
- * -> stage 2 -> final rounding, enqueued on one stream from one host call. Same kernels and results as the separate
- * entry points below; a caller pays one FFI crossing and one workspace instead of six calls and a dozen buffers.
+ * -> stage 2 -> final rounding, enqueued on one stream from one host call. Same arithmetic as the separate entry points
+ * below (large batches run GEMM kernels of their own, with the rows in sorted order and two CTAs on a tile); a caller
+ * pays one FFI crossing and one workspace instead of six calls and a dozen buffers.
  * All pointers are device pointers on `device` (16-byte aligned), all tensors contiguous; optional ones are NULL. */
 typedef struct b200_fused_moe_args {
     const void* hidden;            /* [M,H] bf16 | fp16 | fp8 (hidden_dtype) */
@@ -158,6 +159,9 @@ typedef struct b200_fused_moe_args {
 
 int64_t b200_fused_moe_workspace_size(int64_t M, int64_t H, int64_t I, int64_t global_E, int64_t topk, int quant_type,
                                       int hidden_dtype);
+/* Kernels that b200_fused_moe enqueues for these sizes (callers that report how many kernels they ran) */
+int b200_fused_moe_launches(int64_t M, int64_t H, int64_t I, int64_t global_E, int64_t topk, int quant_type,
+                            int hidden_dtype);
 int b200_fused_moe(const b200_fused_moe_args* args, void* stream);
 
 /* Stage 1: grouped gate/up GEMM over the sorted blocks + SiLU(gate)*up + bf16 rounding +

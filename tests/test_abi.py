@@ -77,6 +77,18 @@ def test_workspace_size(lib):
     assert ws == (16 * 256 + 256) * 4
 
 
+# M, H, I, experts, topk, quant type, hidden dtype; kernels: sort (two above 16384 routes), quantiser (none for fp8, two for one scale
+# per tensor), stage 1, requantisation of row scales, stage 2, final rounding; layers in pairs: two launches a stage, and with row
+# scales the copy into sorted order
+@pytest.mark.parametrize("sizes,kernels", [
+    ((1, 4096, 1536, 128, 8, 4, torch.bfloat16), 5), ((513, 1024, 512, 8, 2, 1, torch.bfloat16), 7),
+    ((32, 4096, 14336, 8, 2, 2, torch.float16), 6), ((2048, 7168, 2048, 256, 8, 4, torch.float8_e4m3fn), 4),
+    ((3000, 7168, 512, 256, 8, 4, torch.bfloat16), 6), ((4096, 4096, 14336, 8, 2, 2, torch.bfloat16), 9),
+    ((9000, 4096, 14336, 8, 2, 1, torch.bfloat16), 11), ((16384, 4096, 1536, 128, 8, 4, torch.bfloat16), 7)])
+def test_kernels_of_a_layer_call(lib, sizes, kernels):
+    assert lib.b200_fused_moe_launches(*sizes[:-1], _lib.AITER_DTYPE[sizes[-1]]) == kernels
+
+
 def test_unsupported_options_are_named():
     x = torch.zeros((4, 256), dtype=torch.bfloat16)
     w1 = torch.zeros((2, 512, 256), dtype=torch.float8_e4m3fn)
