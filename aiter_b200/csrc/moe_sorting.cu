@@ -22,6 +22,7 @@
 // Extra CTAs zero-fill moe_buf when the caller passes one.
 
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -52,10 +53,15 @@ struct SortArgs {
     int M, topk, E, unit;
     int max_padded, max_blocks;
     int nchunks;           // CTAs that sort
-    int* counts;           // {pairs, singles} of blocks, or null (BlockLists)
+    int runs;              // 32-route runs per chunk: 32 times the rounds of kThreads routes a CTA makes
+};
+
+// ... and lists the pairs and single blocks besides (BlockLists). A type of its own, so that the sorts of all other callers
+// carry none of it: with the lists behind a branch of the one kernel a one-token layer took 49.7 us, without them 47.9.
+struct SortArgsLists : SortArgs {
+    int* counts;           // {pairs, singles}
     int* pairs;
     int* singles;
-    int runs;              // 32-route runs per chunk: 32 times the rounds of kThreads routes a CTA makes
 };
 
 __device__ __forceinline__ int eff_tokens(const SortArgs& a) {
@@ -122,12 +128,17 @@ __device__ __forceinline__ int prefix_bytes(const unsigned char* row, int n) {
 }
 
 extern __shared__ __align__(16) unsigned char smem_b[];
-// smem of the sorting CTAs: run_cnt[E][row_bytes] | before[E] | after[E] | start[E] | base[E] | pairs_at[E] | warp_tot[32] | warp_tot2[32]
+// smem of the sorting CTAs: run_cnt[E][row_bytes] | before[E] | after[E] | start[E] | base[E] | warp_tot[32]; with lists, behind it:
+// warp_tot2[32] | pairs_at[E]
 __host__ __device__ inline int row_bytes(int runs) { return runs + 16; }   // + 16: rows start in different banks
+inline size_t sort_smem(int E, int runs, bool with_lists) {
+    return (size_t)E * row_bytes(runs) + 4 * (size_t)E * sizeof(int) + 32 * sizeof(int2) + (with_lists ? 32 * sizeof(int2) + (size_t)E * sizeof(int) : 0);
+}
 
 // FROM_WS: the routes of the other chunks come from the counts in the workspace; else they are counted here.
-template <bool FROM_WS>
-__global__ void __launch_bounds__(kThreads, 1) sort_kernel(SortArgs a) {
+template <bool FROM_WS, typename Args>
+__global__ void __launch_bounds__(kThreads, 1) sort_kernel(Args a) {
+    constexpr bool kLists = std::is_same<Args, SortArgsLists>::value;
     if ((int)blockIdx.x >= a.nchunks) {
         // the fill beside the two-kernel sort starts at once: the kernel before it is the count, which does not touch moe_buf
         if (!FROM_WS) pdl_wait();
@@ -142,8 +153,8 @@ __global__ void __launch_bounds__(kThreads, 1) sort_kernel(SortArgs a) {
     int* after = before + a.E;                                         // ... in later chunks
     int* start = after + a.E;    // position of this chunk's first route of e, -1: expert dropped
     int* base = start + a.E;     // first position of e
-    int* pairs_at = base + a.E;  // pairs of blocks of the experts before e
-    int2* warp_tot = reinterpret_cast<int2*>(pairs_at + ((a.E + 1) & ~1));
+    int2* warp_tot = reinterpret_cast<int2*>(base + a.E);
+    int* pairs_at = reinterpret_cast<int*>(warp_tot + 64);   // pairs of blocks of the experts before e
     for (int i = tid; i < a.E * rb / 16; i += kThreads) reinterpret_cast<uint4*>(run_cnt)[i] = make_uint4(0, 0, 0, 0);
     for (int i = tid; i < a.E; i += kThreads) before[i] = after[i] = 0;
     pdl_wait();
@@ -214,7 +225,7 @@ __global__ void __launch_bounds__(kThreads, 1) sort_kernel(SortArgs a) {
     lid = keep ? 1 : 0;
     at = padded;
     block_scan2_excl(lid, at, warp_tot, total);   // local expert id, first position
-    if (a.counts) {
+    if constexpr (kLists) {
         int np = padded / a.unit / 2, ns = padded / a.unit & 1, singles;
         const int mine = np;
         block_scan2_excl(np, ns, warp_tot + 32, singles);
@@ -255,7 +266,7 @@ __global__ void __launch_bounds__(kThreads, 1) sort_kernel(SortArgs a) {
         if (b < 0 || n == 0) continue;
         const int end = b + (n + a.unit - 1) / a.unit * a.unit;
         for (int k = b / a.unit + lane; k < end / a.unit; k += 32) a.sorted_eids[k] = before[x];
-        if (a.counts) {
+        if constexpr (kLists) {
             const int first = b / a.unit, blocks = (end - b) / a.unit, at = pairs_at[x];
             for (int k = lane; k < blocks / 2; k += 32) a.pairs[at + k] = first + 2 * k;
             if ((blocks & 1) && lane == 0) a.singles[first - 2 * at] = first + blocks - 1;   // blocks before, less those in pairs
@@ -356,7 +367,7 @@ void launch_moe_sorting(const aiter_tensor_t* topk_ids, const aiter_tensor_t* to
                    "local_topk_ids must have the same [tokens, topk] shape as topk_ids");
     }
 
-    SortArgs a{};
+    SortArgsLists a{};
     a.ids = (const int*)topk_ids->ptr;
     a.weights = (const float*)topk_weights->ptr;
     a.mask = mask ? (const int*)mask->ptr : nullptr;
@@ -401,17 +412,20 @@ void launch_moe_sorting(const aiter_tensor_t* topk_ids, const aiter_tensor_t* to
     a.nchunks = std::max(1, num_chunks(routes));
     a.runs = kWarps * (int)((std::min<int64_t>(routes, kChunk) + kThreads - 1) / kThreads);
     if (a.runs < kWarps) a.runs = kWarps;
-    const size_t smem = (size_t)E * row_bytes(a.runs) + (5 * (size_t)E + 2) * sizeof(int) + 64 * sizeof(int2);
+    const size_t smem = sort_smem(E, a.runs, lists != nullptr);
     static bool attr_set[64] = {false};
     const int dev = topk_ids->device_id;
     if (dev >= 64 || !attr_set[dev]) {
-        const int most = kMaxExperts * row_bytes(kChunk / 32) + (5 * kMaxExperts + 2) * (int)sizeof(int) + 64 * (int)sizeof(int2);
-        B200_CUDA(cudaFuncSetAttribute(sort_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-        B200_CUDA(cudaFuncSetAttribute(sort_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+        const int most = (int)sort_smem(kMaxExperts, kChunk / 32, false), most_lists = (int)sort_smem(kMaxExperts, kChunk / 32, true);
+        B200_CUDA(cudaFuncSetAttribute(sort_kernel<false, SortArgs>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+        B200_CUDA(cudaFuncSetAttribute(sort_kernel<true, SortArgs>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+        B200_CUDA(cudaFuncSetAttribute(sort_kernel<false, SortArgsLists>, cudaFuncAttributeMaxDynamicSharedMemorySize, most_lists));
+        B200_CUDA(cudaFuncSetAttribute(sort_kernel<true, SortArgsLists>, cudaFuncAttributeMaxDynamicSharedMemorySize, most_lists));
         if (dev < 64) attr_set[dev] = true;
     }
     if (routes <= kSingleMaxRoutes) {
-        launch_pdl(sort_kernel<false>, a.nchunks + zero_ctas, kThreads, smem, stream, a);
+        if (lists) launch_pdl(sort_kernel<false, SortArgsLists>, a.nchunks + zero_ctas, kThreads, smem, stream, a);
+        else launch_pdl(sort_kernel<false, SortArgs>, a.nchunks + zero_ctas, kThreads, smem, stream, a);
     } else {
         const int64_t need = sorting_workspace_bytes((int)M, E, (int)topk);
         B200_CHECK(workspace != nullptr && workspace->ptr != nullptr,
@@ -422,7 +436,8 @@ void launch_moe_sorting(const aiter_tensor_t* topk_ids, const aiter_tensor_t* to
         B200_CHECK((int64_t)(workspace->numel_ * ws_esz) >= need, "workspace needs ", need, " bytes");
         a.ws_cnt = (int*)workspace->ptr;
         launch_pdl(sort_count_kernel, a.nchunks, kThreads, (size_t)E * sizeof(int), stream, a);
-        launch_pdl(sort_kernel<true>, a.nchunks + zero_ctas, kThreads, smem, stream, a);
+        if (lists) launch_pdl(sort_kernel<true, SortArgsLists>, a.nchunks + zero_ctas, kThreads, smem, stream, a);
+        else launch_pdl(sort_kernel<true, SortArgs>, a.nchunks + zero_ctas, kThreads, smem, stream, a);
     }
 }
 
