@@ -67,7 +67,7 @@ struct Layout {
         lists = take(pairs ? (2 + max_pairs + max_singles) * 4 : 0);
         sort_ws = take(sorting_workspace_bytes((int)M, (int)E, (int)topk));
         a1_scale = take(M * (rowwise ? 1 : H / 128) * 4);
-        a2_scale = take(ld * (rowwise ? 1 : (I + 511) / 512 * 4) * 4);
+        a2_scale = take(rowwise ? P * 4 : pairs ? ld * ((I + 511) / 512 * 4) * 4 : P * (I / 128) * 4);
         words = take(256);                       // per_Tensor: a maximum and a scale word per quantisation
         acc = take(M * H * 4);
         a1 = take(fp8_in ? 0 : M * H);

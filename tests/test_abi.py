@@ -89,6 +89,20 @@ def test_kernels_of_a_layer_call(lib, sizes, kernels):
     assert lib.b200_fused_moe_launches(*sizes[:-1], _lib.AITER_DTYPE[sizes[-1]]) == kernels
 
 
+def test_workspace_of_a_layer(lib):
+    """Bytes of a layer that is not worked in pairs: what its kernels use, buffer by buffer, and nothing for the pairs."""
+    M, H, I, E, topk = 513, 1024, 640, 8, 2
+    P = M * topk + E * 128 - topk
+    def up(n):
+        return -(-n // 256) * 256
+    common = 2 * up(4 * P) + up(4 * (-(-P // 128))) + up(8) + 256 + up(4 * M * H) + up(M * H) + up(P * I)
+    block = common + up(4 * M * H // 128) + up(4 * P * I // 128)
+    rows = common + up(4 * M) + up(4 * P) + up(2 * P * I)
+    bf16 = _lib.AITER_DTYPE[torch.bfloat16]
+    assert lib.b200_fused_moe_workspace_size(M, H, I, E, topk, 4, bf16) == block
+    assert lib.b200_fused_moe_workspace_size(M, H, I, E, topk, 2, bf16) == rows
+
+
 def test_unsupported_options_are_named():
     x = torch.zeros((4, 256), dtype=torch.bfloat16)
     w1 = torch.zeros((2, 512, 256), dtype=torch.float8_e4m3fn)
