@@ -34,7 +34,8 @@ void launch_moe_stage2(const aiter_tensor_t*, const aiter_tensor_t*, const aiter
                        aiter_tensor_t*, aiter_tensor_t*, int, int, int, int, int, bool, SortedStage*, cudaStream_t);
 
 int64_t fused_moe_workspace_bytes(int64_t, int64_t, int64_t, int64_t, int64_t, int, int);
-int fused_moe_launches(int64_t, int64_t, int64_t, int64_t, int64_t, int, int);
+int fused_moe_launches(int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int, int);
+void set_debug_pairs(int);
 void launch_fused_moe(const b200_fused_moe_args&, cudaStream_t);
 void launch_finalize(aiter_tensor_t*, const aiter_tensor_t*, cudaStream_t);
 
@@ -214,6 +215,13 @@ B200_EXPORT int b200_moe_debug_config(int64_t wait_limit_cycles, int stall_weigh
     return safe_call([&] { set_gemm_debug((long long)wait_limit_cycles, stall_weight_producer); });
 }
 
+B200_EXPORT int b200_moe_debug_pairs(int mode) {
+    return safe_call([&] {
+        B200_CHECK(mode >= 0 && mode <= 2, "mode must be 0, 1 or 2, got ", mode);
+        set_debug_pairs(mode);
+    });
+}
+
 B200_EXPORT int b200_biased_grouped_topk(const aiter_tensor_t* gating_output, const aiter_tensor_t* correction_bias,
                                          aiter_tensor_t* topk_weights, aiter_tensor_t* topk_ids, int num_expert_group,
                                          int topk_group, int need_renorm, float routed_scaling_factor, void* stream) {
@@ -249,9 +257,9 @@ B200_EXPORT int64_t b200_fused_moe_workspace_size(int64_t M, int64_t H, int64_t 
     return fused_moe_workspace_bytes(M, H, I, global_E, topk, quant_type, hidden_dtype);
 }
 
-B200_EXPORT int b200_fused_moe_launches(int64_t M, int64_t H, int64_t I, int64_t global_E, int64_t topk, int quant_type,
+B200_EXPORT int b200_fused_moe_launches(int64_t M, int64_t H, int64_t I, int64_t E, int64_t global_E, int64_t topk, int quant_type,
                                         int hidden_dtype) {
-    return fused_moe_launches(M, H, I, global_E, topk, quant_type, hidden_dtype);
+    return fused_moe_launches(M, H, I, E, global_E, topk, quant_type, hidden_dtype);
 }
 
 B200_EXPORT int b200_fused_moe(const b200_fused_moe_args* args, void* stream) {

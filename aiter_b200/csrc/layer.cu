@@ -33,22 +33,40 @@ namespace {
 constexpr int kQuantPerTensor = 1, kQuantPerToken = 2;   // QuantType of the reference (csrc/include/aiter_enum.h:16-26)
 constexpr int64_t kUnit = 128;                           // sort unit == row tile of the GEMM kernels
 
-// Which layers work their row blocks in pairs (moe_gemm_sorted.cu). Both sides timed in turn, in us (pairs / one block a CTA); those
-// named by H and I have 16 experts, 4 of them a token, and 8192 tokens (3000 where H x I is above 8 M). Pairs want two full blocks of most experts: Qwen3-shaped at 62 / 125 / 250 / 1024 rows an expert 618 / 619,
-// 807 / 812, 1195 / 1241, 3804 / 4178; DeepSeek-V3-shaped at 75 / 150 / 256 rows 2455 / 2454, 3496 / 3594, 5069 / 5313. And stage 2
-// wants K steps that hide the reductions of a tile, 128 inner dimensions each: block scales, H 2048 and 7168, I 512 247 / 250 and
-// 858 / 844, I 1024 375 / 399 and 1190 / 1316. With row scales stage 1 is worked in pairs too, and the copy of its rows into sorted
-// order has to pay: H 2048 and 7168, I 2048 667 / 641 and 774 / 689, I 4096 1061 / 1149 and 1242 / 1257; H 1024, I 4096 715 / 715.
-bool works_in_pairs(int64_t M, int64_t H, int64_t I, int64_t E, int64_t topk, bool rowwise) {
-    return M * topk >= 144 * E && M * topk > kUnit && (rowwise ? I >= 4096 && H >= 2048 : I >= 1024);
+// What tests ask of the calls of their thread (b200_moe_debug_pairs): 0 the rule below, 1 pairs wherever there can be one, 2 none.
+thread_local int t_debug_pairs = 0;
+
+// Which layers work their row blocks in pairs (moe_gemm_sorted.cu). E: experts of this layer call, of global_E that are routed to.
+// Timed both ways in turn as graphs: 1132 block-scaled and 699 row-scaled layers, H 512 to 8192, I 1024 to 14336, 8 to 256 experts, 150
+// to 1024 rows an expert, even and Zipf routing. Gain: time with one block a CTA / time in pairs, mean (least).
+//  * Rows. Below 144 an expert most have one block. Experts with three blocks leave one of them single, at the price of a pair each:
+//    block scales at 220 / 300 / 400 rows 1.05 / 1.00 (0.96) / 1.04, row scales 1.15 / 1.00 (0.95) / 1.10; with row scales and I 4096
+//    the fifth block is too much as well, at 600 rows 0.99 (0.97).
+//  * Block scales, stage 2 only: a second launch, 2 to 4 us, and tiles of twice the size want several rounds of tiles. By rounds of
+//    128 x 256 tiles on all SMs below 1: 0.94 (0.88), 1-3: 0.98 (0.90), 3-6: 1.00 (0.95), 6-12: 1.02, 12-24: 1.03, above: 1.05.
+//  * Row scales, both stages: three launches and a copy of the rows, 10 to 20 us, against a gain that grows with the rounds of
+//    stage 1 and with I, less below H 4096. The 291 layers beyond the line 1.085 (0.986; with I 4096 / 6144 / 8192 / 14336 1.03 / 1.07 / 1.08 / 1.10),
+//    the 408 before it 1.00 (0.80).
+bool works_in_pairs(int64_t M, int64_t H, int64_t I, int64_t E, int64_t global_E, int64_t topk, bool rowwise) {
+    constexpr double kSms = 148;
+    const int64_t routes = M * topk;
+    if (t_debug_pairs) return t_debug_pairs == 1 && routes > kUnit;
+    if (global_E < 1 || routes < 144 * global_E || routes <= kUnit) return false;
+    const int64_t rows = routes / global_E, blocks = (rows + kUnit - 8) / kUnit;   // an expert, 8 rows either way
+    if (blocks % 2 && (rows + 8) / kUnit < blocks && blocks <= (rowwise && I < 6144 ? 5 : 3)) return false;
+    const double here = (double)routes * std::min(E, global_E) / global_E / kUnit;   // blocks of rows in this call
+    if (!rowwise) return I >= 1024 && here * H / 256 >= 6 * kSms;
+    return I >= 4096 && H >= 2048 && here * I / 128 / kSms * I * std::min<int64_t>(H, 4096) >= 98304. * 4096;
 }
 
 // Workspace map: every buffer starts on a 256-byte boundary. Offsets depend on sizes only.
 struct Layout {
     bool pairs;
-    int64_t max_pairs, max_singles, lists, P, ld, sorted_ids, sorted_w, sorted_eids, num_valid, sort_ws, acc, a1, a1_scale, a2, a2_scale, a2_half, words, rows, rows_scale, total;
-    Layout(int64_t M, int64_t H, int64_t I, int64_t E, int64_t topk, int qt, bool fp8_in) {
+    int64_t max_pairs, max_singles, lists, P, ld, sorted_ids, sorted_w, sorted_eids, num_valid, sort_ws, acc, a1, a1_scale, a2, a2_scale,
+        a2_half, words, rows, rows_scale, total;
+    Layout(int64_t M, int64_t H, int64_t I, int64_t E, int64_t topk, int qt, bool fp8_in, bool in_pairs) {
         const bool rowwise = qt == kQuantPerToken || qt == kQuantPerTensor;
+        pairs = in_pairs;
         P = M * topk + E * kUnit - topk;
         ld = (P + 31) / 32 * 32;                 // row of a transposed scale array
         int64_t at = 0;
@@ -63,7 +81,6 @@ struct Layout {
         num_valid = take(8);
         max_pairs = M * topk / (kUnit + 1);      // a pair needs more than one block's rows
         max_singles = std::min(E, M * topk);     // at most one per expert
-        pairs = works_in_pairs(M, H, I, E, topk, rowwise);
         lists = take(pairs ? (2 + max_pairs + max_singles) * 4 : 0);
         sort_ws = take(sorting_workspace_bytes((int)M, (int)E, (int)topk));
         a1_scale = take(M * (rowwise ? 1 : H / 128) * 4);
@@ -96,16 +113,21 @@ aiter_tensor_t tensor(const void* ptr, int dtype, int dev, int64_t d0, int64_t d
     return t;
 }
 
+bool rowwise_quant(int qt) { return qt == kQuantPerToken || qt == kQuantPerTensor; }
+
 }  // namespace
 
+void set_debug_pairs(int mode) { t_debug_pairs = mode; }
+
+// For every number of local experts: with all of them here a layer is worked in pairs at the fewest tokens.
 int64_t fused_moe_workspace_bytes(int64_t M, int64_t H, int64_t I, int64_t E, int64_t topk, int qt, int hidden_dtype) {
-    return Layout(M, H, I, E, topk, qt, hidden_dtype == AITER_DTYPE_fp8).total;
+    return Layout(M, H, I, E, topk, qt, hidden_dtype == AITER_DTYPE_fp8, works_in_pairs(M, H, I, E, E, topk, rowwise_quant(qt))).total;
 }
 
 // Kernels that launch_fused_moe below enqueues for these sizes.
-int fused_moe_launches(int64_t M, int64_t H, int64_t I, int64_t E, int64_t topk, int qt, int hidden_dtype) {
-    const bool per_tensor = qt == kQuantPerTensor, rowwise = per_tensor || qt == kQuantPerToken;
-    const bool pairs = works_in_pairs(M, H, I, E, topk, rowwise);
+int fused_moe_launches(int64_t M, int64_t H, int64_t I, int64_t E, int64_t global_E, int64_t topk, int qt, int hidden_dtype) {
+    const bool per_tensor = qt == kQuantPerTensor, rowwise = rowwise_quant(qt);
+    const bool pairs = works_in_pairs(M, H, I, E, global_E, topk, rowwise);
     int n = sorting_launches(M * topk);
     if (hidden_dtype != AITER_DTYPE_fp8) n += per_tensor ? 2 : 1;   // maximum, codes
     n += pairs && rowwise ? 3 : 1;                                  // stage 1: rows in order, pairs, single blocks
@@ -118,10 +140,10 @@ void launch_fused_moe(const b200_fused_moe_args& a, cudaStream_t stream) {
     const int dev = (int)a.device, qt = (int)a.quant_type;
     const int64_t M = a.M, H = a.H, I = a.I, E = a.E;
     const bool fp8_in = a.hidden_dtype == AITER_DTYPE_fp8;
-    const bool per_tensor = qt == kQuantPerTensor, rowwise = per_tensor || qt == kQuantPerToken;
-    B200_CHECK(M >= 1 && H >= 1 && I >= 1 && E >= 1 && a.topk >= 1, "sizes must be positive");
+    const bool per_tensor = qt == kQuantPerTensor, rowwise = rowwise_quant(qt);
+    B200_CHECK(M >= 1 && H >= 1 && I >= 1 && E >= 1 && a.global_E >= 1 && a.topk >= 1, "sizes must be positive");
     B200_CHECK(a.workspace != nullptr && ((uintptr_t)a.workspace & 255) == 0, "workspace must be 256-byte aligned");
-    const Layout at(M, H, I, a.global_E, a.topk, qt, fp8_in);
+    const Layout at(M, H, I, a.global_E, a.topk, qt, fp8_in, works_in_pairs(M, H, I, E, a.global_E, a.topk, rowwise));
     B200_CHECK(a.workspace_bytes >= at.total, "workspace needs ", at.total, " bytes, has ", a.workspace_bytes);
     char* ws = (char*)a.workspace;
     const int F32 = AITER_DTYPE_fp32, I32 = AITER_DTYPE_i32, FP8 = AITER_DTYPE_fp8;

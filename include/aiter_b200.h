@@ -160,7 +160,7 @@ typedef struct b200_fused_moe_args {
 int64_t b200_fused_moe_workspace_size(int64_t M, int64_t H, int64_t I, int64_t global_E, int64_t topk, int quant_type,
                                       int hidden_dtype);
 /* Kernels that b200_fused_moe enqueues for these sizes (callers that report how many kernels they ran) */
-int b200_fused_moe_launches(int64_t M, int64_t H, int64_t I, int64_t global_E, int64_t topk, int quant_type,
+int b200_fused_moe_launches(int64_t M, int64_t H, int64_t I, int64_t E, int64_t global_E, int64_t topk, int quant_type,
                             int hidden_dtype);
 int b200_fused_moe(const b200_fused_moe_args* args, void* stream);
 
@@ -258,6 +258,9 @@ int b200_ep_ipc_close(int64_t ptr, int device);
  * stall_weight_producer makes the weight-loading role issue nothing. With it stalled nothing is in flight, the waits run
  * out, every CTA winds down and frees its tensor memory, and the caller's status word is set to 1. Tests only. */
 int b200_moe_debug_config(int64_t wait_limit_cycles, int stall_weight_producer);
+/* Tests only: whether the calling thread's later b200_fused_moe calls work row blocks in pairs of CTAs. 0: where it pays (default),
+ * 1: wherever a pair is possible, 2: never. Holds for b200_fused_moe_workspace_size and b200_fused_moe_launches as well. */
+int b200_moe_debug_pairs(int mode);
 
 /* DeepSeek-V3 style router: sigmoid scores, correction bias for the choice only, groups ranked by the sum
  * of their two best biased scores, top `topk_group` groups kept, top-k experts among them; weights are the

@@ -77,16 +77,42 @@ def test_workspace_size(lib):
     assert ws == (16 * 256 + 256) * 4
 
 
-# M, H, I, experts, topk, quant type, hidden dtype; kernels: sort (two above 16384 routes), quantiser (none for fp8, two for one scale
-# per tensor), stage 1, requantisation of row scales, stage 2, final rounding; layers in pairs: two launches a stage, and with row
-# scales the copy into sorted order
+# M, H, I, experts here, experts, topk, quant type, hidden dtype; kernels: sort (two above 16384 routes), quantiser (none for fp8, two for
+# one scale per tensor), stage 1, requantisation of row scales, stage 2, final rounding; layers in pairs: two launches a stage, and with
+# row scales the copy into sorted order
 @pytest.mark.parametrize("sizes,kernels", [
-    ((1, 4096, 1536, 128, 8, 4, torch.bfloat16), 5), ((513, 1024, 512, 8, 2, 1, torch.bfloat16), 7),
-    ((32, 4096, 14336, 8, 2, 2, torch.float16), 6), ((2048, 7168, 2048, 256, 8, 4, torch.float8_e4m3fn), 4),
-    ((3000, 7168, 512, 256, 8, 4, torch.bfloat16), 6), ((4096, 4096, 14336, 8, 2, 2, torch.bfloat16), 9),
-    ((9000, 4096, 14336, 8, 2, 1, torch.bfloat16), 11), ((16384, 4096, 1536, 128, 8, 4, torch.bfloat16), 7)])
+    ((1, 4096, 1536, 128, 128, 8, 4, torch.bfloat16), 5), ((513, 1024, 512, 8, 8, 2, 1, torch.bfloat16), 7),
+    ((32, 4096, 14336, 8, 8, 2, 2, torch.float16), 6), ((2048, 7168, 2048, 32, 256, 8, 4, torch.float8_e4m3fn), 4),
+    ((3000, 7168, 512, 256, 256, 8, 4, torch.bfloat16), 6), ((4096, 4096, 14336, 8, 8, 2, 2, torch.bfloat16), 9),
+    ((9000, 4096, 14336, 8, 8, 2, 1, torch.bfloat16), 11), ((16384, 4096, 1536, 128, 128, 8, 4, torch.bfloat16), 7)])
 def test_kernels_of_a_layer_call(lib, sizes, kernels):
     assert lib.b200_fused_moe_launches(*sizes[:-1], _lib.AITER_DTYPE[sizes[-1]]) == kernels
+
+
+# M, H, I, experts here, experts, topk, row scales, in pairs; both sides of every line of the rule
+@pytest.mark.parametrize("M,H,I,local,E,topk,rows,pairs", [
+    (4096, 4096, 1024, 32, 32, 8, False, True), (4096, 4096, 896, 32, 32, 8, False, False),          # inner dimension
+    (2304, 7168, 2048, 128, 128, 8, False, True), (2303, 7168, 2048, 128, 128, 8, False, False),     # 144 rows an expert
+    (1055, 7168, 2048, 32, 32, 8, False, True), (1056, 7168, 2048, 32, 32, 8, False, False),         # mostly three blocks from here
+    (1503, 7168, 2048, 32, 32, 8, False, False), (1504, 7168, 2048, 32, 32, 8, False, True),         # ... to here
+    (7104, 1024, 1024, 8, 8, 4, False, True), (7103, 1024, 1024, 8, 8, 4, False, False),             # six rounds of tiles
+    (1000, 256, 1024, 4, 4, 1, False, False), (601, 4096, 4096, 4, 4, 1, False, False),              # small layers
+    (8192, 7168, 2048, 32, 256, 8, False, True), (8192, 7168, 2048, 15, 256, 8, False, False),       # the share of this rank
+    (592, 4096, 14336, 8, 8, 2, True, True), (578, 4096, 14336, 8, 8, 2, True, False),               # row scales
+    (8192, 2048, 4096, 32, 32, 8, True, True), (8192, 1920, 4096, 32, 32, 8, True, False), (8192, 4096, 3968, 32, 32, 8, True, False),
+    (2400, 4096, 4096, 32, 32, 8, True, False), (2400, 4096, 6144, 32, 32, 8, True, True),           # five blocks
+    (1601, 4096, 4096, 8, 8, 2, True, False), (4096, 2048, 6144, 8, 8, 2, True, False), (4096, 4096, 8192, 8, 8, 2, True, True)])
+def test_layers_in_pairs(lib, M, H, I, local, E, topk, rows, pairs):
+    bf16 = _lib.AITER_DTYPE[torch.bfloat16]
+    kernels = (9 if pairs else 6) if rows else (6 if pairs else 5)
+    assert lib.b200_fused_moe_launches(M, H, I, local, E, topk, 2 if rows else 4, bf16) == kernels + (M * topk > 16384)
+
+
+def test_sizes_that_are_no_layer(lib):
+    """The queries answer, whatever they are asked."""
+    for sizes in ((0, 0, 0, 0, 0, 0), (-1, 4096, 4096, 8, 8, 2), (4096, 4096, 4096, 8, 0, 2)):
+        assert lib.b200_fused_moe_launches(*sizes, 2, 0) >= 4
+        assert lib.b200_fused_moe_workspace_size(*sizes[:3], sizes[4], sizes[5], 2, 0) is not None
 
 
 def test_workspace_of_a_layer(lib):

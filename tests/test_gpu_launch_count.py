@@ -1,6 +1,7 @@
 """``_lib.launch_count`` against the kernels that a captured layer call holds."""
 
 import ctypes
+import importlib
 
 import pytest
 import torch
@@ -8,6 +9,7 @@ import torch
 import aiter_b200
 from aiter_b200 import _lib
 
+fm = importlib.import_module("aiter_b200.fused_moe")
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 QT = aiter_b200.QuantType
@@ -32,9 +34,11 @@ def _kernel_nodes(graph):
 
 @pytest.mark.parametrize("qt", list(SCALES))
 @pytest.mark.parametrize("x_dtype", [torch.bfloat16, FP8])
-# few rows per expert, above 16384 routes, rows enough for pairs of blocks, both
-@pytest.mark.parametrize("M,topk,E,I", [(40, 2, 8, 256), (8200, 2, 256, 256), (300, 2, 4, 4096), (8200, 2, 4, 4096)])
-def test_count_is_what_a_graph_of_the_call_holds(qt, x_dtype, M, topk, E, I):
+# up to 16384 routes, above; one block a CTA and pairs (b200_moe_debug_pairs)
+@pytest.mark.parametrize("M,topk,E,I", [(40, 2, 8, 256), (8200, 2, 256, 256), (300, 2, 4, 1024), (8200, 2, 4, 1024)])
+@pytest.mark.parametrize("pairs", [1, 2])
+def test_count_is_what_a_graph_of_the_call_holds(qt, x_dtype, M, topk, E, I, pairs, monkeypatch):
+    monkeypatch.setattr(fm, "_layer_sizes", fm._layer_sizes.__wrapped__)
     g = torch.Generator(device=DEV).manual_seed(1)
     H = 2048
     x, a1_scale = torch.randn((M, H), generator=g, device=DEV).to(torch.bfloat16), None
@@ -48,10 +52,14 @@ def test_count_is_what_a_graph_of_the_call_holds(qt, x_dtype, M, topk, E, I):
     def run():
         return aiter_b200.fused_moe(x, w1, w2, wts, ids, quant_type=qt, w1_scale=s1, w2_scale=s2, a1_scale=a1_scale)
 
-    run()
-    torch.cuda.synchronize()
-    graph = torch.cuda.CUDAGraph(keep_graph=True)
-    before = _lib.launch_count
-    with torch.cuda.graph(graph):
+    _lib.call_plain("b200_moe_debug_pairs", pairs)
+    try:
         run()
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph(keep_graph=True)
+        before = _lib.launch_count
+        with torch.cuda.graph(graph):
+            run()
+    finally:
+        _lib.call_plain("b200_moe_debug_pairs", 0)
     assert _lib.launch_count - before == _kernel_nodes(graph)
