@@ -63,7 +63,7 @@ _SIGNATURES = {
     "b200_moe_debug_config": (ctypes.c_int, [ctypes.c_int64, ctypes.c_int]),
     "b200_moe_debug_pairs": (ctypes.c_int, [ctypes.c_int]),
     "b200_fused_moe_workspace_size": (ctypes.c_int64, [ctypes.c_int64] * 5 + [ctypes.c_int] * 2),
-    "b200_fused_moe_launches": (ctypes.c_int, [ctypes.c_int64] * 6 + [ctypes.c_int] * 2),
+    "b200_fused_moe_launches": (ctypes.c_int, [ctypes.c_int64] * 6 + [ctypes.c_int] * 3),
     "b200_fused_moe": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p]),
 }
 

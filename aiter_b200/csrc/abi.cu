@@ -34,7 +34,7 @@ void launch_moe_stage2(const aiter_tensor_t*, const aiter_tensor_t*, const aiter
                        aiter_tensor_t*, aiter_tensor_t*, int, int, int, int, int, bool, SortedStage*, cudaStream_t);
 
 int64_t fused_moe_workspace_bytes(int64_t, int64_t, int64_t, int64_t, int64_t, int, int);
-int fused_moe_launches(int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int, int);
+int fused_moe_launches(int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int, int, bool);
 void set_debug_pairs(int);
 void launch_fused_moe(const b200_fused_moe_args&, cudaStream_t);
 void launch_finalize(aiter_tensor_t*, const aiter_tensor_t*, cudaStream_t);
@@ -258,8 +258,8 @@ B200_EXPORT int64_t b200_fused_moe_workspace_size(int64_t M, int64_t H, int64_t 
 }
 
 B200_EXPORT int b200_fused_moe_launches(int64_t M, int64_t H, int64_t I, int64_t E, int64_t global_E, int64_t topk, int quant_type,
-                                        int hidden_dtype) {
-    return fused_moe_launches(M, H, I, E, global_E, topk, quant_type, hidden_dtype);
+                                        int hidden_dtype, int padded) {
+    return fused_moe_launches(M, H, I, E, global_E, topk, quant_type, hidden_dtype, padded != 0);
 }
 
 B200_EXPORT int b200_fused_moe(const b200_fused_moe_args* args, void* stream) {

@@ -37,6 +37,7 @@ constexpr int64_t kUnit = 128;                           // sort unit == row til
 thread_local int t_debug_pairs = 0;
 
 // Which layers work their row blocks in pairs (moe_gemm_sorted.cu). E: experts of this layer call, of global_E that are routed to.
+// padded: how many of the M tokens are live stands on the device.
 // Timed both ways in turn as graphs: 1132 block-scaled and 699 row-scaled layers, H 512 to 8192, I 1024 to 14336, 8 to 256 experts, 150
 // to 1024 rows an expert, even and Zipf routing. Gain: time with one block a CTA / time in pairs, mean (least).
 //  * Rows. Below 144 an expert most have one block. Experts with three blocks leave one of them single, at the price of a pair each:
@@ -47,11 +48,14 @@ thread_local int t_debug_pairs = 0;
 //  * Row scales, both stages: three launches and a copy of the rows, 10 to 20 us, against a gain that grows with the rounds of
 //    stage 1 and with I, less below H 4096. The 291 layers beyond the line 1.085 (0.986; with I 4096 / 6144 / 8192 / 14336 1.03 / 1.07 / 1.08 / 1.10),
 //    the 408 before it 1.00 (0.80).
-bool works_in_pairs(int64_t M, int64_t H, int64_t I, int64_t E, int64_t global_E, int64_t topk, bool rowwise) {
+//  * Padded batches. What pays for the pairs is rows that the host does not know to be there: with all / a half / a quarter / a 64th of
+//    the tokens live, Mixtral-shaped 4097 tokens 1.16 / 1.04 / 1.06 / 0.95 (row scales) and 1.02 / 1.01 / 1.01 / 0.98, DeepSeek-V3-shaped
+//    8193 tokens 1.05 / 1.02 / 0.99 / 0.97, a quarter of its experts and 6401 tokens 1.03 / 0.98 / 0.99 / 0.99 (block scales).
+bool works_in_pairs(int64_t M, int64_t H, int64_t I, int64_t E, int64_t global_E, int64_t topk, bool rowwise, bool padded) {
     constexpr double kSms = 148;
     const int64_t routes = M * topk;
     if (t_debug_pairs) return t_debug_pairs == 1 && routes > kUnit;
-    if (global_E < 1 || routes < 144 * global_E || routes <= kUnit) return false;
+    if (padded || global_E < 1 || routes < 144 * global_E || routes <= kUnit) return false;
     const int64_t rows = routes / global_E, blocks = (rows + kUnit - 8) / kUnit;   // an expert, 8 rows either way
     if (blocks % 2 && (rows + 8) / kUnit < blocks && blocks <= (rowwise && I < 6144 ? 5 : 3)) return false;
     const double here = (double)routes * std::min(E, global_E) / global_E / kUnit;   // blocks of rows in this call
@@ -119,15 +123,16 @@ bool rowwise_quant(int qt) { return qt == kQuantPerToken || qt == kQuantPerTenso
 
 void set_debug_pairs(int mode) { t_debug_pairs = mode; }
 
-// For every number of local experts: with all of them here a layer is worked in pairs at the fewest tokens.
+// For every number of local experts and live tokens: with all of them here a layer is worked in pairs at the fewest tokens.
 int64_t fused_moe_workspace_bytes(int64_t M, int64_t H, int64_t I, int64_t E, int64_t topk, int qt, int hidden_dtype) {
-    return Layout(M, H, I, E, topk, qt, hidden_dtype == AITER_DTYPE_fp8, works_in_pairs(M, H, I, E, E, topk, rowwise_quant(qt))).total;
+    return Layout(M, H, I, E, topk, qt, hidden_dtype == AITER_DTYPE_fp8, works_in_pairs(M, H, I, E, E, topk, rowwise_quant(qt), false)).total;
 }
 
 // Kernels that launch_fused_moe below enqueues for these sizes.
-int fused_moe_launches(int64_t M, int64_t H, int64_t I, int64_t E, int64_t global_E, int64_t topk, int qt, int hidden_dtype) {
+int fused_moe_launches(int64_t M, int64_t H, int64_t I, int64_t E, int64_t global_E, int64_t topk, int qt, int hidden_dtype,
+                       bool padded) {
     const bool per_tensor = qt == kQuantPerTensor, rowwise = rowwise_quant(qt);
-    const bool pairs = works_in_pairs(M, H, I, E, global_E, topk, rowwise);
+    const bool pairs = works_in_pairs(M, H, I, E, global_E, topk, rowwise, padded);
     int n = sorting_launches(M * topk);
     if (hidden_dtype != AITER_DTYPE_fp8) n += per_tensor ? 2 : 1;   // maximum, codes
     n += pairs && rowwise ? 3 : 1;                                  // stage 1: rows in order, pairs, single blocks
@@ -143,7 +148,7 @@ void launch_fused_moe(const b200_fused_moe_args& a, cudaStream_t stream) {
     const bool per_tensor = qt == kQuantPerTensor, rowwise = rowwise_quant(qt);
     B200_CHECK(M >= 1 && H >= 1 && I >= 1 && E >= 1 && a.global_E >= 1 && a.topk >= 1, "sizes must be positive");
     B200_CHECK(a.workspace != nullptr && ((uintptr_t)a.workspace & 255) == 0, "workspace must be 256-byte aligned");
-    const Layout at(M, H, I, a.global_E, a.topk, qt, fp8_in, works_in_pairs(M, H, I, E, a.global_E, a.topk, rowwise));
+    const Layout at(M, H, I, a.global_E, a.topk, qt, fp8_in, works_in_pairs(M, H, I, E, a.global_E, a.topk, rowwise, a.num_local_tokens != nullptr));
     B200_CHECK(a.workspace_bytes >= at.total, "workspace needs ", at.total, " bytes, has ", a.workspace_bytes);
     char* ws = (char*)a.workspace;
     const int F32 = AITER_DTYPE_fp32, I32 = AITER_DTYPE_i32, FP8 = AITER_DTYPE_fp8;

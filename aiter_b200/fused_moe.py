@@ -404,11 +404,11 @@ _LAYER_ARGS = struct.Struct("@13P16q")
 
 
 @functools.lru_cache(maxsize=1024)
-def _layer_sizes(M, H, I, E, global_E, topk, qt, hidden_code):
+def _layer_sizes(M, H, I, E, global_E, topk, qt, hidden_code, padded):
     """Workspace bytes and kernel launches of a layer call."""
     handle = _lib.lib()
     return (int(handle.b200_fused_moe_workspace_size(M, H, I, global_E, topk, qt, hidden_code)),
-            int(handle.b200_fused_moe_launches(M, H, I, E, global_E, topk, qt, hidden_code)))
+            int(handle.b200_fused_moe_launches(M, H, I, E, global_E, topk, qt, hidden_code, padded)))
 
 
 def _ptr(t):
@@ -449,7 +449,7 @@ def _layer(hidden_states, w1, w2, topk_weight, topk_ids, expert_mask, w1_scale, 
         a1_scale = a1_scale.contiguous()
     global_E = E if expert_mask is None else expert_mask.numel()
     code = dtypes.AITER_DTYPE[hidden_states.dtype]
-    nbytes, launches = _layer_sizes(M, H, I, E, global_E, topk, int(quant_type), code)
+    nbytes, launches = _layer_sizes(M, H, I, E, global_E, topk, int(quant_type), code, num_local_tokens is not None)
     workspace = torch.empty(nbytes, dtype=dtypes.u8, device=device)
     out = torch.empty((M, H), dtype=dtype, device=device)
     args = _LAYER_ARGS.pack(

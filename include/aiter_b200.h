@@ -159,9 +159,9 @@ typedef struct b200_fused_moe_args {
 
 int64_t b200_fused_moe_workspace_size(int64_t M, int64_t H, int64_t I, int64_t global_E, int64_t topk, int quant_type,
                                       int hidden_dtype);
-/* Kernels that b200_fused_moe enqueues for these sizes (callers that report how many kernels they ran) */
+/* Kernels that b200_fused_moe enqueues for these sizes (callers that report how many kernels they ran); padded: with num_local_tokens */
 int b200_fused_moe_launches(int64_t M, int64_t H, int64_t I, int64_t E, int64_t global_E, int64_t topk, int quant_type,
-                            int hidden_dtype);
+                            int hidden_dtype, int padded);
 int b200_fused_moe(const b200_fused_moe_args* args, void* stream);
 
 /* Stage 1: grouped gate/up GEMM over the sorted blocks + SiLU(gate)*up + bf16 rounding +

@@ -86,7 +86,7 @@ def test_workspace_size(lib):
     ((3000, 7168, 512, 256, 256, 8, 4, torch.bfloat16), 6), ((4096, 4096, 14336, 8, 8, 2, 2, torch.bfloat16), 9),
     ((9000, 4096, 14336, 8, 8, 2, 1, torch.bfloat16), 11), ((16384, 4096, 1536, 128, 128, 8, 4, torch.bfloat16), 7)])
 def test_kernels_of_a_layer_call(lib, sizes, kernels):
-    assert lib.b200_fused_moe_launches(*sizes[:-1], _lib.AITER_DTYPE[sizes[-1]]) == kernels
+    assert lib.b200_fused_moe_launches(*sizes[:-1], _lib.AITER_DTYPE[sizes[-1]], 0) == kernels
 
 
 # M, H, I, experts here, experts, topk, row scales, in pairs; both sides of every line of the rule
@@ -105,13 +105,19 @@ def test_kernels_of_a_layer_call(lib, sizes, kernels):
 def test_layers_in_pairs(lib, M, H, I, local, E, topk, rows, pairs):
     bf16 = _lib.AITER_DTYPE[torch.bfloat16]
     kernels = (9 if pairs else 6) if rows else (6 if pairs else 5)
-    assert lib.b200_fused_moe_launches(M, H, I, local, E, topk, 2 if rows else 4, bf16) == kernels + (M * topk > 16384)
+    assert lib.b200_fused_moe_launches(M, H, I, local, E, topk, 2 if rows else 4, bf16, 0) == kernels + (M * topk > 16384)
+
+
+def test_padded_batches_are_not_worked_in_pairs(lib):
+    """The rows that pay for the pairs need not be there."""
+    for quant, kernels in ((4, 6), (2, 7), (1, 8)):   # one kernel of them the count in front of the sort
+        assert lib.b200_fused_moe_launches(9000, 4096, 14336, 8, 8, 2, quant, _lib.AITER_DTYPE[torch.bfloat16], 1) == kernels
 
 
 def test_sizes_that_are_no_layer(lib):
     """The queries answer, whatever they are asked."""
     for sizes in ((0, 0, 0, 0, 0, 0), (-1, 4096, 4096, 8, 8, 2), (4096, 4096, 4096, 8, 0, 2)):
-        assert lib.b200_fused_moe_launches(*sizes, 2, 0) >= 4
+        assert lib.b200_fused_moe_launches(*sizes, 2, 0, 0) >= 4
         assert lib.b200_fused_moe_workspace_size(*sizes[:3], sizes[4], sizes[5], 2, 0) is not None
 
 
