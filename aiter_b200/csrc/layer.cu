@@ -148,7 +148,9 @@ void launch_fused_moe(const b200_fused_moe_args& a, cudaStream_t stream) {
     const bool per_tensor = qt == kQuantPerTensor, rowwise = rowwise_quant(qt);
     B200_CHECK(M >= 1 && H >= 1 && I >= 1 && E >= 1 && a.global_E >= 1 && a.topk >= 1, "sizes must be positive");
     B200_CHECK(a.workspace != nullptr && ((uintptr_t)a.workspace & 255) == 0, "workspace must be 256-byte aligned");
-    const Layout at(M, H, I, a.global_E, a.topk, qt, fp8_in, works_in_pairs(M, H, I, E, a.global_E, a.topk, rowwise, a.num_local_tokens != nullptr));
+    Layout at(M, H, I, a.global_E, a.topk, qt, fp8_in, works_in_pairs(M, H, I, E, a.global_E, a.topk, rowwise, a.num_local_tokens != nullptr));
+    if (at.pairs && a.workspace_bytes < at.total)   // no room for the pairs' lists and rows: one block a CTA asks for less
+        at = Layout(M, H, I, a.global_E, a.topk, qt, fp8_in, false);
     B200_CHECK(a.workspace_bytes >= at.total, "workspace needs ", at.total, " bytes, has ", a.workspace_bytes);
     char* ws = (char*)a.workspace;
     const int F32 = AITER_DTYPE_fp32, I32 = AITER_DTYPE_i32, FP8 = AITER_DTYPE_fp8;

@@ -107,6 +107,31 @@ def test_stage2_scales_at_any_address():
     _against_oracle(out, c, QT.per_1x128)
 
 
+@pytest.mark.parametrize("qt,H,I", [(QT.per_1x128, 1152, 1024), (QT.per_Token, 1152, 1280), (QT.per_Tensor, 1024, 1152)])
+def test_workspace_of_a_layer_without_pairs_is_enough(qt, H, I, monkeypatch):
+    """A caller whose workspace holds the layer but not what the pairs ask for besides gets the layer, to the last byte of it."""
+    sizes_of, given = fm._layer_sizes, []
+
+    def without_pairs(*sizes):
+        more = sizes_of(*sizes)[0]
+        _lib.call_plain("b200_moe_debug_pairs", 2)
+        given.append(sizes_of(*sizes))
+        _lib.call_plain("b200_moe_debug_pairs", 1)
+        assert given[-1][0] < more
+        return given[-1][0] - short, given[-1][1]
+
+    monkeypatch.setattr(fm, "_layer_sizes", without_pairs)
+    c = _batch(qt, 2, H, I)
+    d = {k: v.to(DEV) for k, v in c.items()}
+    short = 0
+    out = _call(d, qt)(d["x"], d["wts"], d["ids"])
+    aiter_b200.check_device_status()
+    _against_oracle(out, c, qt)
+    short = 1
+    with pytest.raises(RuntimeError, match="workspace needs"):
+        _call(d, qt)(d["x"], d["wts"], d["ids"])
+
+
 @pytest.mark.parametrize("qt,H,I", [(QT.per_1x128, 1152, 1024), (QT.per_Token, 1152, 1280)])
 def test_captured_layer(qt, H, I):
     """The launches beside one another keep their order in a graph: replays with other inputs, back to back."""
