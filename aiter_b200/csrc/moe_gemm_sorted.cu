@@ -579,6 +579,8 @@ void launch_blocks(const CUtensorMap& tmap_w, const CUtensorMap& tmap_a, SortedG
 template <int STAGE, bool PT, int ACT = 0>
 void launch_lists(const void* w, int64_t w_rows, const void* a, int64_t a_rows, int64_t K, SortedGemmParams p, const BlockLists& lists,
                   int dev, cudaStream_t stream) {
+    // the launch over the single blocks starts without a wait of its own: there has to be one over pairs in front of it
+    B200_CHECK(lists.max_pairs >= 1 && p.n_tiles >= 1, "row blocks cannot be worked in pairs");
     const CUtensorMap tmap_w = make_map(w, (uint64_t)w_rows, (uint64_t)K, 128);
     p.blocks = lists.pairs;
     p.num_blocks = lists.counts;
