@@ -40,14 +40,15 @@ thread_local int t_debug_pairs = 0;
 // padded: how many of the M tokens are live stands on the device.
 // Timed both ways in turn as graphs: 1132 block-scaled and 699 row-scaled layers, H 512 to 8192, I 1024 to 14336, 8 to 256 experts, 150
 // to 1024 rows an expert, even and Zipf routing. Gain: time with one block a CTA / time in pairs, mean (least).
-//  * Rows. Below 144 an expert most have one block. Experts with three blocks leave one of them single, at the price of a pair each:
-//    block scales at 220 / 300 / 400 rows 1.05 / 1.00 (0.96) / 1.04, row scales 1.15 / 1.00 (0.95) / 1.10; with row scales and I 4096
-//    the fifth block is too much as well, at 600 rows 0.99 (0.97).
+//  * Rows. Below 144 an expert most have one block. With three blocks each expert leaves one single, at the price of a pair: block
+//    scales with 7 / 12 to 14 / 29 / 50 rounds of tiles 0.99 / 1.00 to 1.02 / 1.03 / 1.03 at 265 to 375 rows an expert; row scales with
+//    I 4096 / 6144 / 8192 / 10880 / 14336 0.98 (0.96) / 1.00 (0.95) / 0.97 (0.92) / 1.01 / 1.01, and with I 4096 at five blocks 0.99
+//    (0.97). Zipf routing, where the experts differ, gains 1.01 to 1.06 there, but the host does not see the routing.
 //  * Block scales, stage 2 only: a second launch, 2 to 4 us, and tiles of twice the size want several rounds of tiles. By rounds of
 //    128 x 256 tiles on all SMs below 1: 0.94 (0.88), 1-3: 0.98 (0.90), 3-6: 1.00 (0.95), 6-12: 1.02, 12-24: 1.03, above: 1.05.
 //  * Row scales, both stages: three launches and a copy of the rows, 10 to 20 us, against a gain that grows with the rounds of
-//    stage 1 and with I, less below H 4096. The 291 layers beyond the line 1.085 (0.986; with I 4096 / 6144 / 8192 / 14336 1.03 / 1.07 / 1.08 / 1.10),
-//    the 408 before it 1.00 (0.80).
+//    stage 1 and with I, less below H 4096. Three blocks aside, the 291 layers beyond the line 1.085 (0.986; with I 4096 / 6144 / 8192 /
+//    14336 1.03 / 1.07 / 1.08 / 1.10), the 408 before it 1.00 (0.80).
 //  * Padded batches. What pays for the pairs is rows that the host does not know to be there: with all / a half / a quarter / a 64th of
 //    the tokens live, Mixtral-shaped 4097 tokens 1.16 / 1.04 / 1.06 / 0.95 (row scales) and 1.02 / 1.01 / 1.01 / 0.98, DeepSeek-V3-shaped
 //    8193 tokens 1.05 / 1.02 / 0.99 / 0.97, a quarter of its experts and 6401 tokens 1.03 / 0.98 / 0.99 / 0.99 (block scales).
@@ -56,10 +57,11 @@ bool works_in_pairs(int64_t M, int64_t H, int64_t I, int64_t E, int64_t global_E
     const int64_t routes = M * topk;
     if (t_debug_pairs) return t_debug_pairs == 1 && routes > kUnit;
     if (padded || global_E < 1 || routes < 144 * global_E || routes <= kUnit) return false;
-    const int64_t rows = routes / global_E, blocks = (rows + kUnit - 8) / kUnit;   // an expert, 8 rows either way
-    if (blocks % 2 && (rows + 8) / kUnit < blocks && blocks <= (rowwise && I < 6144 ? 5 : 3)) return false;
+    const int64_t rows = routes / global_E, blocks = (rows + kUnit - 8) / kUnit;     // an expert
+    const int64_t odd = blocks % 2 && (rows + 8) / kUnit < blocks ? blocks : 0;      // most experts have this odd number of blocks
     const double here = (double)routes * std::min(E, global_E) / global_E / kUnit;   // blocks of rows in this call
-    if (!rowwise) return I >= 1024 && here * H / 256 >= 6 * kSms;
+    if (!rowwise) return I >= 1024 && here * H / 256 >= (odd == 3 ? 12 : 6) * kSms;
+    if ((odd == 3 && I < 10240) || (odd == 5 && I < 6144)) return false;
     return I >= 4096 && H >= 2048 && here * I / 128 / kSms * I * std::min<int64_t>(H, 4096) >= 98304. * 4096;
 }
 

@@ -93,14 +93,16 @@ def test_kernels_of_a_layer_call(lib, sizes, kernels):
 @pytest.mark.parametrize("M,H,I,local,E,topk,rows,pairs", [
     (4096, 4096, 1024, 32, 32, 8, False, True), (4096, 4096, 896, 32, 32, 8, False, False),          # inner dimension
     (2304, 7168, 2048, 128, 128, 8, False, True), (2303, 7168, 2048, 128, 128, 8, False, False),     # 144 rows an expert
-    (1055, 7168, 2048, 32, 32, 8, False, True), (1056, 7168, 2048, 32, 32, 8, False, False),         # mostly three blocks from here
-    (1503, 7168, 2048, 32, 32, 8, False, False), (1504, 7168, 2048, 32, 32, 8, False, True),         # ... to here
+    (527, 7168, 2048, 16, 16, 8, False, True), (528, 7168, 2048, 16, 16, 8, False, False),           # mostly three blocks from here
+    (751, 7168, 2048, 16, 16, 8, False, False), (752, 7168, 2048, 16, 16, 8, False, True),           # ... to here
+    (1056, 7168, 2048, 32, 32, 8, False, True), (1056, 6784, 2048, 32, 32, 8, False, False),         # ... which want twelve rounds
     (7104, 1024, 1024, 8, 8, 4, False, True), (7103, 1024, 1024, 8, 8, 4, False, False),             # six rounds of tiles
     (1000, 256, 1024, 4, 4, 1, False, False), (601, 4096, 4096, 4, 4, 1, False, False),              # small layers
     (8192, 7168, 2048, 32, 256, 8, False, True), (8192, 7168, 2048, 15, 256, 8, False, False),       # the share of this rank
     (592, 4096, 14336, 8, 8, 2, True, True), (578, 4096, 14336, 8, 8, 2, True, False),               # row scales
     (8192, 2048, 4096, 32, 32, 8, True, True), (8192, 1920, 4096, 32, 32, 8, True, False), (8192, 4096, 3968, 32, 32, 8, True, False),
     (2400, 4096, 4096, 32, 32, 8, True, False), (2400, 4096, 6144, 32, 32, 8, True, True),           # five blocks
+    (1200, 4096, 10240, 8, 8, 2, True, True), (2400, 4096, 10112, 16, 16, 2, True, False),           # three blocks
     (1601, 4096, 4096, 8, 8, 2, True, False), (4096, 2048, 6144, 8, 8, 2, True, False), (4096, 4096, 8192, 8, 8, 2, True, True)])
 def test_layers_in_pairs(lib, M, H, I, local, E, topk, rows, pairs):
     bf16 = _lib.AITER_DTYPE[torch.bfloat16]
