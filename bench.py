@@ -761,7 +761,8 @@ def main():
                 kb_acc.setdefault(n0, []).append(e0.elapsed_time(e1))
         kb = {k: sum(v) / len(v) for k, v in kb_acc.items()}
         line["kernels_ms"] = {k: round(v, 4) for k, v in kb.items()}
-        line["kernels_how"] = "a second loop of the same steps with event marks between the stages, launched one by one"
+        line["kernels_how"] = ("a second loop of the same steps with event marks between the stages, launched one by one; stage 2 by itself "
+                               "works one row block a CTA, in the layer that value and e2e time it works pairs of them")
         s1 = 4.0 * M_PREFILL * TOPK * H * I / (kb["stage1"] * 1e-3) / 1e12
         s2 = 2.0 * M_PREFILL * TOPK * H * I / (kb["stage2"] * 1e-3) / 1e12
         line["roofline"] = {"bound": "tensor", "kernel": "stage-1 GEMM (gate/up + SiLU*up + requant)", "achieved": s1,
@@ -771,7 +772,8 @@ def main():
                             "algorithmic_bytes": 2 * E * I * H + M_PREFILL * H + M_PREFILL * TOPK * I,
                             "peak_source": f"2 x bf16_tflops of {pk['source']} ({pk['bf16_tflops']} TFLOP/s burst); "
                                            "the driver's peak file has no FP8 entry",
-                            "stage2_achieved": s2, "stage2_frac": s2 / fp8_peak}
+                            "stage2_achieved": s2, "stage2_frac": s2 / fp8_peak,
+                            "stage2_kernel": "moe_gemm_kernel<2>, launched by itself; not the kernel of the timed layer"}
         line["layer_frac_of_fp8_peak"] = value / fp8_peak
         lib = library_fp8_gemm_tflops(dev)
         if lib is not None:
