@@ -572,7 +572,7 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
                 // Measured: an SM gets ~20 B/clock of fp32 reductions into L2 whether they are issued as
                 // red.global.v4 from registers or as bulk reductions (plain stores: ~35 B/clock), i.e. ~6k clocks
                 // per tile that the MMA warp, at most two K steps ahead, waits out; hiding them needs a buffer
-                // for the whole 128 KB tile, which neither shared nor tensor memory has room for.
+                // for the whole 128 KB tile, for which three stages of 48 KB leave no room (the pairs' stages of 32 KB do).
                 const uint32_t srow = sbase + S::kOffStage + (uint32_t)((warp - kEpiWarp0) * 32 + lane) * kStageRowBytes;
                 const int n_groups = (nt * 256 + 128 < p.n_rows) ? 2 : 1;
                 if (valid) {

@@ -16,11 +16,14 @@
 //    that puts them in order is 21 us of 1540 for 8192 rows of 4096).
 //  * The reductions of stage 2: see the reducer. K step of the 16384-token Qwen3-shaped layer 1745 clocks in moe_gemm.cu,
 //    1230 here.
-// Measured, layers in turn with the same layers worked one block a CTA: Mixtral-shaped, 4096 tokens 2167 -> 1881 us, Qwen3-shaped, 16384
-// tokens 4178 -> 4044, DeepSeek-V3-shaped, 8192 tokens 5501 -> 5435; stage 2 of the last two 1.48 -> 1.24 and 1.93 -> 1.65 ms (the
-// clock falls as the work gets denser: these run at the power limit). Stage 1 with block scales was built here as well and gained
-// nothing (2.29 against 2.30 + 0.15 ms for putting the rows in order, Qwen3-shaped): its promotion is the serial chain, whose every
-// access to shared memory, barriers included, takes 100 to 300 clocks while the UMMAs read their operands.
+// Measured, layers in turn with the same layers worked one block a CTA, on three boxes, in us: Mixtral-shaped, 4096 tokens, 2056..2108 ->
+// 1804..1825; Qwen3-shaped, 16384 tokens, 4132..4169 -> 3928..3955; DeepSeek-V3-shaped, 8192 tokens, 5328..5426 -> 5218..5278 (the clock
+// falls as the work gets denser: these run at the power limit). Stage 2 of the last two, in one call: 1.48 -> 1.24 and 1.93 -> 1.65 ms.
+// Stage 1 with block scales was built here as well and gained nothing (Qwen3-shaped: 2.29 ms one block a CTA, 2.19 and 2.30 in two
+// builds of pairs, and 0.15 for putting the rows in order): its promotion is the serial chain, whose every access to shared memory,
+// barriers included, takes 100 to 300 clocks while the UMMAs read their operands. Which layers gain and which lose: works_in_pairs
+// (layer.cu). ptxas spills 40 to 100 bytes of the 96 registers the CTA is launched with; 3.2 % of the instructions of stage 2's pairs
+// are reloads of them, whose cost was not measured by itself.
 
 #include <algorithm>
 
